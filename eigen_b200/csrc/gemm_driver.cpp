@@ -87,7 +87,7 @@ int resolve_dgemm_method(int64_t m, int64_t n, int64_t k) {
   const int fc = forced_config();
   if (fc >= kCfgNative && fc <= kCfgCrtSplitK) return fc == kCfgNative ? EB2_METHOD_NATIVE : EB2_METHOD_CRT;
   int cfg = -1, cls = 0;
-  if (picker_weights() != nullptr && picker_predict(m, n, k, 'd', 0.0, 1, settings().dgemm_tol.load(), &cfg, &cls))
+  if (picker_installed() && picker_predict(m, n, k, 'd', 0.0, 1, settings().dgemm_tol.load(), &cfg, &cls))
     return cfg == kCfgNative ? EB2_METHOD_NATIVE : EB2_METHOD_CRT;
   return auto_method_rule(m, n, k);
 }
@@ -141,7 +141,7 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
   }
   const int fc = forced_config();
   const bool forced_cfg = fc >= kCfgCrtCta && fc <= kCfgCrtSplitK;
-  const bool stage2 = picker_weights() != nullptr && !forced_cfg && (auto_tile || forced == 0) &&
+  const bool stage2 = picker_installed() && !forced_cfg && (auto_tile || forced == 0) &&
                       capture == cudaStreamCaptureStatusNone;
   const int nmax = (check || stage2) ? std::max(nmod, kCrtMaxModuli) : nmod;
   int tile = (opt.tile_n == kTilePair || opt.tile_n == kTileWide || opt.tile_n == 256) ? opt.tile_n
@@ -433,7 +433,7 @@ int dgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
     int pick_cfg = -1, pick_s = 0;
     if (fc >= kCfgNative && fc <= kCfgCrtSplitK)
       method = fc == kCfgNative ? EB2_METHOD_NATIVE : EB2_METHOD_CRT;
-    else if (picker_weights() != nullptr &&
+    else if (picker_installed() &&
              picker_predict(m, n, k, 'd', 0.0, 1, opt.tol > 0 ? opt.tol : settings().dgemm_tol.load(), &pick_cfg,
                             &pick_s))
       method = pick_cfg == kCfgNative ? EB2_METHOD_NATIVE : EB2_METHOD_CRT;
@@ -624,7 +624,7 @@ int sgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
     int cfg = -1, cls = 0;
     if (fc >= kCfgSgemmFfma && fc <= kCfgSgemmBf16Pair)
       cfg = fc;
-    else if (picker_weights() == nullptr || !picker_predict(m, n, k, 's', 0.0, 1, kSgemmTolFeature, &cfg, &cls))
+    else if (!picker_installed() || !picker_predict(m, n, k, 's', 0.0, 1, kSgemmTolFeature, &cfg, &cls))
       cfg = -1;
     method = cfg == kCfgSgemmFfma ? EB2_METHOD_NATIVE : EB2_METHOD_EMULATED;
     if (cfg > kCfgSgemmFfma) cfg_tile = cfg == kCfgSgemmBf16_128 ? 128 : (cfg == kCfgSgemmBf16_256 ? 256 : kTilePair);

@@ -61,7 +61,7 @@ GroupedClasses resolve_classes(char dtype, int64_t count, const eb2_gemm_problem
   int cfg = forced_config();
   if (cfg != kCfgBatchClasses && cfg != kCfgBatchTiles) {
     cfg = -1;
-    if (picker_weights() != nullptr && count > 1) {
+    if (picker_installed() && count > 1) {
       double lm = 0, ln = 0, lk = 0;
       int64_t used = 0;
       for (int64_t i = 0; i < count; ++i) {

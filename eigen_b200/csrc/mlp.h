@@ -43,8 +43,8 @@ void picker_features(int64_t m, int64_t n, int64_t k, char dtype, double spread,
                      float* out);
 // Host forward (same arithmetic as the device kernel); logits[kMlpOut].
 void picker_forward(const float* w, const float* x, float* logits);
-// Installed picker weights (null when none).
-const float* picker_weights();
+// Whether picker weights are installed.
+bool picker_installed();
 bool picker_load_file(const char* path, int num_sms);
 void picker_autoload(int num_sms);
 // The class of kind dtype ('d' or 's'; a grouped batch when batch > 1) with the largest
