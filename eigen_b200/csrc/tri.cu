@@ -161,163 +161,190 @@ __global__ void __launch_bounds__(kTriVecs) tri_block_multiply_kernel(const T* _
   }
 }
 
-// Four consecutive elements of a 16-byte aligned shared-memory row as vector accesses.
-__device__ __forceinline__ void load4(double (&v)[4], const double* p) {
-  const double2 lo = *reinterpret_cast<const double2*>(p), hi = *reinterpret_cast<const double2*>(p + 2);
-  v[0] = lo.x;
-  v[1] = lo.y;
-  v[2] = hi.x;
-  v[3] = hi.y;
-}
-__device__ __forceinline__ void load4(float (&v)[4], const float* p) {
-  const float4 q = *reinterpret_cast<const float4*>(p);
-  v[0] = q.x;
-  v[1] = q.y;
-  v[2] = q.z;
-  v[3] = q.w;
-}
-__device__ __forceinline__ void store4(double* p, const double (&v)[4]) {
-  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
-  *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
-}
-__device__ __forceinline__ void store4(float* p, const float (&v)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-
 // x := E^-1 x for a diagonal block E of up to kPanelMax rows and `count` vectors (laid out
-// as above), kPanelVecs per CTA, the CTA's vectors resident in shared memory for the whole
-// block.  Blocked substitution over 32-row sub-blocks:
-//   * two warps solve the sub-block (one lane per vector) against its 32 x 32 triangle,
-//     column by column with the reciprocal of each diagonal entry, in the order of Eigen's
-//     column-major triangular solve kernel (Eigen/src/Core/products/TriangularSolverMatrix.h:61-82);
-//   * all threads subtract its contribution from the rows below, a register-tiled product
-//     (4 rows x 4 vectors per thread) with the coefficient panel staged in shared memory
-//     128 rows at a time.
+// as above), V of them per CTA, resident in shared memory for the whole block.  Blocked
+// substitution over 16-row sub-blocks:
+//   * one lane per vector solves a sub-block against its 16 x 16 triangle in registers, column
+//     by column with the reciprocal of each diagonal entry, in the order of Eigen's column-major
+//     triangular solve kernel (Eigen/src/Core/products/TriangularSolverMatrix.h:61-82);
+//   * its contribution is subtracted from the rows below as 16 x 8 tile products (DMMA for
+//     double), the next sub-block's rows first, so that the next solve runs in one or two warps
+//     while the others update the rest;
+//   * the coefficients of a sub-block's columns (negated) alternate between two shared-memory
+//     panels; the loads of the panel after next are in flight in registers meanwhile.
 // An upper triangle is solved as the lower one of the index-reversed system (row r <->
-// nb-1-r), so both run forward.
-constexpr int kPanelSub = 32;
-constexpr int kPanelThreads = 512;
-constexpr int kPanelChunk = 128;            // coefficient rows staged per pass
-constexpr int kPanelXld = kPanelVecs + 4;   // row stride of the resident vectors (16 B aligned)
-constexpr int kPanelDld = kPanelSub + 1;    // row stride of the diagonal sub-block
+// nb-1-r), so both run forward.  Rows and columns past nb behave as an identity.
+//
+// Bound by the serial chain of 16 sub-blocks (a solve, a small product and two barriers each),
+// so V shrinks until the vectors fill the SMs.  A 4096 solve with 2048 vectors (16 blocks of 256)
+// went from 3047 to 1820 us against 64 vectors per CTA, 32-row sub-blocks without look-ahead and
+// FMA updates (129 us a block on 32 CTAs).
+constexpr int kPanelSub = 16;
 
-template <typename T>
-__global__ void __launch_bounds__(kPanelThreads) tri_panel_solve_kernel(const T* __restrict__ E, int64_t er, int64_t ec,
-                                                                        int nb, bool lower, bool unit,
-                                                                        T* __restrict__ X, int64_t vs, int64_t ts,
-                                                                        int64_t count) {
-  static_assert(kPanelVecs == 64 && kPanelThreads == 512 && kPanelChunk == 128, "thread tiling");
+template <typename T, int V>
+struct PanelCfg {
+  static constexpr int kThreads = V == 64 ? 512 : 256;
+  static constexpr int kXld = V + 4;  // row stride of the vectors: fragment reads hit distinct banks
+  static constexpr int kSolvers = V == 64 ? 2 : 1;  // solving warps
+  static constexpr int kPer = kPanelMax * kPanelSub / kThreads;  // coefficients a thread stages per panel
+  static size_t smem(int nb) {
+    const size_t nbp = size_t(nb + kPanelSub - 1) / kPanelSub * kPanelSub;
+    return (nbp * kXld + 2 * kPanelSub * (nbp + 4) + kPanelSub) * sizeof(T);
+  }
+};
+
+// rows r0 .. r0+15, columns c0 .. c0+7 of the resident vectors += (panel rows) x (the solved
+// 16 rows at xs): the 16 x 8 accumulator in the m16n8 fragment layout.
+__device__ __forceinline__ void panel_tile(const double* pr, int ldp, const double* xs, double* xd, int xld, int g,
+                                           int tig) {
+  double2 u0 = *reinterpret_cast<const double2*>(xd + g * xld + 2 * tig);
+  double2 u1 = *reinterpret_cast<const double2*>(xd + (g + 8) * xld + 2 * tig);
+#pragma unroll
+  for (int k = 0; k < kPanelSub; k += 4) {
+    const double a0 = pr[(k + tig) * ldp + g], a1 = pr[(k + tig) * ldp + g + 8], b0 = xs[(k + tig) * xld + g];
+    asm volatile(
+        "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+        : "+d"(u0.x), "+d"(u0.y), "+d"(u1.x), "+d"(u1.y)
+        : "d"(a0), "d"(a1), "d"(b0));
+  }
+  *reinterpret_cast<double2*>(xd + g * xld + 2 * tig) = u0;
+  *reinterpret_cast<double2*>(xd + (g + 8) * xld + 2 * tig) = u1;
+}
+__device__ __forceinline__ void panel_tile(const float* pr, int ldp, const float* xs, float* xd, int xld, int g,
+                                           int tig) {
+  float2 u0 = *reinterpret_cast<const float2*>(xd + g * xld + 2 * tig);
+  float2 u1 = *reinterpret_cast<const float2*>(xd + (g + 8) * xld + 2 * tig);
+#pragma unroll
+  for (int k = 0; k < kPanelSub; ++k) {
+    const float a0 = pr[k * ldp + g], a1 = pr[k * ldp + g + 8];
+    const float2 b = *reinterpret_cast<const float2*>(xs + k * xld + 2 * tig);
+    u0.x = fma_rn(a0, b.x, u0.x);
+    u0.y = fma_rn(a0, b.y, u0.y);
+    u1.x = fma_rn(a1, b.x, u1.x);
+    u1.y = fma_rn(a1, b.y, u1.y);
+  }
+  *reinterpret_cast<float2*>(xd + g * xld + 2 * tig) = u0;
+  *reinterpret_cast<float2*>(xd + (g + 8) * xld + 2 * tig) = u1;
+}
+
+template <typename T, int V>
+__global__ void __launch_bounds__(PanelCfg<T, V>::kThreads)
+    tri_panel_solve_kernel(const T* __restrict__ E, int64_t er, int64_t ec, int nb, bool lower, bool unit,
+                           T* __restrict__ X, int64_t vs, int64_t ts, int64_t count) {
+  using C = PanelCfg<T, V>;
+  constexpr int kThreads = C::kThreads, kXld = C::kXld, kWarps = kThreads / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* Xs = reinterpret_cast<T*>(smem_raw);      // [nb][kPanelXld]: Xs[r * kPanelXld + t], forward row order
-  T* Ds = Xs + nb * kPanelXld;                 // [kPanelSub][kPanelDld]: the diagonal sub-block
-  T* Dinv = Ds + kPanelSub * kPanelDld;        // [kPanelSub]: reciprocals of the diagonal
-  T* Cs = Dinv + kPanelSub;                    // [kPanelSub][kPanelChunk]: coefficients, Cs[c * chunk + row]
+  const int nsub = (nb + kPanelSub - 1) / kPanelSub, nbp = nsub * kPanelSub, ldp = nbp + 4;
+  T* Xs = reinterpret_cast<T*>(smem_raw);  // [nbp][kXld]: Xs[r * kXld + t], forward row order
+  T* panel0 = Xs + nbp * kXld;             // [kPanelSub][ldp] each: -E'(jb + r, jb + c) at c * ldp + r
+  T* panel1 = panel0 + kPanelSub * ldp;
+  T* Dinv = panel1 + kPanelSub * ldp;      // [kPanelSub]: reciprocals of the diagonal
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tx = tid & 15, ty = tid >> 4;      // product tiling: vectors 4tx.., rows 4ty..
-  const int64_t t0 = int64_t(blockIdx.x) * kPanelVecs;
-  const int nv = int(count - t0 < kPanelVecs ? count - t0 : kPanelVecs);
+  const int g = lane >> 2, tig = lane & 3;
+  const int64_t t0 = int64_t(blockIdx.x) * V;
+  const int nv = int(count - t0 < V ? count - t0 : V);
   // forward row r is row ro(r) of the stored system
   auto ro = [&](int r) -> int64_t { return lower ? r : nb - 1 - r; };
-  const bool vec_fast = (ts == 1);
-  for (int idx = tid; idx < nb * kPanelVecs; idx += kPanelThreads) {
-    const int t = vec_fast ? idx % kPanelVecs : idx / nb;
-    const int r = vec_fast ? idx / kPanelVecs : idx % nb;
-    Xs[r * kPanelXld + t] = t < nv ? X[ro(r) * vs + (t0 + t) * ts] : T(0);
-  }
-  // the coefficient (r, c) of a panel is contiguous along r when the stored rows are
-  const bool row_fast = (er == 1 || er == -1);
-  for (int jb = 0; jb < nb; jb += kPanelSub) {
-    const int bs = nb - jb < kPanelSub ? nb - jb : kPanelSub;
-    __syncthreads();  // the rows of this sub-block are final (and, first, the load is done)
-    for (int idx = tid; idx < bs * bs; idx += kPanelThreads) {
-      const int r = idx / bs, c = idx % bs;
-      T v = T(0);
-      if (r == c)
-        v = unit ? T(1) : E[ro(jb + r) * er + ro(jb + c) * ec];
-      else if (r > c)
-        v = E[ro(jb + r) * er + ro(jb + c) * ec];
-      Ds[r * kPanelDld + c] = v;
-      if (r == c) Dinv[r] = unit ? T(1) : T(1) / v;
+  // the coefficients are contiguous along the rows, or along the columns when transposed
+  const bool row_fast = er == 1;
+  T cv[C::kPer];
+  auto fetch = [&](int sub) {  // the panel of sub-block `sub` into registers
+    const int jb = sub * kPanelSub;
+#pragma unroll
+    for (int q = 0; q < C::kPer; ++q) {
+      const int idx = tid + q * kThreads;
+      const int r = jb + (row_fast ? idx % kPanelMax : idx / kPanelSub);
+      const int c = jb + (row_fast ? idx / kPanelMax : idx % kPanelSub);
+      T v = r == c ? T(1) : T(0);
+      if (r < nb && (r > c || (r == c && !unit))) v = E[ro(r) * er + ro(c) * ec];
+      cv[q] = v;
     }
-    __syncthreads();
-    if (warp < 2) {
-      // column by column, as Eigen's column-major kernel: x_c = s_c / d_c, then s_r -= d_rc x_c
-      // for every later row r -- independent updates, so the dependent chain is two
-      // operations per row instead of one per coefficient
-      T* x = Xs + warp * 32 + lane;
+  };
+  auto stash = [&](int sub, T* panel) {
+    const int rows = nbp - sub * kPanelSub;
+#pragma unroll
+    for (int q = 0; q < C::kPer; ++q) {
+      const int idx = tid + q * kThreads;
+      const int r = row_fast ? idx % kPanelMax : idx / kPanelSub;
+      const int c = row_fast ? idx / kPanelMax : idx % kPanelSub;
+      if (r < rows) panel[c * ldp + r] = -cv[q];
+    }
+  };
+  auto solve = [&](int sub, const T* panel) {  // the solving warps
+    if (lane < kPanelSub && warp == 0) Dinv[lane] = unit ? T(1) : T(-1) / panel[lane * ldp + lane];
+    if constexpr (C::kSolvers > 1)
+      asm volatile("bar.sync 1, 64;" ::: "memory");
+    else
+      __syncwarp();
+    const int t = warp * 32 + lane;
+    if (t < V) {
+      T* x = Xs + sub * kPanelSub * kXld + t;
       T sv[kPanelSub];
 #pragma unroll
-      for (int r = 0; r < kPanelSub; ++r) sv[r] = r < bs ? x[(jb + r) * kPanelXld] : T(0);
+      for (int r = 0; r < kPanelSub; ++r) sv[r] = x[r * kXld];
 #pragma unroll
       for (int c = 0; c < kPanelSub; ++c) {
-        const T xc = sv[c] * Dinv[c < bs ? c : 0];
+        // x_c = s_c / d_c, then s_r -= d_rc x_c for every later row r: independent updates, so
+        // the dependent chain is two operations per row
+        const T xc = sv[c] * Dinv[c];
         sv[c] = xc;
 #pragma unroll
-        for (int r = c + 1; r < kPanelSub; ++r) sv[r] = fma_rn(-Ds[r * kPanelDld + c], xc, sv[r]);
+        for (int r = c + 1; r < kPanelSub; ++r) sv[r] = fma_rn(panel[c * ldp + r], xc, sv[r]);
       }
 #pragma unroll
-      for (int r = 0; r < kPanelSub; ++r)
-        if (r < bs) x[(jb + r) * kPanelXld] = sv[r];
+      for (int r = 0; r < kPanelSub; ++r) x[r * kXld] = sv[r];
     }
-    // rows below: x[r] -= E'(r, jb..jb+bs) x[jb..jb+bs], kPanelChunk rows per pass
-    for (int r0 = jb + bs; r0 < nb; r0 += kPanelChunk) {
-      const int rows = nb - r0 < kPanelChunk ? nb - r0 : kPanelChunk;
-      // every thread's coefficient loads are issued before its first shared store
-      constexpr int kPerThread = kPanelSub * kPanelChunk / kPanelThreads;
-      T cv[kPerThread];
-#pragma unroll
-      for (int q = 0; q < kPerThread; ++q) {
-        const int idx = tid + q * kPanelThreads;
-        const int rr = row_fast ? idx % kPanelChunk : idx / kPanelSub;
-        const int c = row_fast ? idx / kPanelChunk : idx % kPanelSub;
-        cv[q] = (rr < rows && c < bs) ? E[ro(r0 + rr) * er + ro(jb + c) * ec] : T(0);
-      }
-      __syncthreads();  // the sub-block solve is done / the previous chunk's Cs is consumed
-#pragma unroll
-      for (int q = 0; q < kPerThread; ++q) {
-        const int idx = tid + q * kPanelThreads;
-        const int rr = row_fast ? idx % kPanelChunk : idx / kPanelSub;
-        const int c = row_fast ? idx / kPanelChunk : idx % kPanelSub;
-        Cs[c * kPanelChunk + rr] = cv[q];
-      }
-      __syncthreads();
-      T acc[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
-#pragma unroll 8
-      for (int c = 0; c < kPanelSub; ++c) {
-        // four consecutive coefficients / vector entries as 16-byte loads (no bank conflicts)
-        T a[4], b[4];
-        load4(a, Cs + c * kPanelChunk + 4 * ty);
-        load4(b, Xs + (jb + (c < bs ? c : 0)) * kPanelXld + 4 * tx);
-        if (c < bs) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fma_rn(a[i], b[j], acc[i][j]);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int rr = 4 * ty + i;
-        if (rr < rows) {
-          T* xp = Xs + (r0 + rr) * kPanelXld + 4 * tx;
-          T x4[4];
-          load4(x4, xp);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) x4[j] -= acc[i][j];
-          store4(xp, x4);
-        }
-      }
+  };
+
+  fetch(0);
+  if (ts == 1) {
+    for (int idx = tid; idx < nbp * V; idx += kThreads) {
+      const int t = idx % V, r = idx / V;
+      Xs[r * kXld + t] = (t < nv && r < nb) ? X[ro(r) * vs + t0 + t] : T(0);
     }
+  } else {
+    for (int t = warp; t < V; t += kWarps)
+      for (int r = lane; r < nbp; r += 32)
+        Xs[r * kXld + t] = (t < nv && r < nb) ? X[ro(r) * vs + (t0 + t) * ts] : T(0);
+  }
+  stash(0, panel0);
+  if (nsub > 1) {
+    fetch(1);
+    stash(1, panel1);
   }
   __syncthreads();
-  for (int idx = tid; idx < nb * kPanelVecs; idx += kPanelThreads) {
-    const int t = vec_fast ? idx % kPanelVecs : idx / nb;
-    const int r = vec_fast ? idx / kPanelVecs : idx % nb;
-    if (t < nv) X[ro(r) * vs + (t0 + t) * ts] = Xs[r * kPanelXld + t];
+  if (warp < C::kSolvers) solve(0, panel0);
+  __syncthreads();
+  for (int j = 0; j + 1 < nsub; ++j) {
+    T* const panel = (j & 1) ? panel1 : panel0;       // sub-block j's columns
+    const T* const next = (j & 1) ? panel0 : panel1;  // sub-block j+1's
+    if (j + 2 < nsub) fetch(j + 2);
+    const T* xs = Xs + j * kPanelSub * kXld;
+    // the next sub-block's rows
+    if (warp < V / 8)
+      panel_tile(panel + kPanelSub, ldp, xs + 8 * warp, Xs + (j + 1) * kPanelSub * kXld + 8 * warp, kXld, g, tig);
+    __syncthreads();
+    if (warp < C::kSolvers) {
+      solve(j + 1, next);
+    } else {
+      // the rows below them
+      const int tiles = (nsub - j - 2) * (V / 8);
+      for (int w = warp - C::kSolvers; w < tiles; w += kWarps - C::kSolvers) {
+        const int rt = w / (V / 8) + 2, ct = w % (V / 8);
+        panel_tile(panel + rt * kPanelSub, ldp, xs + 8 * ct, Xs + (j + rt) * kPanelSub * kXld + 8 * ct, kXld, g, tig);
+      }
+    }
+    __syncthreads();
+    if (j + 2 < nsub) stash(j + 2, panel);  // read after the next iteration's first barrier
+  }
+  if (ts == 1) {
+    for (int idx = tid; idx < nb * V; idx += kThreads) {
+      const int t = idx % V, r = idx / V;
+      if (t < nv) X[ro(r) * vs + t0 + t] = Xs[r * kXld + t];
+    }
+  } else {
+    for (int t = warp; t < nv; t += kWarps)
+      for (int r = lane; r < nb; r += 32) X[ro(r) * vs + (t0 + t) * ts] = Xs[r * kXld + t];
   }
 }
 
@@ -386,25 +413,34 @@ cudaError_t launch_tri_block_multiply(const T* E, int64_t er, int64_t ec, int nb
   return cudaGetLastError();
 }
 
-size_t tri_panel_smem(int nb, size_t elem) {
-  return (size_t(nb) * kPanelXld + size_t(kPanelSub) * kPanelDld + kPanelSub + size_t(kPanelSub) * kPanelChunk) *
-         elem;
+namespace {
+
+template <typename T, int V>
+cudaError_t launch_panel(const T* E, int64_t er, int64_t ec, int nb, bool lower, bool unit, T* X, int64_t vs,
+                         int64_t ts, int64_t count, cudaStream_t st) {
+  using C = PanelCfg<T, V>;
+  const int64_t blocks = (count + V - 1) / V;
+  if (blocks > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  auto kern = tri_panel_solve_kernel<T, V>;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(C::smem(kPanelMax)));
+  if (e != cudaSuccess) return e;
+  kern<<<unsigned(blocks), C::kThreads, C::smem(nb), st>>>(E, er, ec, nb, lower, unit, X, vs, ts, count);
+  return cudaGetLastError();
 }
+
+}  // namespace
 
 template <typename T>
 cudaError_t launch_tri_panel_solve(const T* E, int64_t er, int64_t ec, int nb, bool lower, bool unit, T* X, int64_t vs,
                                    int64_t ts, int64_t count, cudaStream_t st) {
   if (count == 0 || nb == 0) return cudaSuccess;
   if (nb < 0 || nb > kPanelMax || count < 0) return cudaErrorInvalidValue;
-  const int64_t blocks = (count + kPanelVecs - 1) / kPanelVecs;
-  if (blocks > 0x7fffffff) return cudaErrorInvalidConfiguration;
-  auto kern = tri_panel_solve_kernel<T>;
-  cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tri_panel_smem(kPanelMax, 8)));
-  if (e != cudaSuccess) return e;
-  kern<<<unsigned(blocks), kPanelThreads, tri_panel_smem(nb, sizeof(T)), st>>>(E, er, ec, nb, lower, unit, X, vs, ts,
-                                                                              count);
-  return cudaGetLastError();
+  // the fewest vectors per CTA that still leave one CTA per SM
+  constexpr int64_t kSms = 148;
+  if (count <= 16 * kSms) return launch_panel<T, 16>(E, er, ec, nb, lower, unit, X, vs, ts, count, st);
+  if (count <= 32 * kSms) return launch_panel<T, 32>(E, er, ec, nb, lower, unit, X, vs, ts, count, st);
+  return launch_panel<T, 64>(E, er, ec, nb, lower, unit, X, vs, ts, count, st);
 }
 
 #define EB2_TRI_INSTANTIATE(T)                                                                                     \
