@@ -782,9 +782,10 @@ __device__ __forceinline__ void crt_store(const CrtStoreCtx& S, int64_t i, int64
   }
 }
 
-// One pair of atomics per block (same-address atomics serialise in L2).
-__device__ __forceinline__ void crt_reduce_energies(const CrtRecParams& R, double e_acc, double v_acc) {
-  __shared__ double red[2][8];
+// One pair of atomics per block (same-address atomics serialise in L2).  `red`: shared memory that
+// no warp still uses.
+__device__ __forceinline__ void crt_reduce_energies(const CrtRecParams& R, double e_acc, double v_acc,
+                                                    double (&red)[2][8]) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     e_acc += __shfl_xor_sync(0xffffffffu, e_acc, o);
@@ -808,8 +809,14 @@ __device__ __forceinline__ void crt_reduce_energies(const CrtRecParams& R, doubl
   }
 }
 
-constexpr int kRecCols = 8;  // most columns per block and pass
-static_assert(kRecCols <= 32, "the estimate's column sum takes a lane per column");
+constexpr int kRecCols = 32;  // most columns per block and pass
+static_assert(kRecCols <= 32 && kRecCols % 4 == 0, "the estimate's column sum takes a lane per column");
+
+// Byte of row i, column j in a residue plane ([cols/4][ld_res][4]: the GEMM's epilogue writes four
+// neighbouring columns of a row as one word).
+__device__ __forceinline__ int64_t residue_index(int64_t i, int64_t j, int64_t ld_res) {
+  return (j >> 2) * 4 * ld_res + 4 * i + (j & 3);
+}
 
 // One thread per row i, cols_per_block columns per pass: C'_ij from its residues, then C_ij.
 __global__ void __launch_bounds__(256) crt_reconstruct_kernel(const __grid_constant__ CrtRecParams R) {
@@ -824,7 +831,7 @@ __global__ void __launch_bounds__(256) crt_reconstruct_kernel(const __grid_const
     int64_t jb, je;
     triangle_cols(R.uplo, i, j0, j0 + cpb < R.ncols ? j0 + cpb : R.ncols, jb, je);
     for (int64_t j = jb; j < je; ++j) {
-      const uint8_t* rp = R.res + j * R.ld_res + i;
+      const uint8_t* rp = R.res + residue_index(i, j, R.ld_res);
       unsigned long long acc[kCrtLimbs] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
       // unrolled over the largest modulus count: the weights are immediate constant-bank operands
 #pragma unroll
@@ -893,7 +900,8 @@ __global__ void __launch_bounds__(256) crt_reconstruct_kernel(const __grid_const
       crt_store(sc, i, j, negative ? -d : d, shift, e_acc, v_acc);
     }
   }
-  if (R.err_sq) crt_reduce_energies(R, e_acc, v_acc);
+  __shared__ double red[2][8];
+  if (R.err_sq) crt_reduce_energies(R, e_acc, v_acc, red);
 }
 
 // C' from the residues rc[0..N) of one entry (N <= 16): RN(|C'|) = d 2^shift, returns the
@@ -970,14 +978,14 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct128_kernel(const __grid
     // software pipeline: the residues of column j+1 are loaded while column j is reduced
     uint32_t rn[N];
 #pragma unroll
-    for (int l = 0; l < N; ++l) rn[l] = res[jb * ld_res + i + l * plane];
+    for (int l = 0; l < N; ++l) rn[l] = res[residue_index(i, jb, ld_res) + l * plane];
     for (int64_t j = jb; j < j1; ++j) {
       uint32_t rc[N];
 #pragma unroll
       for (int l = 0; l < N; ++l) rc[l] = rn[l];
       if (j + 1 < j1) {
 #pragma unroll
-        for (int l = 0; l < N; ++l) rn[l] = res[(j + 1) * ld_res + i + l * plane];
+        for (int l = 0; l < N; ++l) rn[l] = res[residue_index(i, j + 1, ld_res) + l * plane];
       }
       double d;
       int shift;
@@ -985,7 +993,8 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct128_kernel(const __grid
       crt_store(sc, i, j, negative ? -d : d, shift, e_acc, v_acc);
     }
   }
-  if (EST) crt_reduce_energies(R, e_acc, v_acc);
+  __shared__ double red[2][8];
+  if (EST) crt_reduce_energies(R, e_acc, v_acc, red);
 }
 
 // RN(|R| 2^escale) with its sign, for R = (r3 r2 r1 r0) in [-P/2, P/2) (128-bit two's
@@ -1180,33 +1189,31 @@ __device__ __forceinline__ void mma_u8_16x8x16(int (&d)[4], uint32_t a0, uint32_
       : "r"(a0), "r"(a1), "r"(b0), "r"(0));
 }
 
-// Rows i0 .. i0+31 of one column per warp.  The warp streams the residues of its columns
-// through its own ring of kRecStages shared-memory slots (a column's 16 moduli x 32 rows, 512
-// bytes), kRecStages - 1 columns ahead, with 16-byte cp.async copies (lane L copies rows
-// 16 (L & 1) .. +15 of modulus L / 2), so that no registers hold loads in flight.  Lane
-// (g, c) = (lane / 4, lane % 4) reads moduli 4c .. 4c+3 at rows i0 + 4g .. i0 + 4g + 3 (one
-// 32-bit word per modulus; the slot's words are swizzled, word w at w ^ ((w >> 2) & 0x18), so
-// that these reads hit 32 distinct banks) and transposes the 4 x 4 bytes so that each word
-// holds the four moduli of one row (the A fragment rows).  The MMAs leave with lane (g, c) the
-// byte sums T_2c, T_2c+1, T_8+2c, T_9+2c of those four rows.  The lane packs them in pairs,
-// X_c = T_2c + 2^8 T_2c+1 and Y_c = T_8+2c + 2^8 T_9+2c (each below 2^29), and the warp passes
-// the pairs through its own rows of shared memory (two buffers, alternating by column, so that
-// writing one never waits for the reads of the other), so that lane L reads the eight of row
-// i0 + L and forms S in four 32-bit-aligned columns, X_0 + 2^16 X_1, X_2 + 2^16 X_3,
-// Y_0 + 2^16 Y_1, Y_2 + 2^16 Y_3; the tail (crt_finish_small) and the store follow.  Bit for
-// bit the per-row kernel: S is the same integer and it is rounded the same way.
-constexpr int kRecStageStride = 10;  // words per staged row: X_0 Y_0 .. X_3 Y_3 and 2 of padding
-constexpr int kRecStages = 4;        // columns of residues in each warp's ring
-__device__ __forceinline__ int rec_swizzle(int w) { return w ^ ((w >> 2) & 0x18); }
+// Rows i0 .. i0+31 of four columns at a time (a group) per warp.  The warp streams the residues of
+// its groups through its own ring of kRecStages shared-memory slots (16 moduli x 32 rows x 4
+// columns, 2 KB), kRecStages - 1 groups ahead, with 16-byte cp.async copies (8 lanes per modulus:
+// 128 contiguous bytes), so that no registers hold loads in flight.  The group is reduced in four
+// steps of 8 rows.  Lane (g, c) = (lane / 4, lane % 4) reads moduli 4c .. 4c+3 of row 8s + g (one
+// 32-bit word per modulus, its four columns; the slot's row bits 3-4 are XORed with c so that these
+// reads hit 32 distinct banks) and transposes the 4 x 4 bytes so that each word holds the four
+// moduli of one column (the A fragment rows).  The MMAs leave with lane (g, c) the byte sums T_2c,
+// T_2c+1, T_8+2c, T_9+2c of those four entries.  The lane packs them in pairs, X_c = T_2c + 2^8
+// T_2c+1 and Y_c = T_8+2c + 2^8 T_9+2c (each below 2^29), and the warp passes the pairs through its
+// own rows of shared memory (two buffers, alternating by step, so that writing one never waits for
+// the reads of the other), so that lane L reads the eight of row 8s + L % 8, column L / 8 and forms
+// S in four 32-bit-aligned columns, X_0 + 2^16 X_1, X_2 + 2^16 X_3, Y_0 + 2^16 Y_1, Y_2 + 2^16 Y_3;
+// the tail (crt_finish_small) and the store follow.  Bit for bit the per-row kernel: S is the same
+// integer and it is rounded the same way.
+constexpr int kRecStages = 2;  // groups of residues in each warp's ring
 template <int N, bool EST>
 __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __grid_constant__ CrtRecParams R) {
   static_assert(N >= kCrtMinModuli && N <= 16, "16 moduli per MMA K step");
-  __shared__ __align__(16) uint32_t stage[8][2][32 * kRecStageStride];
-  __shared__ __align__(16) uint32_t ring[8][kRecStages][128];
+  __shared__ __align__(16) uint32_t stage[8][2][32 * 8];
+  __shared__ __align__(16) uint32_t ring[8][kRecStages][16 * 32];
   if (R.skip_if_flag && *R.skip_if_flag) return;
-  uint32_t (*const wstage)[32 * kRecStageStride] = stage[threadIdx.x >> 5];
+  uint32_t (*const wstage)[32 * 8] = stage[threadIdx.x >> 5];
   int sbuf = 0;
-  const uint32_t (*const wring)[128] = ring[threadIdx.x >> 5];
+  const uint32_t (*const wring)[16 * 32] = ring[threadIdx.x >> 5];
   CrtStoreCtx sc = store_ctx(R);
   const uint8_t* const res = R.res;
   const int64_t ld_res = R.ld_res, plane = R.plane, m = R.m, ncols = R.ncols;
@@ -1215,7 +1222,7 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
   const int lane = int(threadIdx.x & 31);
   const int g = lane >> 2, c = lane & 3;
   const int64_t i0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) - lane;  // the warp's first row
-  const int64_t i = i0 + lane;                                                   // this lane's row
+  const int64_t i = i0 + lane;                                                   // this lane's row of the estimate
   // B fragments: byte (8h + g) of W_4c .. W_4c+3
   uint32_t bfrag[2];
 #pragma unroll
@@ -1230,16 +1237,21 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
     }
     bfrag[h] = w;
   }
-  const int mu_i = i < m ? sc.mu_a[i] : kCrtZeroRow;
   double e_acc = 0.0, v_acc = 0.0;
-  // copies: lane L takes rows 16 (L & 1) .. +15 of modulus L / 2 (16-byte aligned: the planes,
-  // the leading dimension and i0 are multiples of 16)
-  const bool copier = (lane >> 1) < N;
-  const uint8_t* const cbase = res + i0 + 16 * (lane & 1) + int64_t(lane >> 1) * plane;
-  const uint32_t cdst = smem_u32(&wring[0][rec_swizzle(8 * (lane >> 1) + 4 * (lane & 1))]);
-  int rword[4];  // this lane's four words of a slot
+  // copy q of lane L: rows 4 (L % 8) .. +3 of modulus 4q + L / 8 (16-byte aligned: the planes, the
+  // leading dimension and i0 are multiples of 4 words)
+  const uint8_t* const cbase = res + 4 * i0 + 16 * (lane & 7) + int64_t(lane >> 3) * plane;
+  auto copy_group = [&](int slot, int64_t grp) {
+    const uint8_t* src = cbase + grp * 4 * ld_res;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) rword[k] = rec_swizzle(8 * (4 * c + k) + g);
+    for (int q = 0; q < (N + 3) / 4; ++q) {
+      const int l = 4 * q + (lane >> 3);
+      if (4 * q + 4 <= N || l < N) cp_async_16(smem_u32(&wring[slot][l * 32 + ((4 * (lane & 7)) ^ (8 * q))]), src + 4 * q * plane);
+    }
+  };
+  // this lane's words of a stage buffer (pair p of row r at r * 8 + 2 (p ^ (r / 4) % 4): the writes
+  // and the reads of a half-warp hit distinct banks)
+  const int e_row = lane & 7, e_col = lane >> 3;  // the entry this lane finishes
   const int cpb = R.cols_per_block;
   const int64_t jstep = int64_t(gridDim.y) * cpb;
   for (int64_t j0 = int64_t(blockIdx.y) * cpb; i0 < m && j0 < ncols; j0 += jstep) {
@@ -1253,6 +1265,7 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
       // sum_j 2^(-2(nu_j - nu_min)): the column sum is the same for every row of the warp, so
       // lane t takes column jb + t (at most kRecCols of them) and the warp adds them up
       const int cnt = int(j1 - jb);
+      const int mu_i = i < m ? sc.mu_a[i] : kCrtZeroRow;
       const int nu = lane < cnt ? sc.mu_b[jb + lane] : kCrtZeroRow;
       const bool nz = nu != kCrtZeroRow;
       const int nu_min = __reduce_min_sync(0xffffffffu, nz ? nu : INT_MAX);
@@ -1261,85 +1274,88 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
       if (mu_i != kCrtZeroRow && nu_min != INT_MAX) e_acc = fma(exp2_int(2 * (sc.b - mu_i - nu_min)), t, e_acc);
     }
-    // one commit group per column (empty past j1), so that waiting for all but the newest
-    // kRecStages - 1 groups leaves column j landed; every lane reads a slot before the
+    // one commit group per group of columns (empty past the last), so that waiting for all but the
+    // newest leaves the current one landed; every lane reads a slot's last words before the
     // __syncwarp that precedes any copy into it
-    // (32-bit column offsets jj from jb and pointers stepped by their leading dimensions)
-    const int cnt = int(j1 - jb);
-    const uint8_t* csrc = cbase + jb * ld_res;
-#pragma unroll
-    for (int t = 0; t < kRecStages - 1; ++t, csrc += ld_res) {
-      if (copier && t < cnt) cp_async_16(cdst + t * 512u, csrc);
+    const int64_t g0 = jb >> 2;
+    const int groups = int(((j1 + 3) >> 2) - g0);
+    copy_group(0, g0);
+    cp_async_commit();
+    for (int t = 0; t < groups; ++t) {
+      if (t + 1 < groups) copy_group((t + 1) & 1, g0 + t + 1);
       cp_async_commit();
-    }
-    double* cp = sc.C + jb * sc.ldc + i;
-    const int32_t* const nup = sc.mu_b + jb;
-    int slot = 0;
-    for (int jj = 0; jj < cnt; ++jj, csrc += ld_res, cp += sc.ldc) {
-      {
-        const int sn = slot == 0 ? kRecStages - 1 : slot - 1;  // (slot + kRecStages - 1) % kRecStages
-        if (copier && jj + kRecStages - 1 < cnt) cp_async_16(cdst + uint32_t(sn) * 512u, csrc);
-        cp_async_commit();
-      }
       cp_async_wait<kRecStages - 1>();
       __syncwarp();
-      uint32_t w[4];
+      const uint32_t* const slot = wring[t & 1];
+      const int64_t j = 4 * (g0 + t) + e_col;
+      const bool col_ok = j >= jb && j < j1;
+      const int nu_j = col_ok ? sc.mu_b[j] : 0;
+      double* cp = sc.C + j * sc.ldc + i0 + e_row;
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s, cp += 8) {
+        __syncwarp();  // lanes that kept nothing wait here for the MMAs
+        uint32_t w[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) w[k] = 4 * c + k < N ? wring[slot][rword[k]] : 0u;
-      slot = slot == kRecStages - 1 ? 0 : slot + 1;
-      // 4 x 4 byte transpose: w[k] byte e (modulus 4c+k, row 4g+e) -> v[e] byte k
-      const uint32_t t0 = __byte_perm(w[0], w[1], 0x5140), t1 = __byte_perm(w[0], w[1], 0x7362);
-      const uint32_t t2 = __byte_perm(w[2], w[3], 0x5140), t3 = __byte_perm(w[2], w[3], 0x7362);
-      const uint32_t v0 = __byte_perm(t0, t2, 0x5410), v1 = __byte_perm(t0, t2, 0x7632);
-      const uint32_t v2 = __byte_perm(t1, t3, 0x5410), v3 = __byte_perm(t1, t3, 0x7632);
-      // rows 4g+0 / 4g+1 (MMA row slots g / g+8), then rows 4g+2 / 4g+3; bytes 0..7, then 8..15
-      int d0[4], d1[4], d2[4], d3[4];  // the byte sums start from zero (C operand 0)
-      mma_u8_16x8x16(d0, v0, v1, bfrag[0]);
-      mma_u8_16x8x16(d1, v0, v1, bfrag[1]);
-      mma_u8_16x8x16(d2, v2, v3, bfrag[0]);
-      mma_u8_16x8x16(d3, v2, v3, bfrag[1]);
-      // (X_c, Y_c) of rows 4g+e to words 2c, 2c+1 of those rows (stride 10 words: the 64-bit
-      // writes of a half-warp and the 64-bit reads below hit distinct banks)
-      uint32_t* w0 = wstage[sbuf] + (4 * g) * kRecStageStride + 2 * c;
-      *reinterpret_cast<uint2*>(w0) = make_uint2(uint32_t(d0[0]) + uint32_t(d0[1]) * 256u,
-                                                 uint32_t(d1[0]) + uint32_t(d1[1]) * 256u);
-      *reinterpret_cast<uint2*>(w0 + kRecStageStride) = make_uint2(uint32_t(d0[2]) + uint32_t(d0[3]) * 256u,
-                                                                   uint32_t(d1[2]) + uint32_t(d1[3]) * 256u);
-      *reinterpret_cast<uint2*>(w0 + 2 * kRecStageStride) = make_uint2(uint32_t(d2[0]) + uint32_t(d2[1]) * 256u,
-                                                                       uint32_t(d3[0]) + uint32_t(d3[1]) * 256u);
-      *reinterpret_cast<uint2*>(w0 + 3 * kRecStageStride) = make_uint2(uint32_t(d2[2]) + uint32_t(d2[3]) * 256u,
-                                                                       uint32_t(d3[2]) + uint32_t(d3[3]) * 256u);
-      __syncwarp();
-      // this lane's row: S = sum_b T_b 2^(8b) as four 32-bit-aligned columns (each < 2^46)
-      const uint32_t* rrow = wstage[sbuf] + lane * kRecStageStride;
-      sbuf ^= 1;
-      const uint2 q0 = *reinterpret_cast<const uint2*>(rrow), q1 = *reinterpret_cast<const uint2*>(rrow + 2);
-      const uint2 q2 = *reinterpret_cast<const uint2*>(rrow + 4), q3 = *reinterpret_cast<const uint2*>(rrow + 6);
-      const unsigned long long acc[4] = {static_cast<unsigned long long>(q1.x) * 65536ull + q0.x,
-                                         static_cast<unsigned long long>(q3.x) * 65536ull + q2.x,
-                                         static_cast<unsigned long long>(q1.y) * 65536ull + q0.y,
-                                         static_cast<unsigned long long>(q3.y) * 65536ull + q2.y};
-      const int64_t j = jb + jj;
-      const bool keep = i < m && (uplo == 0 || (uplo == 1 ? i <= j : i >= j));
-      if (!keep) continue;
-      const int nu_j = nup[jj];
-      const double v = __dmul_rn(sc.alpha, crt_finish_small<N>(acc, P_inv32, -mu_i - nu_j));
-      if (EST) {
-        if (uplo != 0 && mu_i != kCrtZeroRow && nu_j != kCrtZeroRow) e_acc += exp2_int(2 * (sc.b - mu_i - nu_j));
-        v_acc += v * v;
-      }
-      if (sc.write_c) {
-        if (sc.beta == 0.0) {
-          *cp = v;
-        } else {
-          const double old = *cp;
-          if (sc.save) sc.save[j * sc.ld_save + i] = old;
-          *cp = __fma_rn(sc.beta, old, v);
+        for (int k = 0; k < 4; ++k) w[k] = 4 * c + k < N ? slot[(4 * c + k) * 32 + ((8 * s + g) ^ (8 * c))] : 0u;
+        // 4 x 4 byte transpose: w[k] byte e (modulus 4c+k, column e) -> v[e] byte k
+        const uint32_t t0 = __byte_perm(w[0], w[1], 0x5140), t1 = __byte_perm(w[0], w[1], 0x7362);
+        const uint32_t t2 = __byte_perm(w[2], w[3], 0x5140), t3 = __byte_perm(w[2], w[3], 0x7362);
+        const uint32_t v0 = __byte_perm(t0, t2, 0x5410), v1 = __byte_perm(t0, t2, 0x7632);
+        const uint32_t v2 = __byte_perm(t1, t3, 0x5410), v3 = __byte_perm(t1, t3, 0x7632);
+        // columns 0 / 1 (MMA row slots g / g+8), then columns 2 / 3; bytes 0..7, then 8..15
+        int d0[4], d1[4], d2[4], d3[4];  // the byte sums start from zero (C operand 0)
+        mma_u8_16x8x16(d0, v0, v1, bfrag[0]);
+        mma_u8_16x8x16(d1, v0, v1, bfrag[1]);
+        mma_u8_16x8x16(d2, v2, v3, bfrag[0]);
+        mma_u8_16x8x16(d3, v2, v3, bfrag[1]);
+        // (X_c, Y_c) of column e of this row to stage row 8e + g
+        uint32_t* const st = wstage[sbuf];
+        auto put = [&](int e, int xlo, int xhi, int ylo, int yhi) {
+          const int r = 8 * e + g;
+          *reinterpret_cast<uint2*>(st + r * 8 + 2 * (c ^ ((r >> 2) & 3))) =
+              make_uint2(uint32_t(xlo) + uint32_t(xhi) * 256u, uint32_t(ylo) + uint32_t(yhi) * 256u);
+        };
+        put(0, d0[0], d0[1], d1[0], d1[1]);
+        put(1, d0[2], d0[3], d1[2], d1[3]);
+        put(2, d2[0], d2[1], d3[0], d3[1]);
+        put(3, d2[2], d2[3], d3[2], d3[3]);
+        __syncwarp();
+        // this lane's entry: S = sum_b T_b 2^(8b) as four 32-bit-aligned columns (each < 2^46)
+        const uint32_t* const rrow = st + lane * 8;
+        sbuf ^= 1;
+        const int sw = 2 * ((lane >> 2) & 3);
+        const uint2 q0 = *reinterpret_cast<const uint2*>(rrow + (0 ^ sw)), q1 = *reinterpret_cast<const uint2*>(rrow + (2 ^ sw));
+        const uint2 q2 = *reinterpret_cast<const uint2*>(rrow + (4 ^ sw)), q3 = *reinterpret_cast<const uint2*>(rrow + (6 ^ sw));
+        const unsigned long long acc[4] = {static_cast<unsigned long long>(q1.x) * 65536ull + q0.x,
+                                           static_cast<unsigned long long>(q3.x) * 65536ull + q2.x,
+                                           static_cast<unsigned long long>(q1.y) * 65536ull + q0.y,
+                                           static_cast<unsigned long long>(q3.y) * 65536ull + q2.y};
+        const int64_t ie = i0 + 8 * s + e_row;
+        const bool keep = col_ok && ie < m && (uplo == 0 || (uplo == 1 ? ie <= j : ie >= j));
+        if (!keep) continue;
+        const int mu_e = sc.mu_a[ie];
+        const double v = __dmul_rn(sc.alpha, crt_finish_small<N>(acc, P_inv32, -mu_e - nu_j));
+        if (EST) {
+          if (uplo != 0 && mu_e != kCrtZeroRow && nu_j != kCrtZeroRow) e_acc += exp2_int(2 * (sc.b - mu_e - nu_j));
+          v_acc += v * v;
+        }
+        if (sc.write_c) {
+          if (sc.beta == 0.0) {
+            *cp = v;
+          } else {
+            const double old = *cp;
+            if (sc.save) sc.save[j * sc.ld_save + ie] = old;
+            *cp = __fma_rn(sc.beta, old, v);
+          }
         }
       }
     }
+    __syncwarp();  // the slots are read before the next pass copies into them
   }
-  if (EST) crt_reduce_energies(R, e_acc, v_acc);
+  if (EST) {
+    __syncthreads();
+    crt_reduce_energies(R, e_acc, v_acc, *reinterpret_cast<double(*)[2][8]>(&stage[0][0][0]));
+  }
 }
 
 // Split-K: residue planes (l, s), s = 0 .. splits-1, of modulus l added modulo p_l into
@@ -1537,15 +1553,18 @@ cudaError_t launch_crt_reconstruct(const CrtReconstructArgs& args, cudaStream_t 
   R.save = args.save;
   R.ld_save = args.ld_save;
   R.uplo = args.uplo;
-  // the tensor-core sum: whole warps of 32 rows copy the residue planes 16 bytes at a time, so
-  // the planes must be 16-byte aligned and hold every row of those warps
+  // the tensor-core sum: whole warps of 32 rows copy the residue planes 16 bytes at a time and
+  // four columns together, so the planes must be 16-byte aligned, hold every row of those warps
+  // and whole groups of columns
   const bool mma = args.moduli >= kCrtMinModuli && args.moduli <= 16 && reinterpret_cast<uintptr_t>(args.cres) % 16 == 0 &&
-                   args.ld_res % 32 == 0 && args.plane % 16 == 0 && args.ld_res >= (args.m + 31) / 32 * 32;
+                   args.ld_res % 32 == 0 && args.plane % 16 == 0 && args.ld_res >= (args.m + 31) / 32 * 32 &&
+                   args.plane >= (args.n + 3) / 4 * 4 * args.ld_res;
   const int64_t rows_per_block = 256;
   const unsigned gx = unsigned((args.m + rows_per_block - 1) / rows_per_block);
-  // up to kRecCols columns per block, fewer while the grid is under ~4 blocks per SM
-  int64_t cpb = int64_t(gx) * args.n / (4 * 148);
-  cpb = cpb < 1 ? 1 : (cpb > kRecCols ? kRecCols : cpb);
+  // whole groups of four columns: up to kRecCols per block while that leaves about three rounds of
+  // four blocks per SM, so that a block's set-up and first copies are spread over many columns
+  int64_t cpb = kRecCols;
+  while (cpb > 4 && int64_t(gx) * args.n < cpb * 3 * 4 * 148) cpb /= 2;
   R.cols_per_block = int(cpb);
   const int64_t groups = (args.n + cpb - 1) / cpb;
   const unsigned gy = unsigned(groups < 65535 ? groups : 65535);

@@ -143,14 +143,14 @@ struct CrtGemmArgs {
   uint32_t* status;
   int tile_n;  // 256, kTilePair or kTileWide
   int num_sms;
-  uint8_t* cres;   // [moduli][n_pad][ld_res] residues of C' (uint8 in [0, p))
+  uint8_t* cres;   // [moduli][n_pad/4][ld_res][4] residues of C' (uint8 in [0, p)): four columns a word
   int64_t ld_res;  // = a.rows_pad
   const int* tile_list = nullptr;  // device: the output tiles to compute (null: all)
   int num_listed = 0;
   int tri_k = 0;  // triangular operand whose zero K blocks are skipped: 1/2 = op(A) lower/upper,
                   // 3/4 = op(B) lower/upper (0: dense)
   // split-K: every (tile, modulus) is computed as `splits` K ranges, each into its own residue
-  // plane: cres is [moduli][splits][n_pad][ld_res], merged by launch_crt_merge_splits (dense
+  // plane: cres is [moduli][splits][n_pad/4][ld_res][4], merged by launch_crt_merge_splits (dense
   // operands, no tile list, splits <= the K blocks).  1: none.
   int splits = 1;
   int group_m = 0;  // row tiles per raster group (0: the process-wide tuning)
@@ -237,7 +237,7 @@ template <typename T>
 cudaError_t launch_tri_block_multiply(const T* E, int64_t er, int64_t ec, int nb, bool lower, bool unit, T* X,
                                       int64_t vs, int64_t ts, int64_t count, cudaStream_t stream);
 constexpr int kPanelMax = 256;  // largest diagonal block launch_tri_panel_solve takes
-constexpr int kPanelVecs = 64;  // vectors per CTA of launch_tri_panel_solve
+constexpr int kPanelVecs = 64;  // vectors per CTA of launch_tri_panel_solve_complex
 // x := E^-1 x for `count` vectors laid out as for launch_tri_block_multiply, E the nb x nb
 // (nb <= kPanelMax) triangle, by blocked substitution.
 template <typename T>

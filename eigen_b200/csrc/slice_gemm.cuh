@@ -89,7 +89,7 @@ struct SliceGemmParams {
   uint32_t* status;
   int group_m;           // row-tiles per raster group (>= tiles_m: column-major tile order)
   int crt;               // 1: CRT mode (unit t = modulus t, one slice pair (t, t))
-  uint8_t* residues;     // CRT: [moduli][cols][ld_res] residue planes (uint8 in [0, p))
+  uint8_t* residues;     // CRT: [moduli][cols/4][ld_res][4] residue planes (uint8 in [0, p))
   int64_t ld_res;        // CRT: rows of one residue plane (padded m)
   const int* tile_list;  // CRT: the tiles to compute (indices of the full raster), or null for all
   int num_listed;        // CRT: entries of tile_list
@@ -380,11 +380,10 @@ __device__ __forceinline__ void slice_mma(uint8_t* smem, uint64_t* full, uint64_
   int buf = 0;
   uint32_t tphase = 0u;  // bit b: phase of accumulator buffer b
   bool ok = true;
-  // the MMAs of one stage into accumulator d_tmem (fresh: the first overwrites it)
-  auto consume = [&](uint32_t d_tmem, bool fresh) -> bool {
-    const int stage = int(consumed % STAGES);
-    if (!mbar_wait(&full[stage], (consumed / STAGES) & 1u, abort_flag, P.status, P.wait_limit_ns)) return false;
-    tc_fence_after();
+  // the MMAs of row tiles [mt0, mt1) of the stage used `at` into accumulator d_tmem (fresh: the
+  // first overwrites it)
+  auto stage_mmas = [&](uint32_t at, uint32_t d_tmem, bool fresh, int mt0, int mt1) {
+    const int stage = int(at % STAGES);
     const uint64_t adesc = make_sw128_kmajor_desc(smem_u32(smem + L::kAOff + stage * L::kABytes));
     const uint64_t bdesc = make_sw128_kmajor_desc(smem_u32(smem + L::kBOff + stage * L::kBBytes));
 #pragma unroll
@@ -393,6 +392,7 @@ __device__ __forceinline__ void slice_mma(uint8_t* smem, uint64_t* full, uint64_
       const uint64_t bd = bdesc + uint64_t(2 * kk);
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
+        if (mt < mt0 || mt >= mt1) continue;
         // row tile mt: 128 rows of 128 bytes further on (descriptor addresses count 16 bytes);
         // its accumulator is the TMEM region of columns mt * BN ..
         const uint64_t ad = adesc + uint64_t(mt * (kSliceBM * kSliceKBytes / 16)) + uint64_t(2 * kk);
@@ -410,7 +410,14 @@ __device__ __forceinline__ void slice_mma(uint8_t* smem, uint64_t* full, uint64_
         }
       }
     }
-    commit_to<PAIR>(&empty[stage]);
+  };
+  // the next stage, once it has landed; its slot is handed back when its MMAs are done
+  auto consume = [&](uint32_t d_tmem, bool fresh) -> bool {
+    if (!mbar_wait(&full[consumed % STAGES], (consumed / STAGES) & 1u, abort_flag, P.status, P.wait_limit_ns))
+      return false;
+    tc_fence_after();
+    stage_mmas(consumed, d_tmem, fresh, 0, MT);
+    commit_to<PAIR>(&empty[consumed % STAGES]);
     ++consumed;
     return true;
   };
@@ -465,7 +472,35 @@ __device__ __forceinline__ void slice_mma(uint8_t* smem, uint64_t* full, uint64_
           }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + uint32_t(buf * BN);
-          for (int f = u0; f < u1 && ok; ++f) ok = consume(d_tmem, f == u0);
+          int f = u0;
+          if constexpr (MT == 2) {
+            // one accumulator fills the TMEM, and the epilogue empties its row tiles one after
+            // the other: while row tile 1 still drains, row tile 0 takes the first stages
+            const int most = u1 - u0 < STAGES ? u1 - u0 : STAGES;
+            int lead = 0;
+            while (lead < most && !mbar_test_wait(&tempty[1], (tphase & 1u) ^ 1u)) {
+              const uint32_t at = consumed + uint32_t(lead);
+              if (!mbar_wait(&full[at % STAGES], (at / STAGES) & 1u, abort_flag, P.status, P.wait_limit_ns)) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+              stage_mmas(at, d_tmem, lead == 0, 0, 1);
+              ++lead;
+            }
+            if (!ok) break;
+            if (!mbar_wait(&tempty[1], (tphase & 1u) ^ 1u, abort_flag, P.status, P.wait_limit_ns)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            for (int i = 0; i < lead; ++i, ++f) {
+              stage_mmas(consumed, d_tmem, i == 0, 1, 2);
+              commit_to<PAIR>(&empty[consumed % STAGES]);
+              ++consumed;
+            }
+          }
+          for (; f < u1 && ok; ++f) ok = consume(d_tmem, f == u0);
           if (!ok) break;
           commit_to<PAIR>(&tfull[buf]);
           tphase ^= 1u << buf;
@@ -594,33 +629,66 @@ __device__ __forceinline__ void ozaki_epilogue(uint32_t tmem_base, uint64_t* tfu
 
 // x mod p for a 32-bit x and p <= 256, with m = floor((2^32 - 1) / p): p m >= 2^32 - p, so
 // x/p - x m / 2^32 <= x / 2^32 < 1 and the estimate q = umulhi(x, m) is at most one short
-// of floor(x / p): one conditional subtraction finishes it.
+// of floor(x / p): one conditional subtraction finishes it (r - p wraps above r when r < p).
 __device__ __forceinline__ uint32_t mod_small(uint32_t x, uint32_t p, uint32_t m) {
   const uint32_t r = x - __umulhi(x, m) * p;
-  return r >= p ? r - p : r;
+  return min(r, r - p);
 }
 
-// CRT: unit t is modulus p_t; every INT32 product entry is reduced to [0, p_t) and stored
-// as one byte of residue plane t (column-major, ld_res).  K beyond one unit comes in
+// 32 accumulator columns of one row reduced mod p, four to a word: word q holds columns 4q ..
+// 4q + 3 and goes to dst + q * step.  `add`: onto the residues already there, mod p.
+__device__ __forceinline__ void store_residue_words(const uint32_t (&r)[32], uint32_t bias, uint32_t pm, uint32_t magic,
+                                                    uint8_t* dst, int64_t step, bool add) {
+  if (add) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q, dst += step) {
+      const uint32_t old = *reinterpret_cast<const uint32_t*>(dst);
+      uint32_t w = 0u;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t v = mod_small(r[4 * q + e] + bias, pm, magic) + ((old >> (8 * e)) & 0xFFu);
+        w |= min(v, v - pm) << (8 * e);
+      }
+      *reinterpret_cast<uint32_t*>(dst) = w;
+    }
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q, dst += step) {
+    uint32_t x[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[e] = mod_small(r[4 * q + e] + bias, pm, magic);
+    *reinterpret_cast<uint32_t*>(dst) = __byte_perm(x[0] + x[1] * 256u, x[2] + x[3] * 256u, 0x5410);
+  }
+}
+
+// CRT: unit t is modulus p_t; every INT32 product entry is reduced to [0, p_t) and stored as one
+// byte of residue plane t: [cols/4][ld_res][4], four neighbouring columns of a row in one word, so
+// that a warp (32 rows) writes 128 contiguous bytes per store.  K beyond one unit comes in
 // further chunks whose residues are added mod p_t.
-// MT = 2: warp group g = (warp - 2) / 4 drains row tile g % 2 (TMEM columns (g % 2) * BN ..)
-// and its columns (g / 2) * kCols ..; the accumulator has a single buffer then.
+//
+// MT = 2: the accumulator has a single buffer of two row tiles.  Every warp takes its columns of
+// row tile 0 into registers, hands that half of the TMEM back, reduces and stores, and then does
+// the same with row tile 1, so the MMAs of the next item start on row tile 0 after one TMEM read.
+// Bound by issue slots (about 6 instructions per entry) and hidden behind the MMAs; with byte
+// stores and both halves released together after the last reduction the MMAs waited about 6 us
+// per item (13 us of MMAs at K = 2048, 48 us at 8192).  With the reconstruction's four-column
+// groups, a call went from 342 to 316 us at 2048 and from 8.08 to 7.64 ms at 8192.
 template <int BN, int NW, bool PAIR, bool LISTED, int MT>
 __device__ __forceinline__ void crt_epilogue(uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty,
                                              volatile int* abort_flag, const SliceGemmParams& P) {
-  static_assert(NW % (4 * MT) == 0, "whole warp groups per row tile");
-  constexpr int kCols = BN * 4 * MT / NW;
-  static_assert(kCols % 32 == 0, "column slice");
+  static_assert(NW % 4 == 0, "whole warp groups");
+  constexpr int kCols = BN * 4 / NW;  // columns per warp (of each row tile)
+  static_assert(kCols % 32 == 0 && (MT == 1 || kCols == 64), "column slice; MT = 2 keeps it in registers");
   constexpr int kTileRows = PAIR ? 2 * kSliceBM : MT * kSliceBM;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int quad = warp & 3;
-  const int group = (warp - 2) >> 2;
-  const int region = group % MT;  // row tile within the CTA's tile
-  const int col_base = (group / MT) * kCols;
-  const int row = region * kSliceBM + quad * 32 + lane;
+  const int col_base = ((warp - 2) >> 2) * kCols;
+  const int row = quad * 32 + lane;
   const int nwork = num_work<LISTED>(P);
   const int row_base = PAIR ? int(cluster_ctarank()) * kSliceBM : 0;
   const int64_t plane = P.ld_res * int64_t(P.tiles_n) * BN;
+  const int64_t step = 4 * P.ld_res;  // from one word of a row to the next
   int buf = 0;
   uint32_t ephase = 0u;
   bool ok = true;
@@ -630,7 +698,6 @@ __device__ __forceinline__ void crt_epilogue(uint32_t tmem_base, uint64_t* tfull
     tile_coords(tile, P.tiles_m, P.tiles_n, P.group_m, tm, tn);
     const int64_t m0 = int64_t(tm) * kTileRows + row_base;
     const int64_t n0 = int64_t(tn) * BN + col_base;
-    const int64_t grow = m0 + row;
     for (int t = t_hi; t >= t_lo && ok; --t) {
       int p_lo, total;
       if (!diag_bounds(t, P.slices, P.num_kb, p_lo, total, true)) continue;
@@ -645,35 +712,42 @@ __device__ __forceinline__ void crt_epilogue(uint32_t tmem_base, uint64_t* tfull
       // multiple of p in [2^31 - 2^21, 2^31 - 2^21 + p), v + bias lies in [0, 2^32) and
       // (v + bias) mod p = v mod p: one reduction of an unsigned word, no sign handling
       const uint32_t bias = (0x7FE00000u + pm - 1u) / pm * pm;
-      uint8_t* rp = P.residues + (int64_t(t) * P.splits + split) * plane + grow;
+      // (the rows are padded to whole tiles, so every row of the tile has its place in the plane)
+      uint8_t* rp = P.residues + (int64_t(t) * P.splits + split) * plane + (n0 >> 2) * step + 4 * (m0 + row);
       for (int u0 = 0; u0 < total && ok; u0 += kMaxUnitKbCrt) {
         if (!mbar_wait(&tfull[buf], (ephase >> buf) & 1u, abort_flag, P.status, P.wait_limit_ns)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t taddr =
-            tmem_base + uint32_t((MT == 1 ? buf * BN : region * BN) + col_base) + (uint32_t(quad * 32) << 16);
+        const uint32_t taddr = tmem_base + uint32_t(col_base) + (uint32_t(quad * 32) << 16);
+        if constexpr (MT == 1) {
 #pragma unroll 1
-        for (int c = 0; c < kCols / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + uint32_t(c * 32), r);
-          tmem_ld_wait();
-          if (grow < P.ld_res) {
-            uint8_t* dst = rp + (n0 + c * 32) * P.ld_res;
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj, dst += P.ld_res) {
-              uint32_t res = mod_small(r[jj] + bias, pm, magic);
-              if (u0 > 0) {
-                res += *dst;
-                if (res >= pm) res -= pm;
-              }
-              *dst = uint8_t(res);
-            }
+          for (int c = 0; c < kCols / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(taddr + uint32_t(buf * BN + c * 32), r);
+            tmem_ld_wait();
+            pin_registers(r);
+            store_residue_words(r, bias, pm, magic, rp + c * 8 * step, step, u0 > 0);
+          }
+          tc_fence_before();
+          acc_release<PAIR>(&tempty[buf]);
+        } else {
+#pragma unroll 1
+          for (int mt = 0; mt < MT; ++mt) {
+            uint32_t r0[32], r1[32];
+            tmem_ld_32x32b_x32(taddr + uint32_t(mt * BN), r0);
+            tmem_ld_32x32b_x32(taddr + uint32_t(mt * BN + 32), r1);
+            tmem_ld_wait();
+            pin_registers(r0);
+            pin_registers(r1);
+            tc_fence_before();
+            acc_release<PAIR>(&tempty[mt]);
+            uint8_t* const dst = rp + 4 * kSliceBM * mt;
+            store_residue_words(r0, bias, pm, magic, dst, step, u0 > 0);
+            store_residue_words(r1, bias, pm, magic, dst + 8 * step, step, u0 > 0);
           }
         }
-        tc_fence_before();
-        acc_release<PAIR>(&tempty[buf]);
         ephase ^= 1u << buf;
         if constexpr (MT == 1) buf ^= 1;  // two accumulators alternate; MT = 2 fills the TMEM
       }
@@ -774,7 +848,8 @@ __global__ void __launch_bounds__(64 + 32 * NW, 1)
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
-      mbar_init(&tempty[i], (PAIR ? 2 : 1) * 32 * NW);  // every epilogue thread (of both CTAs)
+      // every epilogue thread (of both CTAs); one barrier per buffer, or per row tile for MT = 2
+      mbar_init(&tempty[i], (PAIR ? 2 : 1) * 32 * NW);
     }
     mbar_init(drain, 1);
     *abort_flag = 0;
