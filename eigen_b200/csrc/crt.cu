@@ -200,25 +200,50 @@ __device__ __forceinline__ double scale2(double x, int e) {
   return __dmul_rn(__dmul_rn(x, exp2_int(e1)), exp2_int(e - e1));
 }
 
+// The operands of one preparation pass (op(A) and op(B)^T, or one of them), walked by one launch
+// per step: tile t of a launch belongs to operand `t >= tiles[0]`.
+struct PrepOperand {
+  const double* X;  // element (r, l) at X[r*sr + l*sl], rows x cols
+  int64_t rows, cols, sr, sl;
+  int64_t rows_pad, k_pad, nchunks;
+  int32_t* chunk_e;
+  unsigned long long* chunk_s;
+  int32_t* mu;
+  int8_t* residues;
+};
+struct PrepArgs {
+  PrepOperand op[2];
+  unsigned tiles0;  // tiles of operand 0
+  unsigned tiles_l[2];  // tiles along K
+};
+// operand, row tile and K tile of a block
+__device__ __forceinline__ const PrepOperand& prep_tile(const PrepArgs& A, unsigned& tr, unsigned& tl) {
+  const bool second = blockIdx.x >= A.tiles0;
+  const unsigned t = second ? blockIdx.x - A.tiles0 : blockIdx.x, n = A.tiles_l[second ? 1 : 0];
+  tr = t / n;
+  tl = t % n;
+  return A.op[second ? 1 : 0];
+}
+
 // One read of the operand for everything the scale exponents need.  Per row r and 128-column
 // chunk c (columns 128c .. 128c+127 of op(X)^T's row, i.e. along K):
-//   * the chunk maximum: row maxima (atomicMax), the NaN/Inf flag, and the exponent-spread
-//     statistic of the configuration picker (the first 64 columns of every 512, as the
-//     digit-slice scan computes it);
+//   * the chunk maximum: the NaN/Inf flag, and the exponent-spread statistic of the configuration
+//     picker (the first 64 columns of every 512, as the digit-slice scan computes it);
 //   * e_c, the exponent of the chunk maximum, and the deterministic integer bound
 //     S_c = sum over nonzero x of ceil(rn(x'^2) 2^32) + 1, x' = x 2^-e_c (|x'| < 1); the +1
-//     covers the rounding of x'^2 and a product that underflows.
-// Every (row, chunk) record is written by exactly one thread group.
-__global__ void __launch_bounds__(kNormThreads) crt_scan_norm_kernel(const double* __restrict__ X, int64_t rows, int64_t cols,
-                                                            int64_t sr, int64_t sl, unsigned long long* maxbits,
-                                                            int32_t* __restrict__ chunk_e,
-                                                            unsigned long long* __restrict__ chunk_s,
-                                                            int64_t nchunks, int* nonfinite, double* spread) {
+//     covers the rounding of x'^2 and a product that underflows.  S_c = 0 marks a chunk without a
+//     nonzero finite entry; the row's exponent is the largest e_c of the others.
+// Every (row, chunk) record is written by exactly one thread group, so nothing needs clearing.
+__global__ void __launch_bounds__(kNormThreads) crt_scan_norm_kernel(const __grid_constant__ PrepArgs args,
+                                                                     int* nonfinite, double* spread) {
   __shared__ double tile[kNormRows][kNormCols + 1];
   __shared__ double spread_part[2][kNormThreads / 32];
-  const int64_t r0 = int64_t(blockIdx.y) * kNormRows;
-  const int64_t l0 = int64_t(blockIdx.x) * kNormCols;
-  load_tile<kNormRows, kNormCols, kNormThreads>(tile, X, r0, l0, rows, cols, sr, sl);
+  unsigned tr, tl;
+  const PrepOperand& O = prep_tile(args, tr, tl);
+  const int64_t rows = O.rows;
+  const int64_t r0 = int64_t(tr) * kNormRows;
+  const int64_t l0 = int64_t(tl) * kNormCols;
+  load_tile<kNormRows, kNormCols, kNormThreads>(tile, O.X, r0, l0, rows, O.cols, O.sr, O.sl);
   __syncthreads();
   // 8 threads per row, reduced with shuffles inside each 8-lane group; thread `sub` takes
   // columns sub, sub + 8, ..., so that the 8 lanes of a row read 8 consecutive words of the
@@ -276,11 +301,9 @@ __global__ void __launch_bounds__(kNormThreads) crt_scan_norm_kernel(const doubl
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (sub == 0 && r < rows) {
-    const int64_t c = int64_t(blockIdx.x);
-    chunk_e[r * nchunks + c] = e;
-    chunk_s[r * nchunks + c] = mb < kInfBitsCrt ? s : 0ull;
+    O.chunk_e[r * O.nchunks + tl] = e;
+    O.chunk_s[r * O.nchunks + tl] = mb < kInfBitsCrt ? s : 0ull;
     if (mb >= kInfBitsCrt) *nonfinite = 1;
-    if (mb) atomicMax(&maxbits[r], mb);
   }
   if (stat) {
     double chunk_spread = 0.0, chunk_count = 0.0;
@@ -316,24 +339,29 @@ __global__ void __launch_bounds__(kNormThreads) crt_scan_norm_kernel(const doubl
 
 // Scale exponent of each row: with e the row maximum's exponent, the chunk bounds fold into
 // S = sum_c ceil(S_c 4^(e_c - e)) (exact shifts), ||x||^2 <= S 2^(2e-32), S <= 2^L (L = bit
-// length of S-1), so 2^c >= ||x|| for c = e - 16 + ceil(L/2) and mu = b - c.
-__global__ void __launch_bounds__(256) crt_mu_kernel(const unsigned long long* __restrict__ maxbits,
-                                                     const int32_t* __restrict__ chunk_e,
-                                                     const unsigned long long* __restrict__ chunk_s, int64_t nchunks,
-                                                     int64_t rows, int64_t rows_pad, int b, int32_t* __restrict__ mu) {
-  // one warp per row: the lanes read consecutive chunk records
-  const int64_t r = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+// length of S-1), so 2^c >= ||x|| for c = e - 16 + ceil(L/2) and mu = b - c.  One warp per row of
+// either operand: the lanes read consecutive chunk records.
+__global__ void __launch_bounds__(256) crt_mu_kernel(const __grid_constant__ PrepArgs args, int b) {
+  int64_t r = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const bool second = r >= args.op[0].rows_pad;
+  if (second) r -= args.op[0].rows_pad;
+  const PrepOperand& O = args.op[second ? 1 : 0];
   const int lane = int(threadIdx.x & 31);
-  if (r >= rows_pad) return;  // whole warps
+  if (r >= O.rows_pad) return;  // whole warps
   int m = kCrtZeroRow;
-  const unsigned long long mb = r < rows ? maxbits[r] : 0ull;
-  if (mb != 0 && mb < kInfBitsCrt) {
-    const int e = frexp_exp(mb);
+  if (r < O.rows) {
+    const int64_t nchunks = O.nchunks;
+    const unsigned long long* const sp = O.chunk_s + r * nchunks;
+    const int32_t* const ep = O.chunk_e + r * nchunks;
+    int e = INT_MIN;
+    for (int64_t c = lane; c < nchunks; c += 32)
+      if (sp[c] != 0) e = max(e, ep[c]);
+    e = __reduce_max_sync(0xffffffffu, e);
     unsigned long long S = 0;
     for (int64_t c = lane; c < nchunks; c += 32) {
-      const unsigned long long sc = chunk_s[r * nchunks + c];
+      const unsigned long long sc = sp[c];
       if (sc == 0) continue;
-      const int sh = 2 * (e - chunk_e[r * nchunks + c]);
+      const int sh = 2 * (e - ep[c]);
       S += sh >= 64 ? 1ull : ((sc - 1) >> sh) + 1;  // ceil(sc / 2^sh), sc >= 1
     }
 #pragma unroll
@@ -343,7 +371,7 @@ __global__ void __launch_bounds__(256) crt_mu_kernel(const unsigned long long* _
       m = b - (e - 16 + (L + 1) / 2);
     }
   }
-  if (lane == 0) mu[r] = m;
+  if (lane == 0) O.mu[r] = m;
 }
 
 // Per-modulus constants: p, floor((2^32 - 1) / p) for mod_small, 2^21, 2^42, 2^63 and 2^32
@@ -514,22 +542,21 @@ __device__ __forceinline__ void store_residues_static(const SplitEntry (&e)[kSpl
 // A 32 x 128 tile per block: each warp takes a row at a time, four consecutive entries per
 // lane, so that every modulus plane receives 128 contiguous bytes per warp store.
 template <bool kWide, int NT>  // kWide: |t| may reach 2^63 (more than 16 moduli)
-__global__ void __launch_bounds__(kSplitThreadsCrt, 3) crt_split_kernel(
-    const double* __restrict__ X, int64_t rows, int64_t cols, int64_t sr, int64_t sl,
-    const int32_t* __restrict__ mu, int n, int8_t* __restrict__ residues, int64_t rows_pad, int64_t k_pad) {
+__global__ void __launch_bounds__(kSplitThreadsCrt, 3) crt_split_kernel(const __grid_constant__ PrepArgs args, int n) {
   static_assert(kSplitColsCrt == 32 * kSplitEntries, "a warp per tile row");
   __shared__ double tile[kSplitRowsCrt][kSplitColsCrt + 1];
   __shared__ int row_mu_s[kSplitRowsCrt];
-  const int64_t r0 = int64_t(blockIdx.y) * kSplitRowsCrt;
-  const int64_t l0 = int64_t(blockIdx.x) * kSplitColsCrt;
-  if (threadIdx.x < kSplitRowsCrt) {
-    const int64_t r = r0 + threadIdx.x;
-    row_mu_s[threadIdx.x] = mu[r];
-  }
-  load_tile<kSplitRowsCrt, kSplitColsCrt, kSplitThreadsCrt>(tile, X, r0, l0, rows, cols, sr, sl);
+  unsigned tr, tl;
+  const PrepOperand& O = prep_tile(args, tr, tl);
+  const int64_t r0 = int64_t(tr) * kSplitRowsCrt;
+  const int64_t l0 = int64_t(tl) * kSplitColsCrt;
+  const int64_t k_pad = O.k_pad;
+  int8_t* const residues = O.residues;
+  if (threadIdx.x < kSplitRowsCrt) row_mu_s[threadIdx.x] = O.mu[r0 + threadIdx.x];
+  load_tile<kSplitRowsCrt, kSplitColsCrt, kSplitThreadsCrt>(tile, O.X, r0, l0, O.rows, O.cols, O.sr, O.sl);
   __syncthreads();
   const int cb = int(threadIdx.x & 31) * kSplitEntries;
-  const size_t plane = size_t(rows_pad) * size_t(k_pad);
+  const size_t plane = size_t(O.rows_pad) * size_t(k_pad);
   constexpr int kRowsPerPass = kSplitThreadsCrt / 32;
 #pragma unroll 1
   for (int rr = int(threadIdx.x >> 5); rr < kSplitRowsCrt; rr += kRowsPerPass) {
@@ -1468,38 +1495,56 @@ void crt_triangle_tiles(int tile_n, int64_t rows_pad, int64_t cols_pad, int64_t 
   *count = c;
 }
 
-cudaError_t launch_crt_scan_norms(const StridedView<double>& x, const CrtOperand& op, int* nonfinite, double* spread,
-                                  cudaStream_t stream) {
-  cudaError_t e = cudaMemsetAsync(op.maxbits, 0, size_t(op.rows) * sizeof(uint64_t), stream);
-  if (e != cudaSuccess || x.rows == 0 || x.cols == 0) return e;
-  if (op.k_pad % kNormCols != 0) return cudaErrorInvalidValue;
-  dim3 grid(unsigned((x.cols + kNormCols - 1) / kNormCols), unsigned((x.rows + kNormRows - 1) / kNormRows));
-  if (grid.y > 65535u) return cudaErrorInvalidConfiguration;
-  crt_scan_norm_kernel<<<grid, kNormThreads, 0, stream>>>(x.ptr, x.rows, x.cols, x.sr, x.sl,
-                                                 reinterpret_cast<unsigned long long*>(op.maxbits), op.chunk_e,
-                                                 reinterpret_cast<unsigned long long*>(op.chunk_s),
-                                                 op.k_pad / kNormCols, nonfinite, spread);
+// The operands of a preparation step whose tiles are `rows` x `cols`; false when the tiles do not
+// fit a grid.  `padded`: the tiles cover the padded panel, else the operand's own extent.
+static bool prep_args(const CrtPrep& p, int rows, int cols, bool padded, PrepArgs& A, unsigned& blocks) {
+  int64_t total = 0;
+  for (int i = 0; i < 2; ++i) {
+    const int q = i < p.count ? i : 0;
+    const StridedView<double>& x = p.x[q];
+    const CrtOperand& op = p.op[q];
+    A.op[i] = PrepOperand{x.ptr, x.rows, x.cols, x.sr, x.sl, op.rows_pad, op.k_pad, op.k_pad / kNormCols, op.chunk_e,
+                          reinterpret_cast<unsigned long long*>(op.chunk_s), op.mu, op.residues};
+    const int64_t tl = padded ? op.k_pad / cols : (x.cols + cols - 1) / cols;
+    const int64_t tr = padded ? op.rows_pad / rows : (x.rows + rows - 1) / rows;
+    A.tiles_l[i] = unsigned(tl);
+    if (i < p.count) total += tr * tl;
+    if (i == 0) A.tiles0 = unsigned(total);
+    if (tr > 65535 || tl > 0x7FFFFFFF || total > 0x7FFFFFFF) return false;
+  }
+  blocks = unsigned(total);
+  return true;
+}
+
+cudaError_t launch_crt_scan_norms(const CrtPrep& p, int* nonfinite, double* spread, cudaStream_t stream) {
+  for (int i = 0; i < p.count; ++i)
+    if (p.op[i].k_pad % kNormCols != 0 || p.x[i].rows <= 0 || p.x[i].cols <= 0) return cudaErrorInvalidValue;
+  PrepArgs A;
+  unsigned blocks = 0;
+  if (!prep_args(p, kNormRows, kNormCols, false, A, blocks)) return cudaErrorInvalidConfiguration;
+  crt_scan_norm_kernel<<<blocks, kNormThreads, 0, stream>>>(A, nonfinite, spread);
   return cudaGetLastError();
 }
 
-cudaError_t launch_crt_split(const StridedView<double>& x, const CrtOperand& op, int moduli, cudaStream_t stream) {
-  if (moduli < 1 || moduli > op.nmax) return cudaErrorInvalidValue;
-  if (op.k_pad % kSplitColsCrt != 0 || op.rows_pad % kSplitRowsCrt != 0) return cudaErrorInvalidValue;
-  dim3 grid(unsigned(op.k_pad / kSplitColsCrt), unsigned(op.rows_pad / kSplitRowsCrt));
-  if (grid.y > 65535u) return cudaErrorInvalidConfiguration;
+cudaError_t launch_crt_split(const CrtPrep& p, int moduli, cudaStream_t stream) {
+  int64_t rows = 0;
+  for (int i = 0; i < p.count; ++i) {
+    if (moduli < 1 || moduli > p.op[i].nmax) return cudaErrorInvalidValue;
+    if (p.op[i].k_pad % kSplitColsCrt != 0 || p.op[i].rows_pad % kSplitRowsCrt != 0) return cudaErrorInvalidValue;
+    rows += p.op[i].rows_pad;
+  }
+  PrepArgs A;
+  unsigned blocks = 0;
+  if (!prep_args(p, kSplitRowsCrt, kSplitColsCrt, true, A, blocks)) return cudaErrorInvalidConfiguration;
+  if (p.count == 1) A.op[1].rows_pad = 0;  // no second operand
   const int b = crt_bits(moduli);
-  crt_mu_kernel<<<unsigned((op.rows_pad + 7) / 8), 256, 0, stream>>>(
-      reinterpret_cast<const unsigned long long*>(op.maxbits), op.chunk_e,
-      reinterpret_cast<const unsigned long long*>(op.chunk_s), op.k_pad / kNormCols, op.rows, op.rows_pad, b, op.mu);
+  crt_mu_kernel<<<unsigned((rows + 7) / 8), 256, 0, stream>>>(A, b);
   if (moduli == kCrtDefaultModuli && b <= 62)
-    crt_split_kernel<false, kCrtDefaultModuli><<<grid, kSplitThreadsCrt, 0, stream>>>(
-        x.ptr, x.rows, x.cols, x.sr, x.sl, op.mu, moduli, op.residues, op.rows_pad, op.k_pad);
+    crt_split_kernel<false, kCrtDefaultModuli><<<blocks, kSplitThreadsCrt, 0, stream>>>(A, moduli);
   else if (b <= 62)
-    crt_split_kernel<false, 0><<<grid, kSplitThreadsCrt, 0, stream>>>(x.ptr, x.rows, x.cols, x.sr, x.sl, op.mu, moduli,
-                                                                     op.residues, op.rows_pad, op.k_pad);
+    crt_split_kernel<false, 0><<<blocks, kSplitThreadsCrt, 0, stream>>>(A, moduli);
   else
-    crt_split_kernel<true, 0><<<grid, kSplitThreadsCrt, 0, stream>>>(x.ptr, x.rows, x.cols, x.sr, x.sl, op.mu, moduli,
-                                                                    op.residues, op.rows_pad, op.k_pad);
+    crt_split_kernel<true, 0><<<blocks, kSplitThreadsCrt, 0, stream>>>(A, moduli);
   return cudaGetLastError();
 }
 

@@ -173,10 +173,6 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
   const int max_splits =
       splits > 1 ? splits : ((stage2 && may_split) ? crt_split_rule(cx, m_pad, n_pad, k_pad, kCrtMinModuli) : 1);
   size_t off = 0;
-  const size_t o_mb_a = off;
-  off = align256(off + size_t(m) * 8);
-  const size_t o_mb_b = off;
-  off = align256(off + size_t(n) * 8);
   const int64_t nchunks = k_pad / kOzakiKBlock;  // 128-column chunks of the norm bounds
   const size_t o_ss_a = off;
   off = align256(off + size_t(m) * nchunks * 8);
@@ -211,28 +207,28 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
   uint8_t* ws = static_cast<uint8_t*>(cx.ws.ptr);
   DeviceFlags* df = cx.dflags;
   CrtOperand oa{reinterpret_cast<int8_t*>(ws + o_res_a), reinterpret_cast<int32_t*>(ws + o_mu_a),
-                reinterpret_cast<uint64_t*>(ws + o_mb_a), reinterpret_cast<uint64_t*>(ws + o_ss_a),
-                reinterpret_cast<int32_t*>(ws + o_ce_a), m, m_pad, k, k_pad, nmax};
+                reinterpret_cast<uint64_t*>(ws + o_ss_a), reinterpret_cast<int32_t*>(ws + o_ce_a), m, m_pad, k, k_pad,
+                nmax};
   const CrtOperand ob = same ? oa
                              : CrtOperand{reinterpret_cast<int8_t*>(ws + o_res_b), reinterpret_cast<int32_t*>(ws + o_mu_b),
-                                          reinterpret_cast<uint64_t*>(ws + o_mb_b),
                                           reinterpret_cast<uint64_t*>(ws + o_ss_b),
                                           reinterpret_cast<int32_t*>(ws + o_ce_b), n, n_pad, k, k_pad, nmax};
 
+  // every preparation step walks both operands in one launch (2048^3: scans, exponents and splits
+  // in three launches instead of six and two clears)
+  const CrtPrep prep{{va, vb}, {oa, ob}, same ? 1 : 2};
   bool ok = check_cuda(cudaMemsetAsync(df, 0, sizeof(DeviceFlags), st), "reset flags");
-  ok = ok && check_cuda(launch_crt_scan_norms(va, oa, &df->nonfinite, &df->spread[0], st), "scan A");
-  if (!same) ok = ok && check_cuda(launch_crt_scan_norms(vb, ob, &df->nonfinite, &df->spread[0], st), "scan B");
+  ok = ok && check_cuda(launch_crt_scan_norms(prep, &df->nonfinite, &df->spread[0], st), "scan");
   if (!ok) return EB2_ERR_CUDA;
-  info.launches = same ? 1 : 2;
+  info.launches = 1;
   // Stage 2 reads the scans' statistics on the host.  The residue split for the current
   // modulus count is launched first, so the GPU works while the host waits and decides; it is
   // redone only if the picker changes the count (both tile configurations use the same
   // residue layout).
   int split_moduli = 0;  // modulus count of the residues already launched (0: none)
   auto split = [&]() -> bool {
-    bool good = check_cuda(launch_crt_split(va, oa, nmod, st), "residues A");
-    if (!same) good = good && check_cuda(launch_crt_split(vb, ob, nmod, st), "residues B");
-    info.launches += same ? 2 : 4;
+    const bool good = check_cuda(launch_crt_split(prep, nmod, st), "residues");
+    info.launches += 2;
     split_moduli = nmod;
     return good;
   };
@@ -313,22 +309,24 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
     return good;
   };
   ok = product(true);
-  // IEEE semantics for NaN/Inf inputs: the FP64 kernel runs only when the scan saw one
-  // (for a triangle into the workspace, then merged into the triangle).
-  if (!tri) {
-    ok = ok && check_cuda(launch_dgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, &df->nonfinite,
-                                              st),
-                          "non-finite fallback");
-    info.launches += 1;
-  } else {
+  // IEEE semantics for NaN/Inf inputs: the FP64 kernel runs only when the scan saw one (for a
+  // triangle into the workspace, then merged into the triangle).  A call that reads the flags on
+  // the host launches it when they say so; a stream-ordered one launches it behind the flag.
+  auto non_finite = [&]() -> bool {
+    if (!tri) {
+      info.launches += 1;
+      return check_cuda(launch_dgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, &df->nonfinite, st),
+                        "non-finite fallback");
+    }
     double* full = reinterpret_cast<double*>(ws + o_full);
-    ok = ok && check_cuda(launch_dgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, 0.0, full, m, &df->nonfinite,
-                                              st),
-                          "non-finite fallback");
-    ok = ok && check_cuda(launch_merge_triangle<double>(full, m, n, opt.uplo == 1, beta, C, ldc, st, &df->nonfinite),
-                          "non-finite merge");
     info.launches += 2;
-  }
+    return check_cuda(launch_dgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, 0.0, full, m, &df->nonfinite, st),
+                      "non-finite fallback") &&
+           check_cuda(launch_merge_triangle<double>(full, m, n, opt.uplo == 1, beta, C, ldc, st, &df->nonfinite),
+                      "non-finite merge");
+  };
+  const bool host_reads = opt.sync || check;
+  if (!host_reads) ok = ok && non_finite();
   if (!ok) return EB2_ERR_CUDA;
   info.slices = nmod;
   info.tile_n = tile;
@@ -342,7 +340,7 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
       set_pending_timing(&cx, gemm_timed);
     }
   };
-  if (!opt.sync && !check) {
+  if (!host_reads) {
     finish_timing(true);
     return EB2_OK;
   }
@@ -361,6 +359,7 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
     }
     if (hf.nonfinite) {
       info.nonfinite = 1;
+      if (!non_finite() || (opt.sync && !check_cuda(cudaStreamSynchronize(st), "DGEMM"))) return EB2_ERR_CUDA;
       break;
     }
     // energies that overflowed (products near the FP64 range) leave the estimate unknown

@@ -138,10 +138,6 @@ extern "C" int eb2_dgemm_device_noalloc(char transa, char transb, int64_t m, int
   const int64_t m_pad = round_up(m, crt_tile_rows(tile)), n_pad = round_up(n, crt_tile_cols(tile)),
                 k_pad = round_up(k, kOzakiKBlock);
   size_t off = align256(sizeof(NoAllocFlags));
-  const size_t o_mb_a = off;
-  off = align256(off + size_t(m) * 8);
-  const size_t o_mb_b = off;
-  off = align256(off + size_t(n) * 8);
   const int64_t nchunks = k_pad / kOzakiKBlock;  // 128-column chunks of the norm bounds
   const size_t o_ss_a = off;
   off = align256(off + size_t(m) * nchunks * 8);
@@ -177,20 +173,18 @@ extern "C" int eb2_dgemm_device_noalloc(char transa, char transb, int64_t m, int
   const StridedView<double> vb =
       tb ? StridedView<double>{b, n, k, 1, ldb} : StridedView<double>{b, n, k, ldb, 1};  // op(B)^T, n x k
   CrtOperand oa{reinterpret_cast<int8_t*>(ws + o_res_a), reinterpret_cast<int32_t*>(ws + o_mu_a),
-                reinterpret_cast<uint64_t*>(ws + o_mb_a), reinterpret_cast<uint64_t*>(ws + o_ss_a),
+                reinterpret_cast<uint64_t*>(ws + o_ss_a),
                 reinterpret_cast<int32_t*>(ws + o_ce_a), m, m_pad, k, k_pad, kNoAllocModuli};
   CrtOperand ob{reinterpret_cast<int8_t*>(ws + o_res_b), reinterpret_cast<int32_t*>(ws + o_mu_b),
-                reinterpret_cast<uint64_t*>(ws + o_mb_b), reinterpret_cast<uint64_t*>(ws + o_ss_b),
+                reinterpret_cast<uint64_t*>(ws + o_ss_b),
                 reinterpret_cast<int32_t*>(ws + o_ce_b), n, n_pad, k, k_pad, kNoAllocModuli};
 
-  // The scratch keeps whatever the previous call left: the flags and the row maxima
-  // (atomicMax, zeroed by the scan launcher) start from zero; the chunk norm bounds, scale
-  // exponents and residues are overwritten.
+  // The scratch keeps whatever the previous call left: the flags start from zero; the chunk norm
+  // bounds, scale exponents and residues are overwritten.
   bool good = ok(cudaMemsetAsync(flags, 0, sizeof(NoAllocFlags), st), "reset flags");
-  good = good && ok(launch_crt_scan_norms(va, oa, &flags->nonfinite, nullptr, st), "scan A");
-  good = good && ok(launch_crt_scan_norms(vb, ob, &flags->nonfinite, nullptr, st), "scan B");
-  good = good && ok(launch_crt_split(va, oa, kNoAllocModuli, st), "residues A");
-  good = good && ok(launch_crt_split(vb, ob, kNoAllocModuli, st), "residues B");
+  const CrtPrep prep{{va, vb}, {oa, ob}, 2};
+  good = good && ok(launch_crt_scan_norms(prep, &flags->nonfinite, nullptr, st), "scan");
+  good = good && ok(launch_crt_split(prep, kNoAllocModuli, st), "residues");
   CrtGemmArgs g{};
   g.m = m;
   g.n = n;
