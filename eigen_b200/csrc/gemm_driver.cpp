@@ -666,8 +666,7 @@ int sgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
   const StridedView<float> vb = tb ? StridedView<float>{B, n, k, 1, ldb} : StridedView<float>{B, n, k, ldb, 1};
   DeviceFlags* df = cx.dflags;
   bool ok = check_cuda(cudaMemsetAsync(df, 0, sizeof(DeviceFlags), st), "reset flags");
-  ok = ok && check_cuda(launch_bf16_split(va, oa, &df->nonfinite, st), "split A");
-  ok = ok && check_cuda(launch_bf16_split(vb, ob, &df->nonfinite, st), "split B");
+  ok = ok && check_cuda(launch_bf16_split(va, oa, vb, ob, &df->nonfinite, st), "split");
   SgemmSplitArgs g{};
   g.m = m;
   g.n = n;
@@ -687,7 +686,7 @@ int sgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
   ok = ok && check_cuda(launch_sgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, &df->nonfinite, st),
                         "non-finite fallback");
   if (!ok) return EB2_ERR_CUDA;
-  info.launches = 4;  // 2 splits, GEMM, non-finite fallback (exits at once when unused)
+  info.launches = 3;  // split, GEMM, non-finite fallback (exits at once when unused)
   info.slices = pieces * (pieces + 1) / 2;
   info.tile_n = tile_n;
   if (opt.timed) {

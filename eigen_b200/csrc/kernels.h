@@ -191,9 +191,9 @@ struct Bf16Operand {
   void* pieces;  // [3][rows_pad][k_pad] bf16: hi, mid, lo pieces, row r contiguous along k
   int64_t rows, rows_pad, k, k_pad;
 };
-// Split op(X) (rows x k view) into its three BF16 pieces; sets *nonfinite on NaN/Inf.
-cudaError_t launch_bf16_split(const StridedView<float>& x, const Bf16Operand& op, int* nonfinite,
-                              cudaStream_t stream);
+// Split op(A) and op(B)^T (rows x k views) into their three BF16 pieces; sets *nonfinite on NaN/Inf.
+cudaError_t launch_bf16_split(const StridedView<float>& xa, const Bf16Operand& oa, const StridedView<float>& xb,
+                              const Bf16Operand& ob, int* nonfinite, cudaStream_t stream);
 
 struct SgemmSplitArgs {
   int64_t m, n, k;
