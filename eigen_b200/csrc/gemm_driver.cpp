@@ -658,6 +658,10 @@ int sgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
   off = align256(off + size_t(3) * m_pad * k_pad * 2);
   const size_t o_b = off;
   off = align256(off + size_t(3) * n_pad * k_pad * 2);
+  const int64_t tile_area = tile_m_of(tile_n, false) * tile_n_of(tile_n, false), tiles = m_pad * n_pad / tile_area;
+  const Bf16Split split = bf16_split_rule(tiles, k_pad, tile_n == kTilePair ? cx.num_sms / 2 : cx.num_sms);
+  const size_t o_part = off;
+  off = align256(off + size_t(split.ranges) * (tiles - split.whole_tiles) * tile_area * 4);
   if (const int rc = reserve_buffer(cx.ws, off, st, "emulation workspace"); rc != EB2_OK) return rc;
   uint8_t* ws = static_cast<uint8_t*>(cx.ws.ptr);
   Bf16Operand oa{ws + o_a, m, m_pad, k, k_pad};
@@ -680,13 +684,16 @@ int sgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
   g.status = &df->status;
   g.tile_n = tile_n;
   g.num_sms = cx.num_sms;
+  g.split = split;
+  g.partial = reinterpret_cast<float*>(ws + o_part);
+  call_config().splits = split.ranges;
   if (opt.timed) cudaEventRecord(cx.ev_gemm0, st);
   ok = ok && check_cuda(launch_sgemm_split_bf16(oa, ob, g, st), "split-BF16 GEMM");
   if (opt.timed) cudaEventRecord(cx.ev_gemm1, st);
   ok = ok && check_cuda(launch_sgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, &df->nonfinite, st),
                         "non-finite fallback");
   if (!ok) return EB2_ERR_CUDA;
-  info.launches = 3;  // split, GEMM, non-finite fallback (exits at once when unused)
+  info.launches = split.ranges > 1 ? 4 : 3;  // split, GEMM (+ sum of K ranges), non-finite fallback (exits at once when unused)
   info.slices = pieces * (pieces + 1) / 2;
   info.tile_n = tile_n;
   if (opt.timed) {

@@ -195,6 +195,15 @@ struct Bf16Operand {
 cudaError_t launch_bf16_split(const StridedView<float>& xa, const Bf16Operand& oa, const StridedView<float>& xb,
                               const Bf16Operand& ob, int* nonfinite, cudaStream_t stream);
 
+// Which output tiles are computed over K in several ranges: all but the first whole_tiles (a
+// multiple of the CTAs in flight), whose last round would leave CTAs idle.
+struct Bf16Split {
+  int64_t whole_tiles;
+  int ranges;  // K ranges of each other tile
+};
+// For a grid of `tiles` output tiles on `ctas` CTAs (or CTA pairs).
+Bf16Split bf16_split_rule(int64_t tiles, int64_t k_pad, int ctas);
+
 struct SgemmSplitArgs {
   int64_t m, n, k;
   float alpha, beta;
@@ -205,6 +214,8 @@ struct SgemmSplitArgs {
   uint32_t* status;
   int tile_n;
   int num_sms;
+  Bf16Split split;
+  float* partial;  // the split tiles' sums: ranges * (tiles - whole_tiles) * tile area
 };
 cudaError_t launch_sgemm_split_bf16(const Bf16Operand& a, const Bf16Operand& b, const SgemmSplitArgs& args,
                                     cudaStream_t stream);

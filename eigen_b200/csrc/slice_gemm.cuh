@@ -97,6 +97,9 @@ struct SliceGemmParams {
                          // triangular (zero blocks of K skipped per tile); 0 = dense
   uint64_t wait_limit_ns;  // wall-time bound of the pipeline waits (the drain waits keep kWaitLimitNs)
   int splits;            // CRT: K ranges per (tile, modulus), each with its own residue plane (1: none)
+                         // split-BF16: K ranges (whole chunks) of every tile from whole_tiles on
+  int whole_tiles;       // split-BF16: the first tiles of the raster, computed over all of K
+  float* partial;        // split-BF16: FP32 sums of the split tiles, [splits][tiles][BN][tile rows]
 };
 
 // Pair range of diagonal t: p = p_lo .. p_lo + total/num_kb - 1 (q = t - p).
@@ -162,7 +165,27 @@ __device__ __forceinline__ void tile_k_range(const SliceGemmParams& P, int tile,
 template <bool LISTED>
 __host__ __device__ __forceinline__ int num_work(const SliceGemmParams& P) {
   if (LISTED) return P.num_listed * P.slices;
-  return P.tiles_m * P.tiles_n * (P.crt ? P.slices * P.splits : 1);
+  if (P.crt) return P.tiles_m * P.tiles_n * P.slices * P.splits;
+  return P.whole_tiles + (P.tiles_m * P.tiles_n - P.whole_tiles) * P.splits;
+}
+
+// Split-BF16 work item w: the tiles [0, whole_tiles) over all of K, then the other tiles split by
+// split, each over the K blocks [kb_lo, kb_hi) of its range (whole chunks, none empty: splits <=
+// the chunks).  split < 0: all of K.
+__device__ __forceinline__ void bf16_item(const SliceGemmParams& P, int w, int& tile, int& split, int& kb_lo,
+                                          int& kb_hi) {
+  if (w < P.whole_tiles) {
+    tile = w;
+    split = -1;
+    kb_lo = 0;
+    kb_hi = P.num_kb;
+    return;
+  }
+  const int rest = P.tiles_m * P.tiles_n - P.whole_tiles, chunks = (P.num_kb + kBf16ChunkKb - 1) / kBf16ChunkKb;
+  tile = P.whole_tiles + (w - P.whole_tiles) % rest;
+  split = (w - P.whole_tiles) / rest;
+  kb_lo = int(int64_t(split) * chunks / P.splits) * kBf16ChunkKb;
+  kb_hi = min(P.num_kb, int(int64_t(split + 1) * chunks / P.splits) * kBf16ChunkKb);
 }
 template <bool LISTED>
 __device__ __forceinline__ void work_item(const SliceGemmParams& P, int w, int& tile, int& t_hi, int& t_lo,
@@ -307,10 +330,11 @@ __device__ __forceinline__ void slice_producer(const CUtensorMap* tmA, const CUt
     // chunks of kBf16ChunkKb K blocks; in each, the diagonals (smallest weight first), their
     // pairs and the chunk's K blocks -- the order slice_mma consumes them in
     for (int w = first_tile<PAIR>(); w < nwork && ok; w += tile_step<PAIR>()) {
-      int tm, tn;
-      tile_coords(w, P.tiles_m, P.tiles_n, P.group_m, tm, tn);
-      for (int kc = 0; kc < P.num_kb && ok; kc += kBf16ChunkKb) {
-        const int kend = min(P.num_kb, kc + kBf16ChunkKb);
+      int tile, split, kb_lo, kb_hi, tm, tn;
+      bf16_item(P, w, tile, split, kb_lo, kb_hi);
+      tile_coords(tile, P.tiles_m, P.tiles_n, P.group_m, tm, tn);
+      for (int kc = kb_lo; kc < kb_hi && ok; kc += kBf16ChunkKb) {
+        const int kend = min(kb_hi, kc + kBf16ChunkKb);
         for (int t = P.diag_hi; t >= P.diag_lo && ok; --t) {
           int p_lo, total;
           if (!diag_bounds(t, P.slices, P.num_kb, p_lo, total)) continue;
@@ -424,8 +448,10 @@ __device__ __forceinline__ void slice_mma(uint8_t* smem, uint64_t* full, uint64_
   if constexpr (MODE == kModeSplitBF16) {
     // one accumulation unit per chunk of kBf16ChunkKb K blocks (order as in slice_producer)
     for (int w = first_tile<PAIR>(); w < nwork && ok; w += tile_step<PAIR>()) {
-      for (int kc = 0; kc < P.num_kb && ok; kc += kBf16ChunkKb) {
-        const int kend = min(P.num_kb, kc + kBf16ChunkKb);
+      int tile, split, kb_lo, kb_hi;
+      bf16_item(P, w, tile, split, kb_lo, kb_hi);
+      for (int kc = kb_lo; kc < kb_hi && ok; kc += kBf16ChunkKb) {
+        const int kend = min(kb_hi, kc + kBf16ChunkKb);
         if (!mbar_wait(&tempty[buf], ((tphase >> buf) & 1u) ^ 1u, abort_flag, P.status, P.wait_limit_ns)) {
           ok = false;
           break;
@@ -755,9 +781,9 @@ __device__ __forceinline__ void crt_epilogue(uint32_t tmem_base, uint64_t* tfull
   }
 }
 
-// Split-BF16: each thread owns one row and kCols columns of the tile.  The units of a tile
+// Split-BF16: each thread owns one row and kCols columns of the tile.  The units of an item
 // (one per kBf16ChunkKb K blocks) are added, rounded to nearest, into FP32 registers; after
-// the last one C = alpha * acc + beta * C in FP32.
+// the last one C = alpha * acc + beta * C in FP32, or the sum goes to its K range's plane.
 template <int BN, int NW, bool PAIR>
 __device__ __forceinline__ void bf16_epilogue(uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty,
                                               volatile int* abort_flag, const SliceGemmParams& P) {
@@ -767,21 +793,22 @@ __device__ __forceinline__ void bf16_epilogue(uint32_t tmem_base, uint64_t* tful
   const int quad = warp & 3;
   const int col_base = ((warp - 2) >> 2) * kCols;
   const int row = quad * 32 + lane;
-  const int num_tiles = P.tiles_m * P.tiles_n;
+  const int nwork = num_work<false>(P);
   const int row_base = PAIR ? int(cluster_ctarank()) * kSliceBM : 0;
   float* C = static_cast<float*>(P.C);
   int buf = 0;
   uint32_t ephase = 0u;
   bool ok = true;
-  for (int tile = first_tile<PAIR>(); tile < num_tiles && ok; tile += tile_step<PAIR>()) {
-    int tm, tn;
+  for (int w = first_tile<PAIR>(); w < nwork && ok; w += tile_step<PAIR>()) {
+    int tile, split, kb_lo, kb_hi, tm, tn;
+    bf16_item(P, w, tile, split, kb_lo, kb_hi);
     tile_coords(tile, P.tiles_m, P.tiles_n, P.group_m, tm, tn);
     const int64_t m0 = int64_t(tm) * (PAIR ? 2 * kSliceBM : kSliceBM) + row_base;
     const int64_t n0 = int64_t(tn) * BN + col_base;
     float acc[kCols];
 #pragma unroll
     for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
-    for (int kc = 0; kc < P.num_kb; kc += kBf16ChunkKb) {
+    for (int kc = kb_lo; kc < kb_hi; kc += kBf16ChunkKb) {
       if (!mbar_wait(&tfull[buf], (ephase >> buf) & 1u, abort_flag, P.status, P.wait_limit_ns)) {
         ok = false;
         break;
@@ -802,6 +829,18 @@ __device__ __forceinline__ void bf16_epilogue(uint32_t tmem_base, uint64_t* tful
       buf ^= 1;
     }
     const int64_t grow = m0 + row;
+    if (split >= 0) {
+      // this K range's sum of the whole (padded) tile, added to the others' by a second launch
+      constexpr int kRows = PAIR ? 2 * kSliceBM : kSliceBM;
+      const int rest = P.tiles_m * P.tiles_n - P.whole_tiles;
+      if (ok) {
+        float* pp = P.partial + (int64_t(split) * rest + (tile - P.whole_tiles)) * (BN * kRows) +
+                    (n0 - int64_t(tn) * BN) * kRows + row_base + row;
+#pragma unroll
+        for (int j = 0; j < kCols; ++j, pp += kRows) *pp = acc[j];
+      }
+      continue;
+    }
     if (ok && grow < P.m) {
       float* cp = C + grow + n0 * P.ldc;
 #pragma unroll
