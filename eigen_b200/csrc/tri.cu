@@ -178,7 +178,8 @@ __global__ void __launch_bounds__(kTriVecs) tri_block_multiply_kernel(const T* _
 // Bound by the serial chain of 16 sub-blocks (a solve, a small product and two barriers each),
 // so V shrinks until the vectors fill the SMs.  A 4096 solve with 2048 vectors (16 blocks of 256)
 // went from 3047 to 1820 us against 64 vectors per CTA, 32-row sub-blocks without look-ahead and
-// FMA updates (129 us a block on 32 CTAs).
+// FMA updates (129 us a block on 32 CTAs), and from 1704 to 1439 us (48 to 31 us a block) with one
+// address step per staged coefficient and the diagonal's reciprocals formed once at the start.
 constexpr int kPanelSub = 16;
 
 template <typename T, int V>
@@ -189,7 +190,7 @@ struct PanelCfg {
   static constexpr int kPer = kPanelMax * kPanelSub / kThreads;  // coefficients a thread stages per panel
   static size_t smem(int nb) {
     const size_t nbp = size_t(nb + kPanelSub - 1) / kPanelSub * kPanelSub;
-    return (nbp * kXld + 2 * kPanelSub * (nbp + 4) + kPanelSub) * sizeof(T);
+    return (nbp * kXld + 2 * kPanelSub * (nbp + 4) + nbp) * sizeof(T);
   }
 };
 
@@ -238,44 +239,45 @@ __global__ void __launch_bounds__(PanelCfg<T, V>::kThreads)
   T* Xs = reinterpret_cast<T*>(smem_raw);  // [nbp][kXld]: Xs[r * kXld + t], forward row order
   T* panel0 = Xs + nbp * kXld;             // [kPanelSub][ldp] each: -E'(jb + r, jb + c) at c * ldp + r
   T* panel1 = panel0 + kPanelSub * ldp;
-  T* Dinv = panel1 + kPanelSub * ldp;      // [kPanelSub]: reciprocals of the diagonal
+  T* Dinv = panel1 + kPanelSub * ldp;      // [nbp]: reciprocals of the diagonal
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, tig = lane & 3;
   const int64_t t0 = int64_t(blockIdx.x) * V;
   const int nv = int(count - t0 < V ? count - t0 : V);
   // forward row r is row ro(r) of the stored system
   auto ro = [&](int r) -> int64_t { return lower ? r : nb - 1 - r; };
-  // the coefficients are contiguous along the rows, or along the columns when transposed
+  // The coefficients are contiguous along the rows, or along the columns when transposed.  A
+  // thread's elements of a panel are a row and kPer columns (or a column and kPer rows) at fixed
+  // offsets from the panel's corner, so their addresses move by one step per element and panel.
   const bool row_fast = er == 1;
+  const int rb = row_fast ? tid % kPanelMax : tid / kPanelSub, cb = row_fast ? tid / kPanelMax : tid % kPanelSub;
+  const int rq = row_fast ? 0 : kThreads / kPanelSub, cq = row_fast ? kThreads / kPanelMax : 0;
+  const int64_t sgn = lower ? 1 : -1;
+  const int64_t qstep = sgn * (row_fast ? cq * ec : rq * er), sub_step = sgn * kPanelSub * (er + ec);
+  const T* corner = E + ro(rb) * er + ro(cb) * ec;  // element q = 0 of the next panel
+  int left = nb;                                    // rows from the next panel's corner to the end
   T cv[C::kPer];
-  auto fetch = [&](int sub) {  // the panel of sub-block `sub` into registers
-    const int jb = sub * kPanelSub;
+  auto fetch = [&]() {  // the next panel into registers
+    const T* p = corner;
 #pragma unroll
-    for (int q = 0; q < C::kPer; ++q) {
-      const int idx = tid + q * kThreads;
-      const int r = jb + (row_fast ? idx % kPanelMax : idx / kPanelSub);
-      const int c = jb + (row_fast ? idx / kPanelMax : idx % kPanelSub);
-      T v = r == c ? T(1) : T(0);
-      if (r < nb && (r > c || (r == c && !unit))) v = E[ro(r) * er + ro(c) * ec];
-      cv[q] = v;
+    for (int q = 0; q < C::kPer; ++q, p += qstep) {
+      const int r = rb + q * rq, c = cb + q * cq;
+      cv[q] = r == c ? T(1) : T(0);
+      if (r < left && (r > c || (r == c && !unit))) cv[q] = *p;
     }
+    corner += sub_step;
+    left -= kPanelSub;
   };
   auto stash = [&](int sub, T* panel) {
     const int rows = nbp - sub * kPanelSub;
+    T* p = panel + cb * ldp + rb;
+    const int pstep = cq * ldp + rq;
 #pragma unroll
-    for (int q = 0; q < C::kPer; ++q) {
-      const int idx = tid + q * kThreads;
-      const int r = row_fast ? idx % kPanelMax : idx / kPanelSub;
-      const int c = row_fast ? idx / kPanelMax : idx % kPanelSub;
-      if (r < rows) panel[c * ldp + r] = -cv[q];
-    }
+    for (int q = 0; q < C::kPer; ++q, p += pstep)
+      if (rb + q * rq < rows) *p = -cv[q];
   };
   auto solve = [&](int sub, const T* panel) {  // the solving warps
-    if (lane < kPanelSub && warp == 0) Dinv[lane] = unit ? T(1) : T(-1) / panel[lane * ldp + lane];
-    if constexpr (C::kSolvers > 1)
-      asm volatile("bar.sync 1, 64;" ::: "memory");
-    else
-      __syncwarp();
+    const T* const dinv = Dinv + sub * kPanelSub;
     const int t = warp * 32 + lane;
     if (t < V) {
       T* x = Xs + sub * kPanelSub * kXld + t;
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(PanelCfg<T, V>::kThreads)
       for (int c = 0; c < kPanelSub; ++c) {
         // x_c = s_c / d_c, then s_r -= d_rc x_c for every later row r: independent updates, so
         // the dependent chain is two operations per row
-        const T xc = sv[c] * Dinv[c];
+        const T xc = sv[c] * dinv[c];
         sv[c] = xc;
 #pragma unroll
         for (int r = c + 1; r < kPanelSub; ++r) sv[r] = fma_rn(panel[c * ldp + r], xc, sv[r]);
@@ -296,7 +298,8 @@ __global__ void __launch_bounds__(PanelCfg<T, V>::kThreads)
     }
   };
 
-  fetch(0);
+  fetch();
+  for (int r = tid; r < nbp; r += kThreads) Dinv[r] = r < nb && !unit ? T(1) / E[ro(r) * (er + ec)] : T(1);
   if (ts == 1) {
     for (int idx = tid; idx < nbp * V; idx += kThreads) {
       const int t = idx % V, r = idx / V;
@@ -309,7 +312,7 @@ __global__ void __launch_bounds__(PanelCfg<T, V>::kThreads)
   }
   stash(0, panel0);
   if (nsub > 1) {
-    fetch(1);
+    fetch();
     stash(1, panel1);
   }
   __syncthreads();
@@ -318,7 +321,7 @@ __global__ void __launch_bounds__(PanelCfg<T, V>::kThreads)
   for (int j = 0; j + 1 < nsub; ++j) {
     T* const panel = (j & 1) ? panel1 : panel0;       // sub-block j's columns
     const T* const next = (j & 1) ? panel0 : panel1;  // sub-block j+1's
-    if (j + 2 < nsub) fetch(j + 2);
+    if (j + 2 < nsub) fetch();
     const T* xs = Xs + j * kPanelSub * kXld;
     // the next sub-block's rows
     if (warp < V / 8)
