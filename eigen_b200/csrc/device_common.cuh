@@ -336,5 +336,21 @@ __device__ __forceinline__ void cp_async_elem(uint32_t dst, const void* src, boo
                "r"(valid ? BYTES : 0)
                : "memory");
 }
+// One element of SIZE bytes to dst + OFF if index < limit (nothing is written otherwise).
+template <int SIZE, int OFF>
+__device__ __forceinline__ void cp_async_elem_if(uint32_t dst, const void* src, int index, int limit) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %2, %3;\n\t@p cp.async.ca.shared.global [%0+%4], [%1], %5;\n\t}" ::"r"(dst),
+      "l"(src), "r"(index), "r"(limit), "n"(OFF), "n"(SIZE)
+      : "memory");
+}
+// The same with `bytes` (0: zero fill) read.
+template <int SIZE>
+__device__ __forceinline__ void cp_async_fill_if(uint32_t dst, const void* src, int bytes, int index, int limit) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %2, %3;\n\t@p cp.async.ca.shared.global [%0], [%1], %4, %5;\n\t}" ::"r"(dst),
+      "l"(src), "r"(index), "r"(limit), "n"(SIZE), "r"(bytes)
+      : "memory");
+}
 
 }  // namespace eb2

@@ -617,8 +617,18 @@ int sgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
   }
   int method = opt.method ? opt.method : settings().sgemm_method.load();
   int cfg_tile = 0;  // tile of an automatic split-BF16 choice (0: the size rule)
+  bool small = false;
   if (method == EB2_METHOD_AUTO) {
-    // a forced configuration class (the tuner), else the learned picker, else split-BF16
+    // a forced configuration class (the tuner), else the small-product kernel where it is the
+    // faster one and no setting asks for a split-BF16 variant, else the learned picker, else
+    // split-BF16
+    const int fc = forced_config();
+    small = fc < 0 && opt.tile_n == 0 && opt.pieces == 0 && settings().tile_n.load() == 0 &&
+            settings().sgemm_pieces.load() == 3 && sgemm_small_applies(m, n, k);
+  }
+  if (small) {
+    method = EB2_METHOD_NATIVE;
+  } else if (method == EB2_METHOD_AUTO) {
     const int fc = forced_config();
     int cfg = -1, cls = 0;
     if (fc >= kCfgSgemmFfma && fc <= kCfgSgemmBf16Pair)
@@ -633,7 +643,8 @@ int sgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
   if (method == EB2_METHOD_NATIVE) {
     call_config().config = kCfgSgemmFfma;
     if (opt.timed) cudaEventRecord(cx.ev_gemm0, st);
-    if (!check_cuda(launch_sgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, st),
+    if (!check_cuda(small ? launch_sgemm_small(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st)
+                          : launch_sgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, st),
                     "native SGEMM"))
       return EB2_ERR_CUDA;
     info.launches = 1;

@@ -36,6 +36,12 @@ cudaError_t launch_dgemm_native(bool transA, bool transB, int64_t m, int64_t n, 
 cudaError_t launch_sgemm_native(bool transA, bool transB, int64_t m, int64_t n, int64_t k, float alpha,
                                 const float* A, int64_t lda, const float* B, int64_t ldb, float beta, float* C,
                                 int64_t ldc, const int* only_if_flag, cudaStream_t stream);
+// FP32 products that fill the chip for less time than a split-BF16 product's launches take: one
+// launch, FP32 sums of 32-step chains and eight K shares.
+bool sgemm_small_applies(int64_t m, int64_t n, int64_t k);
+cudaError_t launch_sgemm_small(bool transA, bool transB, int64_t m, int64_t n, int64_t k, float alpha, const float* A,
+                               int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc,
+                               cudaStream_t stream);
 // C = beta * C (beta == 0 writes exact zeros), the BLAS pre-scale for alpha == 0 or k == 0.
 cudaError_t launch_scale_matrix_d(int64_t m, int64_t n, double beta, double* C, int64_t ldc, cudaStream_t stream);
 cudaError_t launch_scale_matrix_s(int64_t m, int64_t n, float beta, float* C, int64_t ldc, cudaStream_t stream);

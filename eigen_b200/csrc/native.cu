@@ -11,6 +11,9 @@
 // (GeneralBlockPanelKernel.h:1879-2478): they read op(A)/op(B) through lda/ldb and
 // the transpose flags and write one fixed shared-memory layout, so the inner
 // product loop is the same for NN/NT/TN/TT.
+#include <climits>
+#include <utility>
+
 #include "device_common.cuh"
 #include "kernels.h"
 
@@ -340,6 +343,150 @@ __global__ void __launch_bounds__(kSThreads)
   }
 }
 
+// ------------------------------------------------------------------ FP32, small products
+// One launch with FP32 inputs and sums, for products too small to fill the tensor cores with
+// split-BF16 pieces (a split, a GEMM whose K blocks follow one another on a few SMs, a sum of K
+// ranges and a fallback launch: 23 us and more of device time).  The eight warps of a block share
+// a 32 x 32 output tile and split K: each warp computes all 32 x 32 outputs (8 x 4 per lane) over
+// its 8 of every K tile's 64.  K tiles arrive by cp.async in a ring of kFStages; shared memory is
+// [k][row] for both operands, so a lane's rows and columns are 16-byte loads.  A lane adds its
+// products 32 K steps at a time (FMA chains) into running sums, and the eight partial sums are
+// added in a fixed order through shared memory, so rounding errors grow with sqrt(32) and
+// sqrt(K / 256) instead of sqrt(K).  Bound by issue slots: 35 instructions per K step and warp for
+// 1024 FMAs, plus the copies, so a copy is one address and one predicated instruction.
+constexpr int kFTile = 32, kFWarps = 8, kFThreads = 32 * kFWarps;
+constexpr int kFKW = 8, kFKT = kFWarps * kFKW;  // K per warp and per tile
+constexpr int kFLd = kFTile + 4;                // [k] row stride (floats)
+constexpr int kFStages = 4, kFChunk = 32;
+constexpr int kFStage = 2 * kFKT * kFLd;        // floats
+constexpr int kFSmem = 4 * kFStages * kFStage;
+static_assert(kFWarps * kFTile * kFLd * 4 <= kFSmem, "the sums are staged in the ring");
+
+// The copies of one operand (rows x k view at X, tile rows r0 .. r0+31), K tile after K tile:
+// element (r, kk) of a tile to dst[kk * kFLd + r].  MN_CONTIG: the rows are contiguous in global
+// memory, and a warp takes the 32 rows of a K offset; else the K index is, and a warp takes 8
+// neighbours along K of 4 rows (distinct banks).  Rows outside the matrix are not copied (their
+// outputs are not stored); the K tail is zero-filled.
+template <bool MN_CONTIG>
+struct FCopy {
+  static constexpr int kCopies = kFTile * kFKT / kFThreads;  // K offsets kk, kk + 8, ... of one row
+  const char* src;  // first copy of the next tile
+  int64_t step;     // bytes from copy to copy
+  int left;         // K elements from the thread's first one to the end
+  uint32_t dst;
+  int row_ok;
+  __device__ __forceinline__ void start(const float* x, int64_t ld, int64_t rows, int64_t k, int64_t r0, int t) {
+    const int r = MN_CONTIG ? t % 32 : ((t >> 3) & 3) + 4 * (t >> 5), kk = MN_CONTIG ? t / 32 : t & 7;
+    row_ok = r0 + r < rows ? 1 : 0;
+    left = int(k) - kk;
+    step = MN_CONTIG ? 8 * ld * 4 : 32;
+    src = reinterpret_cast<const char*>(MN_CONTIG ? x + (r0 + r) + kk * ld : x + kk + (r0 + r) * ld);
+    dst = uint32_t((kk * kFLd + r) * 4);
+  }
+  template <int... q>
+  __device__ __forceinline__ void whole(uint32_t d, std::integer_sequence<int, q...>) const {
+    (cp_async_elem_if<4, q * 8 * kFLd * 4>(d, src + q * step, 0, row_ok), ...);
+  }
+  __device__ __forceinline__ void issue(uint32_t stage, const void* any) {
+    const uint32_t d = stage + dst;
+    if (left > (kCopies - 1) * 8) {  // every K offset of the tile inside
+      whole(d, std::make_integer_sequence<int, kCopies>{});
+    } else {
+#pragma unroll
+      for (int q = 0; q < kCopies; ++q) {
+        const bool in = left > 8 * q;
+        cp_async_fill_if<4>(d + uint32_t(q * 8 * kFLd * 4), in ? src + q * step : any, in ? 4 : 0, 0, row_ok);
+      }
+    }
+    src += kCopies * step;
+    left -= kFKT;
+  }
+};
+
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(kFThreads, 2)
+    sgemm_small_kernel(int64_t m, int64_t n, int64_t k, float alpha, const float* __restrict__ A, int64_t lda,
+                       const float* __restrict__ B, int64_t ldb, float beta, float* __restrict__ C, int64_t ldc) {
+  extern __shared__ __align__(16) float fsmem[];
+  const int t = int(threadIdx.x), warp = t >> 5, lane = t & 31;
+  const int ty = lane >> 3, tx = lane & 7;  // rows 4 ty .., 16 + 4 ty ..; columns 4 tx ..
+  const int64_t m0 = int64_t(blockIdx.x) * kFTile, n0 = int64_t(blockIdx.y) * kFTile;
+  const int nkt = int((k + kFKT - 1) / kFKT);
+  FCopy<!TA> ca;
+  FCopy<TB> cb;
+  ca.start(A, lda, m, k, m0, t);
+  cb.start(B, ldb, n, k, n0, t);
+  const uint32_t ring = smem_u32(fsmem);
+  auto copy = [&](int stage) {
+    const uint32_t st = ring + uint32_t(stage * kFStage * 4);
+    ca.issue(st, A);
+    cb.issue(st + uint32_t(kFKT * kFLd * 4), B);
+  };
+#pragma unroll
+  for (int s = 0; s < kFStages - 1; ++s) {
+    if (s < nkt) copy(s);
+    cp_async_commit();
+  }
+  float c[8][4], sum[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[i][j] = sum[i][j] = 0.f;
+  auto flush = [&]() {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        sum[i][j] += c[i][j];
+        c[i][j] = 0.f;
+      }
+  };
+  int stage = 0;
+  for (int kt = 0; kt < nkt; ++kt) {
+    cp_async_wait<kFStages - 2>();
+    __syncthreads();  // tile kt has landed for everyone; the slot refilled below is free
+    if (kt + kFStages - 1 < nkt) copy(stage == 0 ? kFStages - 1 : stage - 1);
+    cp_async_commit();
+    const float* sa = fsmem + stage * kFStage + warp * kFKW * kFLd + ty * 4;
+    const float* sb = fsmem + stage * kFStage + (kFKT + warp * kFKW) * kFLd + tx * 4;
+#pragma unroll
+    for (int kk = 0; kk < kFKW; ++kk) {
+      const float4 a0 = *reinterpret_cast<const float4*>(sa + kk * kFLd);
+      const float4 a1 = *reinterpret_cast<const float4*>(sa + kk * kFLd + 16);
+      const float4 b0 = *reinterpret_cast<const float4*>(sb + kk * kFLd);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b0.x, b0.y, b0.z, b0.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[i][j] = fmaf(av[i], bv[j], c[i][j]);
+    }
+    if ((kt + 1) % (kFChunk / kFKW) == 0) flush();
+    stage = stage == kFStages - 1 ? 0 : stage + 1;
+  }
+  flush();
+  cp_async_wait<0>();
+  __syncthreads();  // the ring becomes the staging of the sums: [warp][column][row]
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float* p = fsmem + (warp * kFTile + tx * 4 + j) * kFLd + ty * 4;
+    *reinterpret_cast<float4*>(p) = make_float4(sum[0][j], sum[1][j], sum[2][j], sum[3][j]);
+    *reinterpret_cast<float4*>(p + 16) = make_float4(sum[4][j], sum[5][j], sum[6][j], sum[7][j]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int idx = t; idx < kFTile * kFTile; idx += kFThreads) {
+    const int r = idx % kFTile, cc = idx / kFTile;
+    float v = fsmem[cc * kFLd + r];
+#pragma unroll
+    for (int w = 1; w < kFWarps; ++w) v += fsmem[(w * kFTile + cc) * kFLd + r];
+    if (m0 + r < m && n0 + cc < n) {
+      float* dst = C + (m0 + r) + (n0 + cc) * ldc;
+      v = __fmul_rn(alpha, v);
+      *dst = (beta == 0.f) ? v : __fmaf_rn(beta, *dst, v);
+    }
+  }
+}
+
 template <typename T>
 __global__ void scale_matrix_kernel(int64_t m, int64_t n, T beta, T* C, int64_t ldc) {
   const int64_t total = m * n;
@@ -438,6 +585,33 @@ cudaError_t launch_sgemm_native(bool transA, bool transB, int64_t m, int64_t n, 
     sgemm_ffma_kernel<true, true><<<grid, kSThreads, 0, stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
                                                                    only_if_flag);
   return cudaGetLastError();
+}
+
+bool sgemm_small_applies(int64_t m, int64_t n, int64_t k) {
+  // Rounds of tiles over the SMs times K, up to where split-BF16 takes over (device time, us, this
+  // kernel / split-BF16 or the FFMA kernel before): 64^3 2.9 / 11.6, 128^3 3.9 / 26.2, 256^3 5.7 /
+  // 24.8, 384^3 7.4 / 23.3, 512^3 16.0 / 23.7, 32 x 4096 x 1024 16.1 / 27.7; past the line
+  // 300 x 517 x 1100 33 / 26.9, 640^3 28.9 / 25.8.
+  const int64_t tiles = ((m + kFTile - 1) / kFTile) * ((n + kFTile - 1) / kFTile);
+  return (n + kFTile - 1) / kFTile <= 65535 && (tiles + 147) / 148 * k <= 1200;
+}
+
+cudaError_t launch_sgemm_small(bool transA, bool transB, int64_t m, int64_t n, int64_t k, float alpha, const float* A,
+                               int64_t lda, const float* B, int64_t ldb, float beta, float* C, int64_t ldc,
+                               cudaStream_t stream) {
+  if (m <= 0 || n <= 0) return cudaSuccess;
+  const dim3 grid(unsigned((m + kFTile - 1) / kFTile), unsigned((n + kFTile - 1) / kFTile));
+  if (grid.y > 65535u || k > INT_MAX / 2) return cudaErrorInvalidConfiguration;
+  auto pick = [&](auto kern) -> cudaError_t {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, kFThreads, kFSmem, stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+    return cudaGetLastError();
+  };
+  if (!transA && !transB) return pick(sgemm_small_kernel<false, false>);
+  if (transA && !transB) return pick(sgemm_small_kernel<true, false>);
+  if (!transA) return pick(sgemm_small_kernel<false, true>);
+  return pick(sgemm_small_kernel<true, true>);
 }
 
 cudaError_t launch_scale_matrix_d(int64_t m, int64_t n, double beta, double* C, int64_t ldc, cudaStream_t stream) {
