@@ -253,15 +253,24 @@ __global__ void __launch_bounds__(kNormThreads) crt_scan_norm_kernel(const __gri
   const int64_t r = r0 + rr;
   // the spread statistic: the first 64 columns of every 512 (block-uniform)
   const bool stat = spread != nullptr && (l0 & 511) == 0;
-  // bit patterns of |x| order like the values, NaN above +Inf
-  unsigned long long mb = 0, mb64 = 0;
-  int esum = 0, ecnt = 0;
+  // high words of |x| order like the values down to their exponents (Inf and NaN on top), and `any`
+  // tells a nonzero entry
+  uint32_t top = 0u, any = 0u;
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    const unsigned long long bits =
-        static_cast<unsigned long long>(__double_as_longlong(fabs(tile[rr][sub + 8 * j])));
-    mb = bits > mb ? bits : mb;
-    if (stat && j < 8) {
+    const double x = tile[rr][sub + 8 * j];
+    const uint32_t hw = uint32_t(__double2hiint(x)) & 0x7FFFFFFFu;
+    top = max(top, hw);
+    any |= hw | uint32_t(__double2loint(x));
+  }
+  unsigned long long mb64 = 0;
+  int esum = 0, ecnt = 0;
+  if (stat) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      // bit patterns of |x| order like the values, NaN above +Inf
+      const unsigned long long bits =
+          static_cast<unsigned long long>(__double_as_longlong(fabs(tile[rr][sub + 8 * j])));
       mb64 = bits > mb64 ? bits : mb64;
       if (bits) {
         esum += int(bits >> 52);
@@ -271,8 +280,8 @@ __global__ void __launch_bounds__(kNormThreads) crt_scan_norm_kernel(const __gri
   }
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) {
-    const unsigned long long other = __shfl_xor_sync(0xffffffffu, mb, o);
-    mb = other > mb ? other : mb;
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    any |= __shfl_xor_sync(0xffffffffu, any, o);
     if (stat) {
       const unsigned long long other64 = __shfl_xor_sync(0xffffffffu, mb64, o);
       mb64 = other64 > mb64 ? other64 : mb64;
@@ -280,30 +289,62 @@ __global__ void __launch_bounds__(kNormThreads) crt_scan_norm_kernel(const __gri
       ecnt += __shfl_xor_sync(0xffffffffu, ecnt, o);
     }
   }
-  unsigned long long s = 0;
+  const bool finite = top < 0x7FF00000u;
   int e = 0;
-  if (mb != 0 && mb < kInfBitsCrt) {
-    e = frexp_exp(mb);
-    // scale2(x, -e) with its two power-of-two factors formed once
-    const double f1 = exp2_int((-e) / 2), f2 = exp2_int(-e - (-e) / 2);
+  unsigned long long s = 0;
+  if (any != 0u && finite) {
+    if (top >= 0x00100000u) {
+      e = int(top >> 20) - 1022;  // |x| in [2^(e-1), 2^e)
+    } else {
+      // subnormal entries only: the exponent of the largest, over the row's 8 lanes
+      unsigned long long mb = 0;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const double x = tile[rr][sub + 8 * j];
-      const double xs = __dmul_rn(__dmul_rn(x, f1), f2);
-      // ceil(v) for v = rn(x'^2) 2^32 in [0, 2^32]: v + 2^52 rounded up is 2^52 + ceil(v)
-      // exactly, read from its bits (no rounding or conversion instruction)
-      const double v = __dmul_rn(__dmul_rn(xs, xs), 4294967296.0);
-      const unsigned long long c = static_cast<unsigned long long>(__double_as_longlong(__dadd_ru(v, 0x1p52)) -
-                                                                   __double_as_longlong(0x1p52));
-      s += x != 0.0 ? c + 1ull : 0ull;
+      for (int j = 0; j < 16; ++j) {
+        const unsigned long long bits =
+            static_cast<unsigned long long>(__double_as_longlong(fabs(tile[rr][sub + 8 * j])));
+        mb = bits > mb ? bits : mb;
+      }
+      const unsigned lanes = 0xFFu << (threadIdx.x & 24u);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        const unsigned long long other = __shfl_xor_sync(lanes, mb, o);
+        mb = other > mb ? other : mb;
+      }
+      e = frexp_exp(mb);
     }
+    // ceil(v) for v = rn(x'^2) 2^32 in [0, 2^32]: v + 2^52 rounded up is 2^52 + ceil(v) exactly, so
+    // the bits of the sums are added and the 16 offsets taken off at the end
+    int nonzero = 0;
+    auto add = [&](double x, double xs) {
+      const double v = __dmul_rn(__dmul_rn(xs, xs), 4294967296.0);
+      s += static_cast<unsigned long long>(__double_as_longlong(__dadd_ru(v, 0x1p52)));
+      nonzero += x != 0.0 ? 1 : 0;
+    };
+    if (e >= -1022 && e <= 1021) {
+      // 2^-e is a normal double: one product, exact wherever the square does not vanish
+      const double f = __hiloint2double((1023 - e) << 20, 0);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const double x = tile[rr][sub + 8 * j];
+        add(x, __dmul_rn(x, f));
+      }
+    } else {
+      // scale2(x, -e) with its two power-of-two factors formed once
+      const double f1 = exp2_int((-e) / 2), f2 = exp2_int(-e - (-e) / 2);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const double x = tile[rr][sub + 8 * j];
+        add(x, __dmul_rn(__dmul_rn(x, f1), f2));
+      }
+    }
+    s = s - 16ull * 0x4330000000000000ull + static_cast<unsigned long long>(nonzero);
   }
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (sub == 0 && r < rows) {
     O.chunk_e[r * O.nchunks + tl] = e;
-    O.chunk_s[r * O.nchunks + tl] = mb < kInfBitsCrt ? s : 0ull;
-    if (mb >= kInfBitsCrt) *nonfinite = 1;
+    O.chunk_s[r * O.nchunks + tl] = s;
+    if (!finite) *nonfinite = 1;
   }
   if (stat) {
     double chunk_spread = 0.0, chunk_count = 0.0;
@@ -1177,7 +1218,7 @@ __device__ __forceinline__ double crt_round(uint32_t r0, uint32_t r1, uint32_t r
 // gives columns below 2^46): the columns are exact doubles by one integer add and one FP64
 // subtraction, q = rint(S / P) comes from acc[1..3] (acc[0] / P < 2^-11 left out), or from
 // acc[2..3] for 13 moduli and more (q is off by one at most either way, which the range fix
-// absorbs), and R = S - q P takes its borrows column by column without carrying S first.
+// absorbs), and R = S - q P takes its carries column by column without carrying S first.
 template <int N>
 __device__ __forceinline__ double crt_finish_small(const unsigned long long (&acc)[4], double P_inv32, int escale) {
   static_assert(N >= kCrtMinModuli && N <= 16, "P at least 2^63 and below 2^128");
@@ -1194,15 +1235,17 @@ __device__ __forceinline__ double crt_finish_small(const unsigned long long (&ac
     const double sd = fma(fma(exact(acc[3]), 0x1p32, exact(acc[2])), 0x1p32, exact(acc[1]));
     q = uint32_t(__double2loint(fma(sd, P_inv32, 0x1.8p52)));
   }
-  constexpr uint32_t P0 = kCrtTableC.P[N][0], P1 = kCrtTableC.P[N][1], P2 = kCrtTableC.P[N][2], P3 = kCrtTableC.P[N][3];
-  const long long d0 = static_cast<long long>(acc[0]) - static_cast<long long>(static_cast<unsigned long long>(q) * P0);
-  const long long d1 = static_cast<long long>(acc[1]) - static_cast<long long>(static_cast<unsigned long long>(q) * P1) +
-                       (d0 >> 32);
-  const long long d2 = static_cast<long long>(acc[2]) - static_cast<long long>(static_cast<unsigned long long>(q) * P2) +
-                       (d1 >> 32);
-  const long long d3 = static_cast<long long>(acc[3]) - static_cast<long long>(static_cast<unsigned long long>(q) * P3) +
-                       (d2 >> 32);
-  return crt_round<N>(uint32_t(d0), uint32_t(d1), uint32_t(d2), uint32_t(d3), escale);
+  // R = S + q (2^128 - P) modulo 2^128: only additions, one multiply-add per column and the carry
+  // of the column below (each sum below 2^47)
+  constexpr unsigned __int128 kNegP =
+      0 - ((static_cast<unsigned __int128>(kCrtTableC.P[N][3]) << 96) | (static_cast<unsigned __int128>(kCrtTableC.P[N][2]) << 64) |
+           (static_cast<unsigned __int128>(kCrtTableC.P[N][1]) << 32) | kCrtTableC.P[N][0]);
+  constexpr uint32_t n0 = uint32_t(kNegP), n1 = uint32_t(kNegP >> 32), n2 = uint32_t(kNegP >> 64), n3 = uint32_t(kNegP >> 96);
+  const unsigned long long d0 = acc[0] + static_cast<unsigned long long>(q) * n0;
+  const unsigned long long d1 = acc[1] + static_cast<unsigned long long>(q) * n1 + (d0 >> 32);
+  const unsigned long long d2 = acc[2] + static_cast<unsigned long long>(q) * n2 + (d1 >> 32);
+  const uint32_t d3 = uint32_t(acc[3]) + q * n3 + uint32_t(d2 >> 32);
+  return crt_round<N>(uint32_t(d0), uint32_t(d1), uint32_t(d2), d3, escale);
 }
 
 // ---- reconstruction with the weighted residue sum on the tensor cores
@@ -1321,6 +1364,11 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
 #pragma unroll 1
       for (int s = 0; s < 4; ++s, cp += 8) {
         __syncwarp();  // lanes that kept nothing wait here for the MMAs
+        // this lane's entry: its row's exponent and old C are on their way during the byte sums
+        const int64_t ie = i0 + 8 * s + e_row;
+        const bool keep = col_ok && ie < m && (uplo == 0 || (uplo == 1 ? ie <= j : ie >= j));
+        const int mu_e = keep ? sc.mu_a[ie] : 0;
+        const double old = (keep && sc.write_c && sc.beta != 0.0) ? *cp : 0.0;
         uint32_t w[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) w[k] = 4 * c + k < N ? slot[(4 * c + k) * 32 + ((8 * s + g) ^ (8 * c))] : 0u;
@@ -1357,10 +1405,7 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
                                            static_cast<unsigned long long>(q3.x) * 65536ull + q2.x,
                                            static_cast<unsigned long long>(q1.y) * 65536ull + q0.y,
                                            static_cast<unsigned long long>(q3.y) * 65536ull + q2.y};
-        const int64_t ie = i0 + 8 * s + e_row;
-        const bool keep = col_ok && ie < m && (uplo == 0 || (uplo == 1 ? ie <= j : ie >= j));
         if (!keep) continue;
-        const int mu_e = sc.mu_a[ie];
         const double v = __dmul_rn(sc.alpha, crt_finish_small<N>(acc, P_inv32, -mu_e - nu_j));
         if (EST) {
           if (uplo != 0 && mu_e != kCrtZeroRow && nu_j != kCrtZeroRow) e_acc += exp2_int(2 * (sc.b - mu_e - nu_j));
@@ -1370,7 +1415,6 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
           if (sc.beta == 0.0) {
             *cp = v;
           } else {
-            const double old = *cp;
             if (sc.save) sc.save[j * sc.ld_save + ie] = old;
             *cp = __fma_rn(sc.beta, old, v);
           }
