@@ -344,6 +344,18 @@ __device__ __forceinline__ void cp_async_elem_if(uint32_t dst, const void* src, 
       "l"(src), "r"(index), "r"(limit), "n"(OFF), "n"(SIZE)
       : "memory");
 }
+// Zeros in that element's place under the same condition (an ordinary store).
+template <int SIZE, int OFF>
+__device__ __forceinline__ void zero_elem_if(uint32_t dst, int index, int limit) {
+  if constexpr (SIZE == 8)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %1, %2;\n\t@p st.shared.b64 [%0+%3], %4;\n\t}" ::"r"(dst),
+                 "r"(index), "r"(limit), "n"(OFF), "l"(0ull)
+                 : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %1, %2;\n\t@p st.shared.b32 [%0+%3], %4;\n\t}" ::"r"(dst),
+                 "r"(index), "r"(limit), "n"(OFF), "r"(0)
+                 : "memory");
+}
 // The same with `bytes` (0: zero fill) read.
 template <int SIZE>
 __device__ __forceinline__ void cp_async_fill_if(uint32_t dst, const void* src, int bytes, int index, int limit) {

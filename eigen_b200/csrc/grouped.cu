@@ -8,22 +8,32 @@
 //     output tile of a product; class 16 = two whole products of at most 16 x 16; class 8 =
 //     four whole products of at most 8 x 8 (Eigen's fixed-size range), so that small
 //     products share a warp instead of each filling a 32 x 32 tile;
-//   * every item is computed by ONE warp.  Its operands arrive in K-chunks ("stages") of two
-//     32-line panels (rows of op(A), columns of op(B)) copied by cp.async into a per-warp
-//     shared-memory ring with zero fill outside the products.  The copies of the next stages
-//     -- of the next item too -- are in flight while the current stage computes, which is
-//     what bounds these short, scattered products: the latency of their loads;
+//   * an FP32 item is computed by ONE warp, an FP64 item by a block of TWO (half of the fragments and
+//     one operand's copies each: half the FP64 sums per lane leaves registers for 20 warps per SM
+//     instead of 16).  Its operands arrive in K-chunks ("stages") of two
+//     32-line panels (rows of op(A), columns of op(B)) copied by cp.async into a
+//     shared-memory ring.  The copies of the next stages -- of the next item too -- are in
+//     flight while the current stage computes, which hides the latency of these short,
+//     scattered products' loads;
+//   * bound by the latency of short items (DMMA pipe 36 %, issue slots 48 % busy for FP64; issue slots
+//     51 % for FP32), so a stage carries no work for padding: lines outside the product are not copied
+//     (their outputs are not stored), only the K tail is zero-filled, and the fragments computed are
+//     those the item really has.  10,000 products of sides 3 .. 256: FP64 313.9 -> 305.1 us, FP32
+//     286.6 -> 267.8 us against one warp per item with padded fragments for both;
 //   * FP64: mma.sync m16n8k4 (DMMA), K in steps of 4 from 0 upward for every output, the
 //     same sequence as the native DGEMM kernel, so each product equals one plain native call
-//     bit for bit;  FP32: split-BF16 on the tensor cores (x = h + m + l in bf16 pieces; the
-//     six products hl, lh, mm, hm, mh, hh of every 16-deep chunk, mma.sync m16n8k16 with FP32
-//     accumulation, added to the FP32 result with round-to-nearest);
+//     bit for bit (m16n8k8 takes the same two steps in one instruction);
+//   * FP32: split-BF16 on the tensor cores (x = h + m + l in bf16 pieces; the six products hl, lh, mm,
+//     hm, mh, hh of every 8-deep chunk, mma.sync m16n8k8 with FP32 accumulation, added to the FP32
+//     result with round-to-nearest);
 //   * items are ordered longest-K first by the host and strided over the persistent warps;
 //   * C = alpha*op(A)op(B) + beta*C per problem with the BLAS rules (beta == 0 never reads
 //     C, alpha == 0 or k == 0 leaves beta*C and reads neither A nor B).
 #include <cuda_bf16.h>
 
+#include <climits>
 #include <cstdint>
+#include <utility>
 
 #include "device_common.cuh"
 #include "grouped.h"
@@ -36,26 +46,19 @@ constexpr int kLineStride = 36;  // a panel's k-row: 32 lines (rows of op(A) / c
 constexpr int kKc = 8;           // K per stage: two m16n8k4 steps (FP64) or one m16n8k8 step (FP32)
 constexpr int kWarpsPerBlock = 2;
 
-template <bool F64>
-struct GroupedTraits;
-template <>
-struct GroupedTraits<true> {
-  using T = double;
-  static constexpr int kStages = 3;  // 13.8 KB per warp: eight two-warp blocks per SM
-};
-template <>
-struct GroupedTraits<false> {
-  using T = float;
-  static constexpr int kStages = 6;  // 13.8 KB per warp
-};
+// FP64: a block of two warps shares an item and its ring; FP32: an item per warp.
+constexpr int kStages64 = 4;  // 18.4 KB per block
+constexpr int kStages32 = 6;  // 13.8 KB per warp
+constexpr int kBlocks64 = 10, kBlocks32 = 8;  // per SM
 constexpr int kPanelElems = kKc * kLineStride;
 constexpr int kStageElems = 2 * kPanelElems;
 
-__device__ __forceinline__ void dmma_16x8x4_g(double (&d)[4], double a0, double a1, double b0) {
+__device__ __forceinline__ void dmma_16x8x8_g(double (&d)[4], double a0, double a1, double a2, double a3, double b0,
+                                              double b1) {
   asm volatile(
-      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-      : "d"(a0), "d"(a1), "d"(b0));
+      : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
 }
 
 __device__ __forceinline__ void mma_bf16_1688(float (&d)[4], const uint32_t (&a)[2], uint32_t b) {
@@ -64,20 +67,28 @@ __device__ __forceinline__ void mma_bf16_1688(float (&d)[4], const uint32_t (&a)
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(b));
 }
-
-// x = h + m + l with h, m exact bf16 values and the remainder l (rounded to bf16 when packed);
-// each difference is exact in FP32 (Henry, Tang & Heinecke, ARITH 2019)
-__device__ __forceinline__ void split3(float x, float& h, float& m, float& l) {
-  h = __bfloat162float(__float2bfloat16_rn(x));
-  const float r1 = __fsub_rn(x, h);
-  m = __bfloat162float(__float2bfloat16_rn(r1));
-  l = __fsub_rn(r1, m);
+// the same from a zero accumulator
+__device__ __forceinline__ void mma_bf16_1688_fresh(float (&d)[4], const uint32_t (&a)[2], uint32_t b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(b), "f"(0.f));
 }
 
 // two values as one bf16x2 register (first value in the low half: the smaller k)
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
+}
+// x = h + m + l for two values, each piece packed as bf16x2: h, m exact bf16 values, l the rest
+// rounded to bf16; each difference is exact in FP32 (Henry, Tang & Heinecke, ARITH 2019)
+__device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+  auto low = [](uint32_t v) { return __uint_as_float(v << 16); };
+  auto high = [](uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); };
+  h = pack_bf16(x0, x1);
+  const float r0 = __fsub_rn(x0, low(h)), r1 = __fsub_rn(x1, high(h));
+  m = pack_bf16(r0, r1);
+  l = pack_bf16(__fsub_rn(r0, low(m)), __fsub_rn(r1, high(m)));
 }
 
 // The items of a launch: the plan's list (grouped launch), or the 32 x 32 tiles of one
@@ -87,8 +98,13 @@ struct PlanItems {
   const GroupedItem* items;
   int64_t count;
   __device__ __forceinline__ GroupedItem item(int64_t i) const { return items[i]; }
-  __device__ __forceinline__ GroupedProblem problem(uint32_t p) const { return problems[p]; }
+  __device__ __forceinline__ const GroupedProblem& problem(uint32_t p) const { return problems[p]; }
   __device__ __forceinline__ const void* dummy() const { return problems; }
+  // the first problem of item i, and that problem's descriptor on its way to L1
+  __device__ __forceinline__ uint32_t first_problem(int64_t i) const { return i < count ? items[i].problem[0] : 0u; }
+  __device__ __forceinline__ void prefetch(uint32_t p) const {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(problems + p));
+  }
 };
 struct OneProduct {
   GroupedProblem pr;
@@ -102,10 +118,13 @@ struct OneProduct {
     it.tile_m = uint16_t(i % tiles_m);
     it.tile_n = uint16_t(i / tiles_m);
     it.cls = 32;
+    it.frags = grouped_frags(pr.m, pr.n, it.tile_m, it.tile_n);
     return it;
   }
-  __device__ __forceinline__ GroupedProblem problem(uint32_t) const { return pr; }
+  __device__ __forceinline__ const GroupedProblem& problem(uint32_t) const { return pr; }
   __device__ __forceinline__ const void* dummy() const { return pr.c; }
+  __device__ __forceinline__ uint32_t first_problem(int64_t) const { return 0u; }
+  __device__ __forceinline__ void prefetch(uint32_t) const {}
 };
 
 __device__ __forceinline__ uint32_t slot_problem(const GroupedItem& it, int q) {
@@ -117,182 +136,181 @@ __device__ __forceinline__ uint32_t slot_problem(const GroupedItem& it, int q) {
 // the item's class: lines per problem).  Along the panel's contiguous direction consecutive
 // lanes take consecutive elements: if the lines are contiguous (op(A) not transposed, op(B)
 // transposed) lane ls takes line ls and element t is K offset t; otherwise lane ls takes K
-// offset ls % 8 of lines ls / 8 + t R/8.  Either way the address, the shared-memory slot, the
-// K offset and the line of element t are affine in t.  Extents fit 32 bits: a plan holds at
-// most 65535 tiles of 32 per side, and its items' K are 32-bit.
+// offset ls % 8 of lines ls / 8 + t R/8.  Either way the address and the shared-memory slot of
+// element t are affine in t.  A line outside the product is not copied: what its slot holds
+// reaches only outputs that are not stored.  The K tail is zero-filled.
 template <typename T>
 struct PanelCopy {
-  const T* ptr;     // element t = 0 at K chunk 0
-  int64_t ld;       // the operand's leading dimension
-  int line0, kk0;   // line and K offset of element t = 0
-  int dline;        // lines contiguous: 0 (element t is K offset kk0 + t); else R/8 (line0 + t*dline)
-  int lines, k;     // the product's extent along the lines, and its K (0: empty slot)
+  static constexpr int kSize = int(sizeof(T));
+  const char* ptr;  // element t = 0 of the next stage
+  int64_t step;     // bytes from element t to t + 1
   uint32_t dst0;    // shared-memory byte offset of element t = 0 within the panel
+  int valid;        // the elements t < valid lie on lines of the product
 
-  __device__ __forceinline__ void set(const T* base, int64_t ldx, bool lines_contig, int first_line, int slot_off,
-                                      int ls, int r, int64_t extent, int64_t kdim) {
-    ld = ldx;
-    lines = int(extent);
-    k = int(kdim);
-    if (lines_contig) {  // X(line, kk) = base[line + kk * ld]
-      line0 = first_line + ls;
-      dline = 0;
-      kk0 = 0;
-      ptr = base + line0;
-      dst0 = uint32_t((slot_off + ls) * sizeof(T));
+  __device__ __forceinline__ void set(const T* base, int64_t ldx, bool contig, int first_line, int slot_off, int ls,
+                                      int r, int64_t extent) {
+    if (contig) {  // X(line, kk) = base[line + kk * ld]
+      const int line0 = first_line + ls;
+      ptr = reinterpret_cast<const char*>(base + line0);
+      step = ldx * kSize;
+      dst0 = uint32_t((slot_off + ls) * kSize);
+      valid = line0 < extent ? kKc : 0;
     } else {  // X(line, kk) = base[kk + line * ld]
-      line0 = first_line + ls / kKc;
-      dline = r / kKc;
-      kk0 = ls % kKc;
-      ptr = base + kk0 + int64_t(line0) * ld;
-      dst0 = uint32_t((kk0 * kLineStride + slot_off + ls / kKc) * sizeof(T));
+      const int line0 = first_line + ls / kKc, dline = r / kKc, kk0 = ls % kKc;
+      ptr = reinterpret_cast<const char*>(base + kk0 + int64_t(line0) * ldx);
+      step = int64_t(dline) * ldx * kSize;
+      dst0 = uint32_t((kk0 * kLineStride + slot_off + ls / kKc) * kSize);
+      const int64_t rest = extent - line0;
+      valid = rest <= 0 ? 0 : (rest > (kKc - 1) * dline ? kKc : (int(rest) + dline - 1) / dline);
     }
   }
 
-  __device__ __forceinline__ void issue(uint32_t panel, int k0, const void* dummy) const {
-    const bool contig = dline == 0;
-    const int dkk = contig ? 1 : 0;
-    const int64_t step_t = contig ? ld : int64_t(dline) * ld;
-    const uint32_t dst_step = uint32_t((contig ? kLineStride : dline) * sizeof(T));
-    const T* p = ptr + (contig ? int64_t(k0) * ld : int64_t(k0));
-    // the whole stage inside the product: no per-element checks
-    const bool inside = k0 + kk0 + (kKc - 1) * dkk < k && line0 + (kKc - 1) * dline < lines;
-    uint32_t d = panel + dst0;
-    if (inside) {
-#pragma unroll
-      for (int t = 0; t < kKc; ++t, p += step_t, d += dst_step) cp_async_elem<sizeof(T)>(d, p, true);
+  // A stage of a class-32 item, the slots DSTEP bytes apart: one address and one predicated copy per
+  // element.  CONTIG: the first `left` elements lie inside K (all lanes alike); else a lane's K offset
+  // is inside or not.  What lies past K is zeroed.
+  template <bool CONTIG, int DSTEP, int... t>
+  __device__ __forceinline__ void issue_wide(uint32_t d, int left, std::integer_sequence<int, t...>) const {
+    const uint32_t st = uint32_t(step);
+    if (left >= kKc) {
+      (cp_async_elem_if<kSize, t * DSTEP>(d, ptr + uint64_t(st) * uint32_t(t), t, valid), ...);
+    } else if constexpr (CONTIG) {
+      ((t < left ? cp_async_elem_if<kSize, t * DSTEP>(d, ptr + uint64_t(st) * uint32_t(t), t, valid)
+                 : zero_elem_if<kSize, t * DSTEP>(d, t, valid)),
+       ...);
     } else {
-#pragma unroll
-      for (int t = 0; t < kKc; ++t, p += step_t, d += dst_step) {
-        const bool v = k0 + kk0 + t * dkk < k && line0 + t * dline < lines;
-        cp_async_elem<sizeof(T)>(d, v ? static_cast<const void*>(p) : dummy, v);
+      const bool in = int(threadIdx.x) % kKc < left;
+      const int copied = in ? valid : 0, zeroed = in ? 0 : valid;
+      (cp_async_elem_if<kSize, t * DSTEP>(d, ptr + uint64_t(st) * uint32_t(t), t, copied), ...);
+      (zero_elem_if<kSize, t * DSTEP>(d, t, zeroed), ...);
+    }
+  }
+
+  // `contig`: the lines are contiguous (element t is K offset t); `left`: K from the stage's start to
+  // the end; `wide`: class 32 and the step fits 32 bits (`left` and `contig` are then the warp's).
+  __device__ __forceinline__ void issue(uint32_t panel, const void* dummy, bool contig, int left, int r, bool wide) {
+    const uint32_t d = panel + dst0;
+    if (wide) {
+      using Seq = std::make_integer_sequence<int, kKc>;
+      if (contig)
+        issue_wide<true, kLineStride * kSize>(d, left, Seq{});
+      else
+        issue_wide<false, 32 / kKc * kSize>(d, left, Seq{});
+    } else {
+      const char* p = ptr;
+      uint32_t dt = d;
+      const uint32_t dstep = uint32_t((contig ? kLineStride : r / kKc) * kSize);
+      const int kk0 = contig ? 0 : int(threadIdx.x) % kKc;  // ls % kKc: R is a multiple of kKc
+#pragma unroll 2
+      for (int t = 0; t < kKc; ++t, p += step, dt += dstep) {
+        const bool in = kk0 + (contig ? t : 0) < left;
+        cp_async_fill_if<kSize>(dt, in ? static_cast<const void*>(p) : dummy, in ? kSize : 0, t, valid);
       }
     }
+    ptr += contig ? kKc * step : int64_t(kKc * kSize);
   }
 };
 
-// The copies of one stage of an item for one lane: its slot's rows of op(A) and columns of op(B).
-template <bool F64, class Src>
-struct StageCopier {
-  using T = typename GroupedTraits<F64>::T;
-  PanelCopy<T> pa, pb;
-  const void* dummy;
+// The copies of an item's stages for one lane: its slot's rows of op(A) and / or columns of op(B).
+template <typename T>
+struct ItemCopy {
+  int left;      // K of the lane's product from the next stage on
+  uint32_t how;  // the item's class, | 64: op(A)'s lines contiguous, | 128: op(B)'s, | 256: wide
 
-  __device__ __forceinline__ void load(const Src& src, const GroupedItem& it, int lane) {
+  template <class Src>
+  __device__ __forceinline__ void open(const Src& src, const GroupedItem& it, int lane, PanelCopy<T>* pa,
+                                       PanelCopy<T>* pb) {
     const int r = it.cls;
     const int log_r = r == 8 ? 3 : (r == 16 ? 4 : 5);
     const int q = lane >> log_r;
     const int ls = lane & (r - 1);
-    dummy = src.dummy();
     const uint32_t pid = slot_problem(it, q);
     const bool ok = pid != kNoProblem;
-    const GroupedProblem pr = ok ? src.problem(pid) : GroupedProblem{};
-    const T* a = static_cast<const T*>(ok ? pr.a : dummy);
-    const T* b = static_cast<const T*>(ok ? pr.b : dummy);
-    const int first_a = r == 32 ? int(it.tile_m) * 32 : 0, first_b = r == 32 ? int(it.tile_n) * 32 : 0;
+    const GroupedProblem& pr = src.problem(ok ? pid : it.problem[0]);
+    left = ok ? int(pr.k < INT_MAX ? pr.k : INT_MAX) : 0;
     // op(A)(i, l): contiguous along i unless transposed; op(B)(l, j): along j only if transposed
-    pa.set(a, pr.lda, (pr.trans & 1) == 0, first_a, q * r, ls, r, ok ? pr.m : 0, ok ? pr.k : 0);
-    pb.set(b, pr.ldb, (pr.trans & 2) != 0, first_b, q * r, ls, r, ok ? pr.n : 0, ok ? pr.k : 0);
+    const bool ca = (pr.trans & 1) == 0, cb = (pr.trans & 2) != 0;
+    bool narrow = true;
+    if (pa) {
+      pa->set(static_cast<const T*>(pr.a), pr.lda, ca, r == 32 ? int(it.tile_m) * 32 : 0, q * r, ls, r, ok ? pr.m : 0);
+      narrow = narrow && pa->step <= INT_MAX;
+    }
+    if (pb) {
+      pb->set(static_cast<const T*>(pr.b), pr.ldb, cb, r == 32 ? int(it.tile_n) * 32 : 0, q * r, ls, r, ok ? pr.n : 0);
+      narrow = narrow && pb->step <= INT_MAX;
+    }
+    how = uint32_t(r) | (ca ? 64u : 0u) | (cb ? 128u : 0u) | (r == 32 && narrow ? 256u : 0u);
   }
-
-  __device__ __forceinline__ void issue(T* stage, int k0) const {
-    const uint32_t sa = static_cast<uint32_t>(__cvta_generic_to_shared(stage));
-    pa.issue(sa, k0, dummy);
-    pb.issue(sa + uint32_t(kPanelElems * sizeof(T)), k0, dummy);
+  __device__ __forceinline__ void issue(PanelCopy<T>& p, const T* panel, bool rhs, const void* dummy) const {
+    p.issue(smem_u32(panel), dummy, (how & (rhs ? 128u : 64u)) != 0u, left, int(how & 63u), (how & 256u) != 0u);
   }
 };
 
-// ---------------------------------------------------------------- FP64 compute
-// Accumulator fragments: class 32: (row block i, column block j) -> i*4 + j; class 16:
-// (problem p, column block j) -> p*2 + j; class 8: problem p -> p (rows 8-15 unused).
-__device__ __forceinline__ void compute_f64(double (&acc)[8][4], const double* st, int cls, int g, int tig) {
-  const double* sA = st;
-  const double* sB = st + kPanelElems;
-#pragma unroll
-  for (int ks = 0; ks < 2; ++ks) {
-    const int kr = (ks * 4 + tig) * kLineStride;
-    if (cls == 32) {
-      double a[2][2], b[4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        a[i][0] = sA[kr + i * 16 + g];
-        a[i][1] = sA[kr + i * 16 + g + 8];
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = sB[kr + j * 8 + g];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma_16x8x4_g(acc[i * 4 + j], a[i][0], a[i][1], b[j]);
-    } else if (cls == 16) {
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        const double a0 = sA[kr + p * 16 + g], a1 = sA[kr + p * 16 + g + 8];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) dmma_16x8x4_g(acc[p * 2 + j], a0, a1, sB[kr + p * 16 + j * 8 + g]);
-      }
-    } else {
-#pragma unroll
-      for (int p = 0; p < 4; ++p) dmma_16x8x4_g(acc[p], sA[kr + p * 8 + g], 0.0, sB[kr + p * 8 + g]);
-    }
-  }
+__device__ __forceinline__ int item_stages(const GroupedItem& it) {
+  return it.k > 0 ? (int(it.k) + kKc - 1) / kKc : 1;
 }
 
-// ---------------------------------------------------------------- FP32 (split-BF16) compute
-// The m16n8k8 A fragment of the 16 lines at l0 (rows 8-15 zero when `half`) and the B
+// ---------------------------------------------------------------- FP64 compute
+// NJ 8-column fragments of one 16-row block: sA, sB at the lane's K offset tig, row g / column g of
+// the first fragment.  The m16n8k8 fragments are two m16n8k4 steps' taken in K order (same bits).
+template <int NJ>
+__device__ __forceinline__ void stage_f64(double (&acc)[4][4], const double* sA, const double* sB) {
+  const double a0 = sA[0], a1 = sA[8], a2 = sA[4 * kLineStride], a3 = sA[4 * kLineStride + 8];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j)
+    dmma_16x8x8_g(acc[j], a0, a1, a2, a3, sB[j * 8], sB[4 * kLineStride + j * 8]);
+}
+
+// ---------------------------------------------------------------- FP32 compute
+// Accumulator fragments: class 32: (row block i, column block j) -> i*4 + j; class 16:
+// (problem p, column block j) -> p*2 + j; class 8: problem p -> p (rows 8-15 unused).
+//
+// FP32: the m16n8k8 A fragment of the 16 lines at l0 (rows 8-15 zero when `half`) and the B
 // fragment of the 8 lines at l0, each as its three bf16 pieces.
 __device__ __forceinline__ void frag_a(const float* sA, int l0, bool half, int g, int tig, uint32_t (&p)[3][2]) {
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    const int row = l0 + g + 8 * r;
-    const bool zero = half && r == 1;
-    const float x0 = zero ? 0.f : sA[(2 * tig) * kLineStride + row];
-    const float x1 = zero ? 0.f : sA[(2 * tig + 1) * kLineStride + row];
-    float h0, m0, l0v, h1, m1, l1v;
-    split3(x0, h0, m0, l0v);
-    split3(x1, h1, m1, l1v);
-    p[0][r] = pack_bf16(h0, h1);
-    p[1][r] = pack_bf16(m0, m1);
-    p[2][r] = pack_bf16(l0v, l1v);
+    p[0][r] = p[1][r] = p[2][r] = 0u;
+    const float* x = sA + (2 * tig) * kLineStride + l0 + g + 8 * r;
+    if (!(half && r == 1)) split_pair(x[0], x[kLineStride], p[0][r], p[1][r], p[2][r]);
   }
 }
 __device__ __forceinline__ void frag_b(const float* sB, int l0, int g, int tig, uint32_t (&p)[3]) {
-  float h0, m0, x0, h1, m1, x1;
-  split3(sB[(2 * tig) * kLineStride + l0 + g], h0, m0, x0);
-  split3(sB[(2 * tig + 1) * kLineStride + l0 + g], h1, m1, x1);
-  p[0] = pack_bf16(h0, h1);
-  p[1] = pack_bf16(m0, m1);
-  p[2] = pack_bf16(x0, x1);
+  const float* x = sB + (2 * tig) * kLineStride + l0 + g;
+  split_pair(x[0], x[kLineStride], p[0], p[1], p[2]);
 }
 // the six piece products of one 8-deep chunk, smallest first, into a fresh fragment that is
 // then added to the result (round to nearest)
 __device__ __forceinline__ void chunk_product(float (&acc)[4], const uint32_t (&pa)[3][2], const uint32_t (&pb)[3]) {
-  float d[4] = {0.f, 0.f, 0.f, 0.f};
-  mma_bf16_1688(d, pa[0], pb[2]);  // h l
-  mma_bf16_1688(d, pa[2], pb[0]);  // l h
-  mma_bf16_1688(d, pa[1], pb[1]);  // m m
-  mma_bf16_1688(d, pa[0], pb[1]);  // h m
-  mma_bf16_1688(d, pa[1], pb[0]);  // m h
-  mma_bf16_1688(d, pa[0], pb[0]);  // h h
+  float d[4];
+  mma_bf16_1688_fresh(d, pa[0], pb[2]);  // h l
+  mma_bf16_1688(d, pa[2], pb[0]);        // l h
+  mma_bf16_1688(d, pa[1], pb[1]);        // m m
+  mma_bf16_1688(d, pa[0], pb[1]);        // h m
+  mma_bf16_1688(d, pa[1], pb[0]);        // m h
+  mma_bf16_1688(d, pa[0], pb[0]);        // h h
 #pragma unroll
   for (int e = 0; e < 4; ++e) acc[e] = __fadd_rn(acc[e], d[e]);
 }
+// MI row blocks (of 16) by NJ column blocks (of 8) of a class-32 stage.
+template <int MI, int NJ>
+__device__ __forceinline__ void stage32(float (&acc)[8][4], const float* st, int g, int tig) {
+  uint32_t pa[MI][3][2];
+#pragma unroll
+  for (int i = 0; i < MI; ++i) frag_a(st, i * 16, false, g, tig, pa[i]);
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    uint32_t pb[3];
+    frag_b(st + kPanelElems, j * 8, g, tig, pb);
+#pragma unroll
+    for (int i = 0; i < MI; ++i) chunk_product(acc[i * 4 + j], pa[i], pb);
+  }
+}
 
-__device__ __forceinline__ void compute_f32(float (&acc)[8][4], const float* st, int cls, int g, int tig) {
+// A stage of two products of at most 16 x 16, or of four of at most 8 x 8.
+__device__ __forceinline__ void stage_small(float (&acc)[8][4], const float* st, bool mid, int g, int tig) {
   const float* sA = st;
   const float* sB = st + kPanelElems;
-  if (cls == 32) {
-    uint32_t pa[2][3][2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) frag_a(sA, i * 16, false, g, tig, pa[i]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint32_t pb[3];
-      frag_b(sB, j * 8, g, tig, pb);
-#pragma unroll
-      for (int i = 0; i < 2; ++i) chunk_product(acc[i * 4 + j], pa[i], pb);
-    }
-  } else if (cls == 16) {
+  if (mid) {
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       uint32_t pa[3][2];
@@ -315,11 +333,27 @@ __device__ __forceinline__ void compute_f32(float (&acc)[8][4], const float* st,
   }
 }
 
+// One stage of an item: the fragments it has (grouped_frags), nothing for padding.
+__device__ __forceinline__ void compute_stage(float (&acc)[8][4], const float* st, const GroupedItem& it, int g,
+                                              int tig) {
+  if (it.cls != 32) return stage_small(acc, st, it.cls == 16, g, tig);
+  switch (it.frags) {
+    case 0: return stage32<1, 1>(acc, st, g, tig);
+    case 1: return stage32<1, 2>(acc, st, g, tig);
+    case 2: return stage32<1, 3>(acc, st, g, tig);
+    case 3: return stage32<1, 4>(acc, st, g, tig);
+    case 4: return stage32<2, 1>(acc, st, g, tig);
+    case 5: return stage32<2, 2>(acc, st, g, tig);
+    case 6: return stage32<2, 3>(acc, st, g, tig);
+    default: return stage32<2, 4>(acc, st, g, tig);
+  }
+}
+
 // ---------------------------------------------------------------- epilogue
 // C = alpha * acc + beta * C for the fragment elements of one product: element (h, c) of the
 // fragment at rows r0.., columns c0.. is row r0 + g + 8h, column c0 + 2 tig + c.  The
 // descriptor's fields are copied to registers first (C stores could otherwise alias them).
-template <typename T, int NF>
+template <typename T>
 struct ProductStore {
   T* c;
   int64_t ldc, m, n;
@@ -333,29 +367,49 @@ struct ProductStore {
     beta = T(pr.beta);
   }
   __device__ __forceinline__ void put(int64_t row, int64_t col, T v) const {
-    if (row < m && col < n) {
-      T* dst = c + row + col * ldc;
-      const T a = sizeof(T) == 8 ? T(__dmul_rn(double(alpha), double(v))) : T(__fmul_rn(float(alpha), float(v)));
-      if (beta == T(0))
-        *dst = a;
-      else if constexpr (sizeof(T) == 8)
-        *dst = __fma_rn(double(beta), double(*dst), double(a));
-      else
-        *dst = __fmaf_rn(float(beta), float(*dst), float(a));
-    }
+    if (row < m && col < n) put_at(c + row + col * ldc, v);
+  }
+  __device__ __forceinline__ void put_at(T* dst, T v) const {
+    const T a = sizeof(T) == 8 ? T(__dmul_rn(double(alpha), double(v))) : T(__fmul_rn(float(alpha), float(v)));
+    if (beta == T(0))
+      *dst = a;
+    else if constexpr (sizeof(T) == 8)
+      *dst = __fma_rn(double(beta), double(*dst), double(a));
+    else
+      *dst = __fmaf_rn(float(beta), float(*dst), float(a));
   }
 };
 
-template <typename T, class Src>
-__device__ __forceinline__ void epilogue(const Src& src, const GroupedItem& it, T (&acc)[8][4], int g, int tig) {
-  ProductStore<T, 8> ps;
+// C of NJ column fragments of ROWS rows: element e of fragment j of row block h is row 16h + 8 (e / 2),
+// column 8j + e % 2 from (r0, c0), the lane's first place.
+template <int H, int NJ, typename T, int F>
+__device__ __forceinline__ void store_tile(const ProductStore<T>& ps, int64_t r0, int64_t c0, int nj,
+                                           const T (&acc)[F][4]) {
+  const int64_t rest_r = ps.m - r0, rest_c = ps.n - c0;
+  const int rows = int(rest_r < 32 ? rest_r : 32), cols = int(rest_c < 32 ? rest_c : 32);
+  T* cp = ps.c + r0 + c0 * ps.ldc;
+  const int64_t next = 7 * ps.ldc;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j, cp += next) {
+    if (j >= nj) break;  // not computed
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (8 * j + c < cols) {
+#pragma unroll
+        for (int h = 0; h < 2 * H; ++h)
+          if (8 * h < rows) ps.put_at(cp + 8 * h, acc[(h >> 1) * NJ + j][(h & 1) * 2 + c]);
+      }
+      if (c == 0) cp += ps.ldc;
+    }
+  }
+}
+
+template <class Src>
+__device__ __forceinline__ void epilogue_f32(const Src& src, const GroupedItem& it, float (&acc)[8][4], int g, int tig) {
+  ProductStore<float> ps;
   if (it.cls == 32) {
     ps.load(src.problem(it.problem[0]));
-    const int64_t r0 = int64_t(it.tile_m) * 32 + g, c0 = int64_t(it.tile_n) * 32 + 2 * tig;
-#pragma unroll
-    for (int f = 0; f < 8; ++f)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) ps.put(r0 + (f >> 2) * 16 + (e >> 1) * 8, c0 + (f & 3) * 8 + (e & 1), acc[f][e]);
+    store_tile<2, 4>(ps, int64_t(it.tile_m) * 32 + g, int64_t(it.tile_n) * 32 + 2 * tig, (it.frags & 3) + 1, acc);
   } else if (it.cls == 16) {
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
@@ -379,38 +433,41 @@ __device__ __forceinline__ void epilogue(const Src& src, const GroupedItem& it, 
   }
 }
 
-// ---------------------------------------------------------------- the warp's pipeline
-// Items w0, w0 + W, w0 + 2W, ... in stage order; copies run kStages - 1 stages ahead of the
+// ---------------------------------------------------------------- FP32: a warp's pipeline
+// Items w0, w0 + W, w0 + 2W, ... in stage order; copies run kStages32 - 1 stages ahead of the
 // compute, across item boundaries.
-template <bool F64, class Src>
-__device__ __forceinline__ void run_items(const Src& src, int64_t w0, int64_t W,
-                                          typename GroupedTraits<F64>::T* ring) {
-  using T = typename GroupedTraits<F64>::T;
-  constexpr int S = GroupedTraits<F64>::kStages;
+template <class Src>
+__device__ __forceinline__ void run_items_f32(const Src& src, int64_t w0, int64_t W, float* ring) {
+  constexpr int S = kStages32;
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
-  auto stages_of = [](const GroupedItem& it) { return it.k > 0 ? (int(it.k) + kKc - 1) / kKc : 1; };
 
   // producer position
   int64_t p_idx = w0;
-  int p_stage = 0, p_stages = 0;
-  StageCopier<F64, Src> cp;
-  if (p_idx < src.count) {
+  int p_left = 0;  // stages of the producer's item still to copy
+  uint32_t p_next = 0;  // first problem of its next item
+  ItemCopy<float> cp;
+  PanelCopy<float> pa, pb;
+  auto open_item = [&]() {
     const GroupedItem it = src.item(p_idx);
-    cp.load(src, it, lane);
-    p_stages = stages_of(it);
-  }
+    cp.open(src, it, lane, &pa, &pb);
+    p_left = item_stages(it);
+    // the next item's record comes to L1 with this read, its problem one stage later
+    p_next = src.first_problem(p_idx + W);
+  };
+  if (p_idx < src.count) open_item();
+  const void* const dummy = src.dummy();
   auto produce = [&](int slot) {
     if (p_idx < src.count) {
-      cp.issue(ring + slot * kStageElems, p_stage * kKc);
-      if (++p_stage == p_stages) {
-        p_stage = 0;
+      const float* stage = ring + slot * kStageElems;
+      cp.issue(pa, stage, false, dummy);
+      cp.issue(pb, stage + kPanelElems, true, dummy);
+      cp.left -= kKc;
+      if (--p_left == 0) {
         p_idx += W;
-        if (p_idx < src.count) {
-          const GroupedItem it = src.item(p_idx);
-          cp.load(src, it, lane);
-          p_stages = stages_of(it);
-        }
+        if (p_idx < src.count) open_item();
+      } else if (p_left == 1) {
+        src.prefetch(p_next);
       }
     }
     cp_async_commit();  // an empty group past the end keeps the group count uniform
@@ -420,70 +477,190 @@ __device__ __forceinline__ void run_items(const Src& src, int64_t w0, int64_t W,
 
   // consumer position
   int64_t c_idx = w0;
-  int c_stage = 0;
-  GroupedItem cur{};
   int c_stages = 0;
+  GroupedItem cur{};
   if (c_idx < src.count) {
     cur = src.item(c_idx);
-    c_stages = stages_of(cur);
+    c_stages = item_stages(cur);
   }
-  T acc[8][4];
+  float acc[8][4];
 #pragma unroll
   for (int f = 0; f < 8; ++f)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc[f][e] = T(0);
+    for (int e = 0; e < 4; ++e) acc[f][e] = 0.f;
   int slot = 0;
   while (c_idx < src.count) {
     cp_async_wait<S - 2>();
     __syncwarp();  // every lane's copies of this stage have landed; the slot refilled below is free
     produce(slot == 0 ? S - 1 : slot - 1);
-    const T* st = ring + slot * kStageElems;
-    if constexpr (F64)
-      compute_f64(acc, st, cur.cls, g, tig);
-    else
-      compute_f32(acc, st, cur.cls, g, tig);
+    compute_stage(acc, ring + slot * kStageElems, cur, g, tig);
     slot = slot == S - 1 ? 0 : slot + 1;
-    if (++c_stage == c_stages) {
-      epilogue(src, cur, acc, g, tig);
+    if (--c_stages == 0) {
+      epilogue_f32(src, cur, acc, g, tig);
 #pragma unroll
       for (int f = 0; f < 8; ++f)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[f][e] = T(0);
-      c_stage = 0;
+        for (int e = 0; e < 4; ++e) acc[f][e] = 0.f;
       c_idx += W;
       if (c_idx < src.count) {
         cur = src.item(c_idx);
-        c_stages = stages_of(cur);
+        c_stages = item_stages(cur);
       }
     }
   }
   cp_async_wait<0>();  // no copy may outlive the warp (the trailing groups are empty)
 }
 
-template <bool F64>
-constexpr size_t warp_ring_bytes() {
-  return size_t(GroupedTraits<F64>::kStages) * kStageElems * sizeof(typename GroupedTraits<F64>::T);
+// ---------------------------------------------------------------- FP64: a block's pipeline
+// The same order for a block of two warps: warp 0 copies the items' rows of op(A), warp 1 their
+// columns of op(B); each computes half of the fragments: a 16-row block of a 32 x 32 tile (or half
+// of its columns when it has one row block), one of two products, two of four.  Half the FP64 sums
+// per lane leaves registers for 20 warps per SM instead of 16, with half the copies each.
+template <class Src>
+__device__ __forceinline__ void run_items_f64(const Src& src, int64_t w0, int64_t W, double* ring) {
+  constexpr int S = kStages64;
+  const int warp = int(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int g = lane >> 2, tig = lane & 3;
+
+  int64_t p_idx = w0;
+  int p_left = 0;
+  uint32_t p_next = 0;
+  ItemCopy<double> cp;
+  PanelCopy<double> pc;  // the warp's operand
+  auto open_item = [&]() {
+    const GroupedItem it = src.item(p_idx);
+    cp.open(src, it, lane, warp == 0 ? &pc : nullptr, warp == 0 ? nullptr : &pc);
+    p_left = item_stages(it);
+    p_next = src.first_problem(p_idx + W);
+  };
+  if (p_idx < src.count) open_item();
+  const void* const dummy = src.dummy();
+  auto produce = [&](int slot) {
+    if (p_idx < src.count) {
+      cp.issue(pc, ring + slot * kStageElems + warp * kPanelElems, warp != 0, dummy);
+      cp.left -= kKc;
+      if (--p_left == 0) {
+        p_idx += W;
+        if (p_idx < src.count) open_item();
+      } else if (p_left == 1) {
+        src.prefetch(p_next);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < S - 1; ++s) produce(s);
+
+  int64_t c_idx = w0;
+  int c_stages = 0;
+  GroupedItem cur{};
+  // the warp's part of the item: fragments of row block rb from column block j0, nj of them (class 8:
+  // one column block of products 2 warp and 2 warp + 1)
+  int rb = 0, j0 = 0, nj = 0;
+  auto take = [&]() {
+    cur = src.item(c_idx);
+    c_stages = item_stages(cur);
+    const int n = (cur.frags & 3) + 1;
+    if (cur.cls == 16) {
+      rb = warp;
+      j0 = 2 * warp;
+      nj = 2;
+    } else if (cur.cls == 8 || (cur.frags & 4)) {
+      rb = warp;
+      j0 = 0;
+      nj = cur.cls == 8 ? 0 : n;
+    } else {
+      rb = 0;
+      j0 = warp ? (n + 1) / 2 : 0;
+      nj = warp ? n / 2 : (n + 1) / 2;
+    }
+  };
+  if (c_idx < src.count) take();
+  double acc[4][4];
+#pragma unroll
+  for (int f = 0; f < 4; ++f)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[f][e] = 0.0;
+  int slot = 0;
+  while (c_idx < src.count) {
+    cp_async_wait<S - 2>();
+    __syncthreads();  // both warps' copies of this stage have landed; the slot refilled below is free
+    produce(slot == 0 ? S - 1 : slot - 1);
+    const double* st = ring + slot * kStageElems + tig * kLineStride + g;
+    if (cur.cls == 8) {
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const double* x = st + (2 * warp + p) * 8;
+        dmma_16x8x8_g(acc[p], x[0], 0.0, x[4 * kLineStride], 0.0, x[kPanelElems], x[kPanelElems + 4 * kLineStride]);
+      }
+    } else {
+      const double *sA = st + 16 * rb, *sB = st + kPanelElems + 8 * j0;
+      switch (nj) {
+        case 1: stage_f64<1>(acc, sA, sB); break;
+        case 2: stage_f64<2>(acc, sA, sB); break;
+        case 3: stage_f64<3>(acc, sA, sB); break;
+        case 4: stage_f64<4>(acc, sA, sB); break;
+        default: break;
+      }
+    }
+    slot = slot == S - 1 ? 0 : slot + 1;
+    if (--c_stages == 0) {
+      ProductStore<double> ps;
+      if (cur.cls == 32) {
+        ps.load(src.problem(cur.problem[0]));
+        store_tile<1, 4>(ps, int64_t(cur.tile_m) * 32 + 16 * rb + g, int64_t(cur.tile_n) * 32 + 8 * j0 + 2 * tig, nj, acc);
+      } else if (cur.cls == 16) {
+        const uint32_t pid = warp == 0 ? cur.problem[0] : cur.problem[1];
+        if (pid != kNoProblem) {
+          ps.load(src.problem(pid));
+          store_tile<1, 4>(ps, g, 2 * tig, 2, acc);
+        }
+      } else {
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const uint32_t pid = slot_problem(cur, 2 * warp + p);
+          if (pid == kNoProblem) continue;
+          ps.load(src.problem(pid));
+#pragma unroll
+          for (int e = 0; e < 2; ++e) ps.put(g, tig * 2 + e, acc[p][e]);
+        }
+      }
+#pragma unroll
+      for (int f = 0; f < 4; ++f)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[f][e] = 0.0;
+      c_idx += W;
+      if (c_idx < src.count) take();
+    }
+  }
+  cp_async_wait<0>();
 }
 
-template <bool F64>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 8) grouped_gemm_kernel(const GroupedProblem* __restrict__ problems,
-                                                                          const GroupedItem* __restrict__ items,
-                                                                          int64_t num_items) {
+constexpr size_t kRing64 = size_t(kStages64) * kStageElems * sizeof(double);
+constexpr size_t kRing32 = size_t(kStages32) * kStageElems * sizeof(float);
+
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, kBlocks64)
+    grouped_f64_kernel(const GroupedProblem* __restrict__ problems, const GroupedItem* __restrict__ items,
+                       int64_t num_items) {
   extern __shared__ __align__(16) unsigned char grouped_smem[];
-  using T = typename GroupedTraits<F64>::T;
+  run_items_f64(PlanItems{problems, items, num_items}, int64_t(blockIdx.x), int64_t(gridDim.x),
+                reinterpret_cast<double*>(grouped_smem));
+}
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, kBlocks32)
+    grouped_f32_kernel(const GroupedProblem* __restrict__ problems, const GroupedItem* __restrict__ items,
+                       int64_t num_items) {
+  extern __shared__ __align__(16) unsigned char grouped_smem[];
   const int warp = threadIdx.x >> 5;
-  T* ring = reinterpret_cast<T*>(grouped_smem) + size_t(warp) * GroupedTraits<F64>::kStages * kStageElems;
-  const PlanItems src{problems, items, num_items};
-  run_items<F64>(src, int64_t(blockIdx.x) * kWarpsPerBlock + warp, int64_t(gridDim.x) * kWarpsPerBlock, ring);
+  run_items_f32(PlanItems{problems, items, num_items}, int64_t(blockIdx.x) * kWarpsPerBlock + warp,
+                int64_t(gridDim.x) * kWarpsPerBlock,
+                reinterpret_cast<float*>(grouped_smem) + size_t(warp) * kStages32 * kStageElems);
 }
 
-// One product, one warp per 32 x 32 tile: the per-product launches of the same arithmetic.
-template <bool F64>
+// One FP32 product, one warp per 32 x 32 tile: the per-product launches of the same arithmetic.
 __global__ void __launch_bounds__(32) grouped_one_kernel(const GroupedProblem pr, int tiles_m, int64_t tiles) {
   extern __shared__ __align__(16) unsigned char grouped_smem[];
-  using T = typename GroupedTraits<F64>::T;
-  const OneProduct src{pr, tiles_m, tiles};
-  run_items<F64>(src, int64_t(blockIdx.x), int64_t(gridDim.x), reinterpret_cast<T*>(grouped_smem));
+  run_items_f32(OneProduct{pr, tiles_m, tiles}, int64_t(blockIdx.x), int64_t(gridDim.x),
+                reinterpret_cast<float*>(grouped_smem));
 }
 
 cudaError_t set_smem(const void* kern, size_t bytes) {
@@ -492,21 +669,20 @@ cudaError_t set_smem(const void* kern, size_t bytes) {
 
 }  // namespace
 
-size_t grouped_block_smem(bool f64) {
-  return kWarpsPerBlock * (f64 ? warp_ring_bytes<true>() : warp_ring_bytes<false>());
-}
+size_t grouped_block_smem(bool f64) { return f64 ? kRing64 : kWarpsPerBlock * kRing32; }
 
 cudaError_t grouped_grid(bool f64, int64_t num_items, int num_sms, unsigned* blocks) {
   *blocks = 0;
   const size_t smem = grouped_block_smem(f64);
-  const void* kern = f64 ? reinterpret_cast<const void*>(grouped_gemm_kernel<true>)
-                         : reinterpret_cast<const void*>(grouped_gemm_kernel<false>);
+  const void* kern =
+      f64 ? reinterpret_cast<const void*>(grouped_f64_kernel) : reinterpret_cast<const void*>(grouped_f32_kernel);
   cudaError_t e = set_smem(kern, smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarpsPerBlock, smem);
   if (e != cudaSuccess) return e;
-  int64_t b = (num_items + kWarpsPerBlock - 1) / kWarpsPerBlock;
+  const int64_t per_block = f64 ? 1 : kWarpsPerBlock;  // items at a time
+  int64_t b = (num_items + per_block - 1) / per_block;
   const int64_t cap = int64_t(num_sms) * (per_sm > 0 ? per_sm : 1);
   if (b > cap) b = cap;
   *blocks = unsigned(b > 0 ? b : 0);
@@ -518,26 +694,21 @@ cudaError_t launch_grouped_gemm(bool f64, const GroupedProblem* problems, const 
   if (num_items <= 0 || blocks == 0) return cudaSuccess;
   const size_t smem = grouped_block_smem(f64);
   if (f64)
-    grouped_gemm_kernel<true><<<blocks, 32 * kWarpsPerBlock, smem, stream>>>(problems, items, num_items);
+    grouped_f64_kernel<<<blocks, 32 * kWarpsPerBlock, smem, stream>>>(problems, items, num_items);
   else
-    grouped_gemm_kernel<false><<<blocks, 32 * kWarpsPerBlock, smem, stream>>>(problems, items, num_items);
+    grouped_f32_kernel<<<blocks, 32 * kWarpsPerBlock, smem, stream>>>(problems, items, num_items);
   return cudaGetLastError();
 }
 
-cudaError_t launch_grouped_one(bool f64, const GroupedProblem& pr, cudaStream_t stream) {
+cudaError_t launch_grouped_one(const GroupedProblem& pr, cudaStream_t stream) {
   if (pr.m <= 0 || pr.n <= 0) return cudaSuccess;
   const int64_t tm = (pr.m + 31) / 32, tn = (pr.n + 31) / 32;
   if (tm > 65535 || tn > 65535) return cudaErrorInvalidValue;
-  const size_t smem = f64 ? warp_ring_bytes<true>() : warp_ring_bytes<false>();
-  cudaError_t e = f64 ? set_smem(reinterpret_cast<const void*>(grouped_one_kernel<true>), smem)
-                      : set_smem(reinterpret_cast<const void*>(grouped_one_kernel<false>), smem);
+  const cudaError_t e = set_smem(reinterpret_cast<const void*>(grouped_one_kernel), kRing32);
   if (e != cudaSuccess) return e;
   const int64_t tiles = tm * tn;
   const unsigned grid = unsigned(tiles < 65535 ? tiles : 65535);
-  if (f64)
-    grouped_one_kernel<true><<<grid, 32, smem, stream>>>(pr, int(tm), tiles);
-  else
-    grouped_one_kernel<false><<<grid, 32, smem, stream>>>(pr, int(tm), tiles);
+  grouped_one_kernel<<<grid, 32, kRing32, stream>>>(pr, int(tm), tiles);
   return cudaGetLastError();
 }
 

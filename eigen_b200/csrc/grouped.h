@@ -20,29 +20,37 @@ struct GroupedProblem {
 
 constexpr uint32_t kNoProblem = 0xFFFFFFFFu;
 
-// One warp's work: class 32 = the 32 x 32 output tile (tile_m, tile_n) of problem[0];
-// class 16 = problems problem[0..1], each at most 16 x 16; class 8 = problem[0..3], each at
+// One work item (a warp's, or of a block of two warps for FP64): class 32 = the 32 x 32 output
+// tile (tile_m, tile_n) of problem[0]; class 16 = problems problem[0..1], each at most 16 x 16; class 8 = problem[0..3], each at
 // most 8 x 8 (empty slots hold kNoProblem).  k = the largest k of the item's problems.
 struct GroupedItem {
   uint32_t problem[4];
   int32_t k;
   uint16_t tile_m, tile_n;
   uint8_t cls;
-  uint8_t pad_[7];
+  uint8_t frags;  // class 32: grouped_frags of the tile
+  uint8_t pad_[6];
 };
 static_assert(sizeof(GroupedItem) == 32, "one 32-byte load per item");
 
+// The 16-row and 8-column fragments a 32 x 32 tile of an m x n product has, as 4 (row blocks - 1)
+// + (column blocks - 1).
+__host__ __device__ inline uint8_t grouped_frags(int64_t m, int64_t n, int tile_m, int tile_n) {
+  const int64_t rows = m - int64_t(tile_m) * 32, cols = n - int64_t(tile_n) * 32;
+  return uint8_t((rows > 16 ? 4 : 0) + (cols > 24 ? 3 : int(cols - 1) / 8));
+}
+
 // Grid of the persistent grouped kernel for `num_items` items (as many two-warp blocks as fit
-// on the SMs, at most one warp per item); sets the kernel's shared-memory attribute.  Call it
+// on the SMs, at most one worker per item); sets the kernel's shared-memory attribute.  Call it
 // outside any stream capture.
 cudaError_t grouped_grid(bool f64, int64_t num_items, int num_sms, unsigned* blocks);
 // Launches the persistent grouped kernel for `num_items` items on `stream` with `blocks`
 // blocks from grouped_grid (capturable).
 cudaError_t launch_grouped_gemm(bool f64, const GroupedProblem* problems, const GroupedItem* items,
                                 int64_t num_items, unsigned blocks, cudaStream_t stream);
-// The same arithmetic for one product (one warp per 32 x 32 tile): the per-product launches
-// that a grouped launch replaces.
-cudaError_t launch_grouped_one(bool f64, const GroupedProblem& pr, cudaStream_t stream);
+// The same arithmetic for one FP32 product (one warp per 32 x 32 tile): the per-product launches
+// that a grouped launch replaces (FP64: the native kernel's, the same bits).
+cudaError_t launch_grouped_one(const GroupedProblem& pr, cudaStream_t stream);
 // Dynamic shared memory of one block of the grouped kernel.
 size_t grouped_block_smem(bool f64);
 

@@ -146,6 +146,7 @@ int build(char dtype, int64_t count, const eb2_gemm_problem* ps, std::vector<Gro
           it.tile_m = uint16_t(b);
           it.tile_n = uint16_t(a);
           it.cls = 32;
+          it.frags = grouped_frags(q.m, q.n, b, a);
           keyed.push_back({g.k, it});
         }
     }
@@ -299,7 +300,7 @@ int eb2_gemm_each(char dtype, int64_t count, const eb2_gemm_problem* problems, v
     } else {
       // FP32: the split-BF16 tile arithmetic of the grouped launch, one launch per product
       const eb2::GroupedProblem& g = ps[size_t(i)];
-      e = (g.k == 0 && g.beta == 1.0) ? cudaSuccess : eb2::launch_grouped_one(false, g, st);
+      e = (g.k == 0 && g.beta == 1.0) ? cudaSuccess : eb2::launch_grouped_one(g, st);
     }
     if (!eb2::cuda_ok(e, "per-product launch")) return EB2_ERR_CUDA;
   }
