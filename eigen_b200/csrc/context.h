@@ -62,7 +62,8 @@ struct Context {
   static constexpr int kPipeChunks = 16;
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
   cudaEvent_t ev_a = nullptr;
-  cudaEvent_t ev_scan = nullptr;  // the scans' statistics have reached the host (picker stage 2)
+  cudaEvent_t ev_scanned = nullptr;  // the scans are done (picker stage 2)
+  cudaEvent_t ev_scan = nullptr;  // their statistics have reached the host
   cudaEvent_t ev_in[kPipeChunks] = {};
   cudaEvent_t ev_done[kPipeChunks] = {};
   double* hchunk = nullptr;  // pinned [kPipeChunks][2]: per-block error-estimate energies

@@ -233,10 +233,16 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
     return good;
   };
   if (stage2) {
-    if (!check_cuda(cudaMemcpyAsync(cx.hflags, df, sizeof(DeviceFlags), cudaMemcpyDeviceToHost, st), "read scan") ||
-        !check_cuda(cudaEventRecord(cx.ev_scan, st), "scan event") || !split() ||
-        !check_cuda(cudaEventSynchronize(cx.ev_scan), "scan"))
-      return EB2_ERR_CUDA;
+    // The statistics reach the host on the copy stream: a copy on the product's stream, between the
+    // scan and the split, holds the split up by its own start and end
+    // (4096 x 1024 x 3000: 358.7 -> 352.0 us; 2048^3: 284.1 -> 281.0 us).
+    bool read = check_cuda(cudaEventRecord(cx.ev_scanned, st), "scan event") && split();
+    read = read && check_cuda(cudaStreamWaitEvent(cx.copy_out, cx.ev_scanned, 0), "scan event") &&
+           check_cuda(cudaMemcpyAsync(cx.hflags, df, sizeof(DeviceFlags), cudaMemcpyDeviceToHost, cx.copy_out),
+                      "read scan") &&
+           check_cuda(cudaEventRecord(cx.ev_scan, cx.copy_out), "scan event") &&
+           check_cuda(cudaEventSynchronize(cx.ev_scan), "scan");
+    if (!read) return EB2_ERR_CUDA;
     const double spread = cx.hflags->spread[1] > 0 ? cx.hflags->spread[0] / cx.hflags->spread[1] : 0.0;
     int cfg = -1, cls = 0;
     if (picker_predict(m, n, k, 'd', spread, 1, opt.tol > 0 ? opt.tol : settings().dgemm_tol.load(), &cfg, &cls)) {
