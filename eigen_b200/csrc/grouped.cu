@@ -9,17 +9,19 @@
 //     four whole products of at most 8 x 8 (Eigen's fixed-size range), so that small
 //     products share a warp instead of each filling a 32 x 32 tile;
 //   * an FP32 item is computed by ONE warp, an FP64 item by a block of TWO (half of the fragments and
-//     one operand's copies each: half the FP64 sums per lane leaves registers for 20 warps per SM
+//     one operand's copies each: half the FP64 sums per lane leaves registers for 24 warps per SM
 //     instead of 16).  Its operands arrive in K-chunks ("stages") of two
 //     32-line panels (rows of op(A), columns of op(B)) copied by cp.async into a
 //     shared-memory ring.  The copies of the next stages -- of the next item too -- are in
 //     flight while the current stage computes, which hides the latency of these short,
 //     scattered products' loads;
-//   * bound by the latency of short items (DMMA pipe 36 %, issue slots 48 % busy for FP64; issue slots
-//     51 % for FP32), so a stage carries no work for padding: lines outside the product are not copied
-//     (their outputs are not stored), only the K tail is zero-filled, and the fragments computed are
-//     those the item really has.  10,000 products of sides 3 .. 256: FP64 313.9 -> 305.1 us, FP32
-//     286.6 -> 267.8 us against one warp per item with padded fragments for both;
+//   * bound by the L1 data pipe (66 % busy for FP64: element-wise copies in, fragments out) and issue
+//     slots (57 %; DMMA pipe 46 %), so a stage carries no work for padding: lines outside the product are
+//     not copied (their outputs are not stored), only the K tail is zero-filled, and the fragments
+//     computed are those the item has (FP32: column fragments in pairs, four variants of the stage
+//     instead of eight, which the instruction cache holds: 262 -> 249 us).  10,000 products of sides
+//     3 .. 256: FP64 313.9 -> 240.7 us, FP32 286.6 -> 230.2 us against one warp per item with padded
+//     fragments and longer rings for both;
 //   * FP64: mma.sync m16n8k4 (DMMA), K in steps of 4 from 0 upward for every output, the
 //     same sequence as the native DGEMM kernel, so each product equals one plain native call
 //     bit for bit (m16n8k8 takes the same two steps in one instruction);
@@ -46,11 +48,18 @@ constexpr int kLineStride = 36;  // a panel's k-row: 32 lines (rows of op(A) / c
 constexpr int kKc = 8;           // K per stage: two m16n8k4 steps (FP64) or one m16n8k8 step (FP32)
 constexpr int kWarpsPerBlock = 2;
 
-// FP64: a block of two warps shares an item and its ring; FP32: an item per warp.
-constexpr int kStages64 = 4;  // 18.4 KB per block
-constexpr int kStages32 = 6;  // 13.8 KB per warp
-constexpr int kBlocks64 = 10, kBlocks32 = 8;  // per SM
+// FP64: a block of two warps shares an item and its ring; FP32: an item per warp.  Short rings leave
+// more of the SM's memory to L1, where the copies find the sectors that neighbouring stages share
+// (us for 10,000 products of sides 3 .. 256, stages x blocks: FP64 5 x 9 332, 4 x 10 252, 3 x 12 253,
+// 3 x 14 270, 2 x 12 243, 2 x 16 312; FP32 6 x 8 249, 5 x 8 233, 4 x 8 231, 3 x 8 230).
+constexpr int kStages64 = 2;  // 9.2 KB per block
+constexpr int kStages32 = 3;  // 6.9 KB per warp
+constexpr int kBlocks64 = 12, kBlocks32 = 8;  // per SM
 constexpr int kPanelElems = kKc * kLineStride;
+// K rows 4 .. 7 of an FP64 panel start two elements later: the 8-byte copies of a half-warp, 8 K
+// offsets of two lines, then hit distinct banks, and so do its fragment reads (307.5 -> 299.3 us).
+template <typename T>
+constexpr int kRowGap = sizeof(T) == 8 ? 2 : 0;
 constexpr int kStageElems = 2 * kPanelElems;
 
 __device__ __forceinline__ void dmma_16x8x8_g(double (&d)[4], double a0, double a1, double a2, double a3, double b0,
@@ -159,29 +168,34 @@ struct PanelCopy {
       const int line0 = first_line + ls / kKc, dline = r / kKc, kk0 = ls % kKc;
       ptr = reinterpret_cast<const char*>(base + kk0 + int64_t(line0) * ldx);
       step = int64_t(dline) * ldx * kSize;
-      dst0 = uint32_t((kk0 * kLineStride + slot_off + ls / kKc) * kSize);
+      dst0 = uint32_t((kk0 * kLineStride + (kk0 >> 2) * kRowGap<T> + slot_off + ls / kKc) * kSize);
       const int64_t rest = extent - line0;
       valid = rest <= 0 ? 0 : (rest > (kKc - 1) * dline ? kKc : (int(rest) + dline - 1) / dline);
     }
   }
 
-  // A stage of a class-32 item, the slots DSTEP bytes apart: one address and one predicated copy per
-  // element.  CONTIG: the first `left` elements lie inside K (all lanes alike); else a lane's K offset
-  // is inside or not.  What lies past K is zeroed.
-  template <bool CONTIG, int DSTEP, int... t>
+  // byte offset of element t from element 0 in the panel of a class-32 item
+  template <bool CONTIG>
+  static constexpr int place(int t) {
+    return (CONTIG ? t * kLineStride + (t >> 2) * kRowGap<T> : t * (32 / kKc)) * kSize;
+  }
+  // A stage of a class-32 item: one address and one predicated copy per element.  CONTIG: the first
+  // `left` elements lie inside K (all lanes alike); else a lane's K offset is inside or not.  What
+  // lies past K is zeroed.
+  template <bool CONTIG, int... t>
   __device__ __forceinline__ void issue_wide(uint32_t d, int left, std::integer_sequence<int, t...>) const {
     const uint32_t st = uint32_t(step);
     if (left >= kKc) {
-      (cp_async_elem_if<kSize, t * DSTEP>(d, ptr + uint64_t(st) * uint32_t(t), t, valid), ...);
+      (cp_async_elem_if<kSize, place<CONTIG>(t)>(d, ptr + uint64_t(st) * uint32_t(t), t, valid), ...);
     } else if constexpr (CONTIG) {
-      ((t < left ? cp_async_elem_if<kSize, t * DSTEP>(d, ptr + uint64_t(st) * uint32_t(t), t, valid)
-                 : zero_elem_if<kSize, t * DSTEP>(d, t, valid)),
+      ((t < left ? cp_async_elem_if<kSize, place<CONTIG>(t)>(d, ptr + uint64_t(st) * uint32_t(t), t, valid)
+                 : zero_elem_if<kSize, place<CONTIG>(t)>(d, t, valid)),
        ...);
     } else {
       const bool in = int(threadIdx.x) % kKc < left;
       const int copied = in ? valid : 0, zeroed = in ? 0 : valid;
-      (cp_async_elem_if<kSize, t * DSTEP>(d, ptr + uint64_t(st) * uint32_t(t), t, copied), ...);
-      (zero_elem_if<kSize, t * DSTEP>(d, t, zeroed), ...);
+      (cp_async_elem_if<kSize, place<CONTIG>(t)>(d, ptr + uint64_t(st) * uint32_t(t), t, copied), ...);
+      (zero_elem_if<kSize, place<CONTIG>(t)>(d, t, zeroed), ...);
     }
   }
 
@@ -192,9 +206,9 @@ struct PanelCopy {
     if (wide) {
       using Seq = std::make_integer_sequence<int, kKc>;
       if (contig)
-        issue_wide<true, kLineStride * kSize>(d, left, Seq{});
+        issue_wide<true>(d, left, Seq{});
       else
-        issue_wide<false, 32 / kKc * kSize>(d, left, Seq{});
+        issue_wide<false>(d, left, Seq{});
     } else {
       const char* p = ptr;
       uint32_t dt = d;
@@ -203,7 +217,8 @@ struct PanelCopy {
 #pragma unroll 2
       for (int t = 0; t < kKc; ++t, p += step, dt += dstep) {
         const bool in = kk0 + (contig ? t : 0) < left;
-        cp_async_fill_if<kSize>(dt, in ? static_cast<const void*>(p) : dummy, in ? kSize : 0, t, valid);
+        const uint32_t gap = contig && t >= 4 ? kRowGap<T> * kSize : 0;
+        cp_async_fill_if<kSize>(dt + gap, in ? static_cast<const void*>(p) : dummy, in ? kSize : 0, t, valid);
       }
     }
     ptr += contig ? kKc * step : int64_t(kKc * kSize);
@@ -216,9 +231,9 @@ struct ItemCopy {
   int left;      // K of the lane's product from the next stage on
   uint32_t how;  // the item's class, | 64: op(A)'s lines contiguous, | 128: op(B)'s, | 256: wide
 
+  // the lane's lines of op(A) (rhs = false) or op(B) into p
   template <class Src>
-  __device__ __forceinline__ void open(const Src& src, const GroupedItem& it, int lane, PanelCopy<T>* pa,
-                                       PanelCopy<T>* pb) {
+  __device__ __forceinline__ void open(const Src& src, const GroupedItem& it, int lane, bool rhs, PanelCopy<T>& p) {
     const int r = it.cls;
     const int log_r = r == 8 ? 3 : (r == 16 ? 4 : 5);
     const int q = lane >> log_r;
@@ -229,16 +244,18 @@ struct ItemCopy {
     left = ok ? int(pr.k < INT_MAX ? pr.k : INT_MAX) : 0;
     // op(A)(i, l): contiguous along i unless transposed; op(B)(l, j): along j only if transposed
     const bool ca = (pr.trans & 1) == 0, cb = (pr.trans & 2) != 0;
-    bool narrow = true;
-    if (pa) {
-      pa->set(static_cast<const T*>(pr.a), pr.lda, ca, r == 32 ? int(it.tile_m) * 32 : 0, q * r, ls, r, ok ? pr.m : 0);
-      narrow = narrow && pa->step <= INT_MAX;
-    }
-    if (pb) {
-      pb->set(static_cast<const T*>(pr.b), pr.ldb, cb, r == 32 ? int(it.tile_n) * 32 : 0, q * r, ls, r, ok ? pr.n : 0);
-      narrow = narrow && pb->step <= INT_MAX;
-    }
-    how = uint32_t(r) | (ca ? 64u : 0u) | (cb ? 128u : 0u) | (r == 32 && narrow ? 256u : 0u);
+    const int64_t extent = rhs ? pr.n : pr.m;
+    p.set(static_cast<const T*>(rhs ? pr.b : pr.a), rhs ? pr.ldb : pr.lda, rhs ? cb : ca,
+          r == 32 ? int(rhs ? it.tile_n : it.tile_m) * 32 : 0, q * r, ls, r, ok ? extent : 0);
+    how = uint32_t(r) | (ca ? 64u : 0u) | (cb ? 128u : 0u) | (r == 32 && p.step <= INT_MAX ? 256u : 0u);
+  }
+  template <class Src>
+  __device__ __forceinline__ void open(const Src& src, const GroupedItem& it, int lane, PanelCopy<T>& pa,
+                                       PanelCopy<T>& pb) {
+    open(src, it, lane, true, pb);
+    const uint32_t wide_b = how;
+    open(src, it, lane, false, pa);
+    how &= wide_b;
   }
   __device__ __forceinline__ void issue(PanelCopy<T>& p, const T* panel, bool rhs, const void* dummy) const {
     p.issue(smem_u32(panel), dummy, (how & (rhs ? 128u : 64u)) != 0u, left, int(how & 63u), (how & 256u) != 0u);
@@ -254,10 +271,11 @@ __device__ __forceinline__ int item_stages(const GroupedItem& it) {
 // the first fragment.  The m16n8k8 fragments are two m16n8k4 steps' taken in K order (same bits).
 template <int NJ>
 __device__ __forceinline__ void stage_f64(double (&acc)[4][4], const double* sA, const double* sB) {
-  const double a0 = sA[0], a1 = sA[8], a2 = sA[4 * kLineStride], a3 = sA[4 * kLineStride + 8];
+  constexpr int kUp = 4 * kLineStride + kRowGap<double>;  // K offset 4
+  const double a0 = sA[0], a1 = sA[8], a2 = sA[kUp], a3 = sA[kUp + 8];
 #pragma unroll
   for (int j = 0; j < NJ; ++j)
-    dmma_16x8x8_g(acc[j], a0, a1, a2, a3, sB[j * 8], sB[4 * kLineStride + j * 8]);
+    dmma_16x8x8_g(acc[j], a0, a1, a2, a3, sB[j * 8], sB[kUp + j * 8]);
 }
 
 // ---------------------------------------------------------------- FP32 compute
@@ -337,14 +355,10 @@ __device__ __forceinline__ void stage_small(float (&acc)[8][4], const float* st,
 __device__ __forceinline__ void compute_stage(float (&acc)[8][4], const float* st, const GroupedItem& it, int g,
                                               int tig) {
   if (it.cls != 32) return stage_small(acc, st, it.cls == 16, g, tig);
-  switch (it.frags) {
-    case 0: return stage32<1, 1>(acc, st, g, tig);
-    case 1: return stage32<1, 2>(acc, st, g, tig);
-    case 2: return stage32<1, 3>(acc, st, g, tig);
-    case 3: return stage32<1, 4>(acc, st, g, tig);
-    case 4: return stage32<2, 1>(acc, st, g, tig);
-    case 5: return stage32<2, 2>(acc, st, g, tig);
-    case 6: return stage32<2, 3>(acc, st, g, tig);
+  switch (it.frags >> 1) {
+    case 0: return stage32<1, 2>(acc, st, g, tig);
+    case 1: return stage32<1, 4>(acc, st, g, tig);
+    case 2: return stage32<2, 2>(acc, st, g, tig);
     default: return stage32<2, 4>(acc, st, g, tig);
   }
 }
@@ -450,7 +464,7 @@ __device__ __forceinline__ void run_items_f32(const Src& src, int64_t w0, int64_
   PanelCopy<float> pa, pb;
   auto open_item = [&]() {
     const GroupedItem it = src.item(p_idx);
-    cp.open(src, it, lane, &pa, &pb);
+    cp.open(src, it, lane, pa, pb);
     p_left = item_stages(it);
     // the next item's record comes to L1 with this read, its problem one stage later
     p_next = src.first_problem(p_idx + W);
@@ -515,7 +529,7 @@ __device__ __forceinline__ void run_items_f32(const Src& src, int64_t w0, int64_
 // The same order for a block of two warps: warp 0 copies the items' rows of op(A), warp 1 their
 // columns of op(B); each computes half of the fragments: a 16-row block of a 32 x 32 tile (or half
 // of its columns when it has one row block), one of two products, two of four.  Half the FP64 sums
-// per lane leaves registers for 20 warps per SM instead of 16, with half the copies each.
+// per lane leaves registers for 24 warps per SM instead of 16, with half the copies each.
 template <class Src>
 __device__ __forceinline__ void run_items_f64(const Src& src, int64_t w0, int64_t W, double* ring) {
   constexpr int S = kStages64;
@@ -529,7 +543,7 @@ __device__ __forceinline__ void run_items_f64(const Src& src, int64_t w0, int64_
   PanelCopy<double> pc;  // the warp's operand
   auto open_item = [&]() {
     const GroupedItem it = src.item(p_idx);
-    cp.open(src, it, lane, warp == 0 ? &pc : nullptr, warp == 0 ? nullptr : &pc);
+    cp.open(src, it, lane, warp != 0, pc);
     p_left = item_stages(it);
     p_next = src.first_problem(p_idx + W);
   };
@@ -591,7 +605,8 @@ __device__ __forceinline__ void run_items_f64(const Src& src, int64_t w0, int64_
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
         const double* x = st + (2 * warp + p) * 8;
-        dmma_16x8x8_g(acc[p], x[0], 0.0, x[4 * kLineStride], 0.0, x[kPanelElems], x[kPanelElems + 4 * kLineStride]);
+        constexpr int kUp = 4 * kLineStride + kRowGap<double>;
+        dmma_16x8x8_g(acc[p], x[0], 0.0, x[kUp], 0.0, x[kPanelElems], x[kPanelElems + kUp]);
       }
     } else {
       const double *sA = st + 16 * rb, *sB = st + kPanelElems + 8 * j0;
