@@ -25,6 +25,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <mutex>
 
 #include "device_common.cuh"
@@ -1122,23 +1123,29 @@ __device__ __forceinline__ double crt_round_magnitude(uint32_t r0, uint32_t r1, 
   return __longlong_as_double(static_cast<long long>(bits));
 }
 
+// bit length of P_N / 2
+template <int N>
+constexpr int crt_half_bits() {
+  int bits = 0;
+  for (int w = 0; w < 4; ++w)
+    for (int i = 0; i < 32; ++i)
+      if ((kCrtTableC.half[N][w] >> i) & 1u) bits = 32 * w + i + 1;
+  return bits;
+}
+
 // RN(R 2^escale) for R = (r3 r2 r1 r0) in 128-bit two's complement, congruent to C' modulo P
-// and within one P of [-P/2, P/2).  The range fix runs only when R's top 64-bit window does
-// not already place it in [-P/2, P/2).  Then, with hi = the signed 64-bit window of R at limbs
-// kW, kW+1 (|R| < 2^(63 + 32 kW)) and lo the limbs below it, R = hi 2^(32 kW) + lo, and two
-// one-rounding forms cover all but tiny |R|:
-//   * |hi| >= 2^54: RN(hi | [lo != 0]) 2^(32 kW).  The sticky bit sits below the guard bit
-//     (hi has at least 55 significant bits), and hi and hi | 1 lie strictly between the same
-//     two even integers, so both round like R;
-//   * 8 <= |hi| < 2^54: R = h 2^(32 kW + 1) + X with h = hi >> 1 (|h| < 2^53, exact in a
-//     double) and X = (hi & 1) 2^(32 kW) + lo.  For kW = 1, X < 2^33 is exact and
-//     RN(R) = fma(h, 2^33, X).  For kW = 2, X >> 12 with a sticky bit in its lowest place is
-//     below 2^53 and exact, and R, at least 2^67 in magnitude, has its guard bit at 2^13 or
-//     above, so RN(R) = fma(h, 2^53, (X >> 12) | [X mod 2^12 != 0]) 2^12;
-//   * kW = 0 (P < 2^64): R = hi exactly.
-// The result is scaled by adding to the exponent field when it stays normal.  Everything else
-// (|hi| < 8, subnormal or overflowing results) takes crt_round_magnitude, the per-row kernel's
-// steps, so every result is bit for bit that kernel's.
+// and within one P of [-P/2, P/2).  The range fix runs only when R's top words do not already place
+// it in [-P/2, P/2).  Then, with |R| < 2^L, R splits at fixed places into
+//     A = floor(R / 2^kA), |A| < 2^51,   B = the 52 bits below,   and the kB = kA - 52 bits below those,
+// and A and B are formed as doubles without a conversion: their bits under the exponent of 2^52, minus
+// an offset (exact).  Nonzero bits below B set B's last bit: (A 2^52 + B) is then R / 2^kB rounded to
+// odd, and one FMA rounds it to nearest as it would round R, provided two bits of it lie below the
+// last place of the result, |A 2^52 + B| >= 2^55 (for kB = 0 nothing lies below B and any size will
+// do).  The result is scaled by adding to the exponent field when it stays normal.  Everything
+// else (smaller |R|, zero, subnormal or overflowing results) takes crt_round_magnitude, the per-row
+// kernel's steps, so every result is bit for bit that kernel's.  One path for every size of R: with
+// entries spread over many binades a warp would otherwise walk both of two (a 64-bit conversion for
+// large |R|, an FMA of two parts for the others).
 template <int N>
 __device__ __forceinline__ double crt_round(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3, int escale) {
   constexpr uint32_t P0 = kCrtTableC.P[N][0], P1 = kCrtTableC.P[N][1], P2 = kCrtTableC.P[N][2], P3 = kCrtTableC.P[N][3];
@@ -1147,12 +1154,20 @@ __device__ __forceinline__ double crt_round(uint32_t r0, uint32_t r1, uint32_t r
   constexpr int kW = kCrtTableC.half[N][3] != 0 ? 2 : (kCrtTableC.half[N][2] != 0 ? 1 : 0);
   constexpr long long Hw = static_cast<long long>((static_cast<unsigned long long>(kCrtTableC.half[N][kW + 1]) << 32) |
                                                   kCrtTableC.half[N][kW]);
-  const uint32_t rl[4] = {r0, r1, r2, r3};
-  const long long win = static_cast<long long>((static_cast<unsigned long long>(rl[kW + 1]) << 32) | rl[kW]);
-  const uint32_t ext = win < 0 ? 0xFFFFFFFFu : 0u;
-  bool in_range = win >= -Hw && win < Hw;
+  bool in_range;
+  if constexpr (kW == 2 && (Hw >> 32) >= 256) {
+    // the top word alone decides but for one value in Hw / 2^32 at either end, which the fix leaves
+    // as it is
+    constexpr uint32_t Ht = uint32_t(Hw >> 32);
+    in_range = r3 + Ht < 2u * Ht;
+  } else {
+    const uint32_t rl[4] = {r0, r1, r2, r3};
+    const long long win = static_cast<long long>((static_cast<unsigned long long>(rl[kW + 1]) << 32) | rl[kW]);
+    const uint32_t ext = win < 0 ? 0xFFFFFFFFu : 0u;
+    in_range = win >= -Hw && win < Hw;
 #pragma unroll
-  for (int t = kW + 2; t < 4; ++t) in_range = in_range && rl[t] == ext;
+    for (int t = kW + 2; t < 4; ++t) in_range = in_range && rl[t] == ext;
+  }
   if (!in_range) {
     using u128 = unsigned __int128;
     using s128 = __int128;
@@ -1169,46 +1184,21 @@ __device__ __forceinline__ double crt_round(uint32_t r0, uint32_t r1, uint32_t r
     r2 = uint32_t(ur >> 64);
     r3 = uint32_t(ur >> 96);
   }
-  const uint32_t rl2[4] = {r0, r1, r2, r3};
-  const long long hi = static_cast<long long>((static_cast<unsigned long long>(rl2[kW + 1]) << 32) | rl2[kW]);
-  double d;
-  int s;
-  bool fast;
-  if constexpr (kW == 0) {
-    d = __ll2double_rn(hi);
-    s = 0;
-    fast = hi != 0;
-  } else if constexpr (kW == 1) {
-    if (static_cast<unsigned long long>(hi + (1ll << 54)) >= (1ull << 55)) {
-      d = __ll2double_rn(hi | (r0 != 0u ? 1ll : 0ll));
-      s = 32;
-    } else {
-      const long long h = hi >> 1;
-      const unsigned long long X = (static_cast<unsigned long long>(hi & 1) << 32) | r0;
-      d = fma(__ll2double_rn(h), 0x1p33, __ull2double_rn(X));
-      s = 0;
-    }
-    fast = static_cast<unsigned long long>(hi + 8) >= 16ull;
-  } else {
-    if (static_cast<unsigned long long>(hi + (1ll << 54)) >= (1ull << 55)) {
-      d = __ll2double_rn(hi | ((r0 | r1) != 0u ? 1ll : 0ll));
-      s = 64;
-    } else {
-      const long long h = hi >> 1;
-      // x = (X >> 12) | sticky = (hi & 1) 2^52 + X', X' = (lo >> 12) | [lo mod 2^12 != 0] below
-      // 2^52: the bits of 2^52 + X' assembled directly, minus 2^52 unless hi is odd (exact)
-      const uint32_t xlo = (r1 << 20) | (r0 >> 12) | ((r0 & 0xFFFu) != 0u ? 1u : 0u);
-      const double x = __hiloint2double(static_cast<int>(0x43300000u | (r1 >> 12)), static_cast<int>(xlo)) -
-                       ((hi & 1) != 0 ? 0.0 : 0x1p52);
-      d = fma(__ll2double_rn(h), 0x1p53, x);
-      s = 12;
-    }
-    fast = static_cast<unsigned long long>(hi + 8) >= 16ull;
-  }
-  const int k = s + escale;
+  constexpr int kL = crt_half_bits<N>() + 1;  // |R| <= P/2 < 2^(kL - 1); one more for R = -P/2
+  constexpr int kA = kL > 103 ? kL - 51 : 52, kB = kA - 52;
+  static_assert(kL <= 128 && kB < 32, "B starts in the lowest word");
+  const uint32_t rl[5] = {r0, r1, r2, r3, uint32_t(int(r3) >> 31)};
+  auto word = [&](int p) { return __funnelshift_r(rl[p / 32], rl[p / 32 + 1], uint32_t(p % 32)); };  // bits p .. p+31
+  const double a = __hiloint2double(int(word(kA + 32) + 0x43380000u), int(word(kA))) - 0x1.8p52;
+  uint32_t b_lo = word(kB);
+  if constexpr (kB > 0) b_lo |= (r0 << (32 - kB)) != 0u ? 1u : 0u;
+  const double b = __hiloint2double(int((word(kB + 32) & 0xFFFFFu) | 0x43300000u), int(b_lo)) - 0x1p52;
+  const double d = fma(a, 0x1p52, b);
+  const int k = kB + escale;
   const int hw = __double2hiint(d);
-  const int be = ((hw >> 20) & 0x7FF) + k;  // biased exponent of d 2^k
-  if (fast && static_cast<unsigned>(be - 1) < 2046u)
+  const int de = (hw >> 20) & 0x7FF;  // biased exponent of d
+  constexpr int kLeast = kB > 0 ? 1023 + 56 : 1;
+  if (de >= kLeast && static_cast<unsigned>(de + k - 1) < 2046u)
     return __hiloint2double(static_cast<int>(static_cast<unsigned>(hw) + (static_cast<unsigned>(k) << 20)),
                             __double2loint(d));
   return crt_round_magnitude(r0, r1, r2, r3, escale);
@@ -1274,6 +1264,10 @@ __device__ __forceinline__ void mma_u8_16x8x16(int (&d)[4], uint32_t a0, uint32_
 // S in four 32-bit-aligned columns, X_0 + 2^16 X_1, X_2 + 2^16 X_3, Y_0 + 2^16 Y_1, Y_2 + 2^16 Y_3;
 // the tail (crt_finish_small) and the store follow.  Bit for bit the per-row kernel: S is the same
 // integer and it is rounded the same way.
+// Bound by issue slots and, with few groups per warp, by the wait for the first one (2048^3: 191
+// warp instructions per 32 entries, 55 % of the slots).  Groups of which every entry is kept take a
+// path without per-entry conditions, its four steps unrolled: with the one rounding path above, 243
+// instructions before, 52.4 -> 46.9 us; the call 275.9 -> 269.7 us, 8192^3 7.73 -> 7.62 ms.
 constexpr int kRecStages = 2;  // groups of residues in each warp's ring
 template <int N, bool EST>
 __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __grid_constant__ CrtRecParams R) {
@@ -1282,7 +1276,6 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
   __shared__ __align__(16) uint32_t ring[8][kRecStages][16 * 32];
   if (R.skip_if_flag && *R.skip_if_flag) return;
   uint32_t (*const wstage)[32 * 8] = stage[threadIdx.x >> 5];
-  int sbuf = 0;
   const uint32_t (*const wring)[16 * 32] = ring[threadIdx.x >> 5];
   CrtStoreCtx sc = store_ctx(R);
   const uint8_t* const res = R.res;
@@ -1351,6 +1344,7 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
     const int groups = int(((j1 + 3) >> 2) - g0);
     copy_group(0, g0);
     cp_async_commit();
+    const int32_t* const mu_rows = sc.mu_a + i0 + e_row;  // this lane's rows: every 8th
     for (int t = 0; t < groups; ++t) {
       if (t + 1 < groups) copy_group((t + 1) & 1, g0 + t + 1);
       cp_async_commit();
@@ -1360,66 +1354,77 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
       const int64_t j = 4 * (g0 + t) + e_col;
       const bool col_ok = j >= jb && j < j1;
       const int nu_j = col_ok ? sc.mu_b[j] : 0;
-      double* cp = sc.C + j * sc.ldc + i0 + e_row;
-#pragma unroll 1
-      for (int s = 0; s < 4; ++s, cp += 8) {
-        __syncwarp();  // lanes that kept nothing wait here for the MMAs
-        // this lane's entry: its row's exponent and old C are on their way during the byte sums
-        const int64_t ie = i0 + 8 * s + e_row;
-        const bool keep = col_ok && ie < m && (uplo == 0 || (uplo == 1 ? ie <= j : ie >= j));
-        const int mu_e = keep ? sc.mu_a[ie] : 0;
-        const double old = (keep && sc.write_c && sc.beta != 0.0) ? *cp : 0.0;
-        uint32_t w[4];
+      double* const cp = sc.C + j * sc.ldc + i0 + e_row;
+      // four entries per lane, one of every 8 rows; ALL: every one of the warp's is kept
+      auto entries = [&](auto all) {
+        constexpr bool kAll = decltype(all)::value;
+#pragma unroll(kAll ? 4 : 1)
+        for (int s = 0; s < 4; ++s) {
+          __syncwarp();  // lanes that kept nothing wait here for the MMAs
+          const int64_t ie = i0 + 8 * s + e_row;
+          const bool keep = kAll || (col_ok && ie < m && (uplo == 0 || (uplo == 1 ? ie <= j : ie >= j)));
+          // its row's exponent and old C are on their way during the byte sums
+          const int mu_e = keep ? mu_rows[8 * s] : 0;
+          const double old = (keep && sc.write_c && sc.beta != 0.0) ? cp[8 * s] : 0.0;
+          uint32_t w[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) w[k] = 4 * c + k < N ? slot[(4 * c + k) * 32 + ((8 * s + g) ^ (8 * c))] : 0u;
-        // 4 x 4 byte transpose: w[k] byte e (modulus 4c+k, column e) -> v[e] byte k
-        const uint32_t t0 = __byte_perm(w[0], w[1], 0x5140), t1 = __byte_perm(w[0], w[1], 0x7362);
-        const uint32_t t2 = __byte_perm(w[2], w[3], 0x5140), t3 = __byte_perm(w[2], w[3], 0x7362);
-        const uint32_t v0 = __byte_perm(t0, t2, 0x5410), v1 = __byte_perm(t0, t2, 0x7632);
-        const uint32_t v2 = __byte_perm(t1, t3, 0x5410), v3 = __byte_perm(t1, t3, 0x7632);
-        // columns 0 / 1 (MMA row slots g / g+8), then columns 2 / 3; bytes 0..7, then 8..15
-        int d0[4], d1[4], d2[4], d3[4];  // the byte sums start from zero (C operand 0)
-        mma_u8_16x8x16(d0, v0, v1, bfrag[0]);
-        mma_u8_16x8x16(d1, v0, v1, bfrag[1]);
-        mma_u8_16x8x16(d2, v2, v3, bfrag[0]);
-        mma_u8_16x8x16(d3, v2, v3, bfrag[1]);
-        // (X_c, Y_c) of column e of this row to stage row 8e + g
-        uint32_t* const st = wstage[sbuf];
-        auto put = [&](int e, int xlo, int xhi, int ylo, int yhi) {
-          const int r = 8 * e + g;
-          *reinterpret_cast<uint2*>(st + r * 8 + 2 * (c ^ ((r >> 2) & 3))) =
-              make_uint2(uint32_t(xlo) + uint32_t(xhi) * 256u, uint32_t(ylo) + uint32_t(yhi) * 256u);
-        };
-        put(0, d0[0], d0[1], d1[0], d1[1]);
-        put(1, d0[2], d0[3], d1[2], d1[3]);
-        put(2, d2[0], d2[1], d3[0], d3[1]);
-        put(3, d2[2], d2[3], d3[2], d3[3]);
-        __syncwarp();
-        // this lane's entry: S = sum_b T_b 2^(8b) as four 32-bit-aligned columns (each < 2^46)
-        const uint32_t* const rrow = st + lane * 8;
-        sbuf ^= 1;
-        const int sw = 2 * ((lane >> 2) & 3);
-        const uint2 q0 = *reinterpret_cast<const uint2*>(rrow + (0 ^ sw)), q1 = *reinterpret_cast<const uint2*>(rrow + (2 ^ sw));
-        const uint2 q2 = *reinterpret_cast<const uint2*>(rrow + (4 ^ sw)), q3 = *reinterpret_cast<const uint2*>(rrow + (6 ^ sw));
-        const unsigned long long acc[4] = {static_cast<unsigned long long>(q1.x) * 65536ull + q0.x,
-                                           static_cast<unsigned long long>(q3.x) * 65536ull + q2.x,
-                                           static_cast<unsigned long long>(q1.y) * 65536ull + q0.y,
-                                           static_cast<unsigned long long>(q3.y) * 65536ull + q2.y};
-        if (!keep) continue;
-        const double v = __dmul_rn(sc.alpha, crt_finish_small<N>(acc, P_inv32, -mu_e - nu_j));
-        if (EST) {
-          if (uplo != 0 && mu_e != kCrtZeroRow && nu_j != kCrtZeroRow) e_acc += exp2_int(2 * (sc.b - mu_e - nu_j));
-          v_acc += v * v;
-        }
-        if (sc.write_c) {
-          if (sc.beta == 0.0) {
-            *cp = v;
-          } else {
-            if (sc.save) sc.save[j * sc.ld_save + ie] = old;
-            *cp = __fma_rn(sc.beta, old, v);
+          for (int k = 0; k < 4; ++k) w[k] = 4 * c + k < N ? slot[(4 * c + k) * 32 + ((8 * s + g) ^ (8 * c))] : 0u;
+          // 4 x 4 byte transpose: w[k] byte e (modulus 4c+k, column e) -> v[e] byte k
+          const uint32_t t0 = __byte_perm(w[0], w[1], 0x5140), t1 = __byte_perm(w[0], w[1], 0x7362);
+          const uint32_t t2 = __byte_perm(w[2], w[3], 0x5140), t3 = __byte_perm(w[2], w[3], 0x7362);
+          const uint32_t v0 = __byte_perm(t0, t2, 0x5410), v1 = __byte_perm(t0, t2, 0x7632);
+          const uint32_t v2 = __byte_perm(t1, t3, 0x5410), v3 = __byte_perm(t1, t3, 0x7632);
+          // columns 0 / 1 (MMA row slots g / g+8), then columns 2 / 3; bytes 0..7, then 8..15
+          int d0[4], d1[4], d2[4], d3[4];  // the byte sums start from zero (C operand 0)
+          mma_u8_16x8x16(d0, v0, v1, bfrag[0]);
+          mma_u8_16x8x16(d1, v0, v1, bfrag[1]);
+          mma_u8_16x8x16(d2, v2, v3, bfrag[0]);
+          mma_u8_16x8x16(d3, v2, v3, bfrag[1]);
+          // (X_c, Y_c) of column e of this row to stage row 8e + g
+          uint32_t* const st = wstage[s & 1];
+          auto put = [&](int e, int xlo, int xhi, int ylo, int yhi) {
+            const int r = 8 * e + g;
+            *reinterpret_cast<uint2*>(st + r * 8 + 2 * (c ^ ((r >> 2) & 3))) =
+                make_uint2(uint32_t(xlo) + uint32_t(xhi) * 256u, uint32_t(ylo) + uint32_t(yhi) * 256u);
+          };
+          put(0, d0[0], d0[1], d1[0], d1[1]);
+          put(1, d0[2], d0[3], d1[2], d1[3]);
+          put(2, d2[0], d2[1], d3[0], d3[1]);
+          put(3, d2[2], d2[3], d3[2], d3[3]);
+          __syncwarp();
+          // this lane's entry: S = sum_b T_b 2^(8b) as four 32-bit-aligned columns (each < 2^46)
+          const uint32_t* const rrow = st + lane * 8;
+          const int sw = 2 * ((lane >> 2) & 3);
+          const uint2 q0 = *reinterpret_cast<const uint2*>(rrow + (0 ^ sw));
+          const uint2 q1 = *reinterpret_cast<const uint2*>(rrow + (2 ^ sw));
+          const uint2 q2 = *reinterpret_cast<const uint2*>(rrow + (4 ^ sw));
+          const uint2 q3 = *reinterpret_cast<const uint2*>(rrow + (6 ^ sw));
+          const unsigned long long acc[4] = {static_cast<unsigned long long>(q1.x) * 65536ull + q0.x,
+                                             static_cast<unsigned long long>(q3.x) * 65536ull + q2.x,
+                                             static_cast<unsigned long long>(q1.y) * 65536ull + q0.y,
+                                             static_cast<unsigned long long>(q3.y) * 65536ull + q2.y};
+          if (!keep) continue;
+          const double v = __dmul_rn(sc.alpha, crt_finish_small<N>(acc, P_inv32, -mu_e - nu_j));
+          if (EST) {
+            if (!kAll && uplo != 0 && mu_e != kCrtZeroRow && nu_j != kCrtZeroRow)
+              e_acc += exp2_int(2 * (sc.b - mu_e - nu_j));
+            v_acc += v * v;
+          }
+          if (sc.write_c) {
+            if (sc.beta == 0.0) {
+              cp[8 * s] = v;
+            } else {
+              if (sc.save) sc.save[j * sc.ld_save + ie] = old;
+              cp[8 * s] = __fma_rn(sc.beta, old, v);
+            }
           }
         }
-      }
+      };
+      const int64_t jg = 4 * (g0 + t);
+      if (uplo == 0 && i0 + 32 <= m && jg >= jb && jg + 4 <= j1)
+        entries(std::true_type{});
+      else
+        entries(std::false_type{});
     }
     __syncwarp();  // the slots are read before the next pass copies into them
   }
