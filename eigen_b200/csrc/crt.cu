@@ -762,7 +762,7 @@ struct CrtRecParams {
   int write_c;
   double* save;
   int64_t ld_save;
-  int cols_per_block;  // columns one block handles per pass (fewer when the grid would be small)
+  int64_t cols_per_block;  // columns of a block (a multiple of 4; the per-row kernels: per pass)
   int uplo;            // 0: all of C; 1: i <= j only; 2: i >= j only
 };
 
@@ -878,8 +878,7 @@ __device__ __forceinline__ void crt_reduce_energies(const CrtRecParams& R, doubl
   }
 }
 
-constexpr int kRecCols = 32;  // most columns per block and pass
-static_assert(kRecCols <= 32 && kRecCols % 4 == 0, "the estimate's column sum takes a lane per column");
+constexpr int kRecCols = 32;  // columns of a block that finishes a part of a triangle
 
 // Byte of row i, column j in a residue plane ([cols/4][ld_res][4]: the GEMM's epilogue writes four
 // neighbouring columns of a row as one word).
@@ -894,7 +893,7 @@ __global__ void __launch_bounds__(256) crt_reconstruct_kernel(const __grid_const
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   double e_acc = 0.0, v_acc = 0.0;
   // blockIdx.y walks groups of cols_per_block columns
-  const int cpb = R.cols_per_block;
+  const int64_t cpb = R.cols_per_block;
   const int64_t jstep = int64_t(gridDim.y) * cpb;
   for (int64_t j0 = int64_t(blockIdx.y) * cpb; i < R.m && j0 < R.ncols; j0 += jstep) {
     int64_t jb, je;
@@ -1038,7 +1037,7 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct128_kernel(const __grid
   const double P_inv = R.P_inv;
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   double e_acc = 0.0, v_acc = 0.0;
-  const int cpb = R.cols_per_block;
+  const int64_t cpb = R.cols_per_block;
   const int64_t jstep = int64_t(gridDim.y) * cpb;
   for (int64_t j0 = int64_t(blockIdx.y) * cpb; i < m && j0 < ncols; j0 += jstep) {
     int64_t jb, j1;
@@ -1267,7 +1266,8 @@ __device__ __forceinline__ void mma_u8_16x8x16(int (&d)[4], uint32_t a0, uint32_
 // Bound by issue slots and, with few groups per warp, by the wait for the first one (2048^3: 191
 // warp instructions per 32 entries, 55 % of the slots).  Groups of which every entry is kept take a
 // path without per-entry conditions, its four steps unrolled: with the one rounding path above, 243
-// instructions before, 52.4 -> 46.9 us; the call 275.9 -> 269.7 us, 8192^3 7.73 -> 7.62 ms.
+// instructions before, 52.4 -> 46.9 us; the call 275.9 -> 269.7 us, 8192^3 7.73 -> 7.62 ms.  A block
+// takes one run of columns, so that set-up and first copies are paid once.
 constexpr int kRecStages = 2;  // groups of residues in each warp's ring
 template <int N, bool EST>
 __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __grid_constant__ CrtRecParams R) {
@@ -1315,28 +1315,13 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
   // this lane's words of a stage buffer (pair p of row r at r * 8 + 2 (p ^ (r / 4) % 4): the writes
   // and the reads of a half-warp hit distinct banks)
   const int e_row = lane & 7, e_col = lane >> 3;  // the entry this lane finishes
-  const int cpb = R.cols_per_block;
-  const int64_t jstep = int64_t(gridDim.y) * cpb;
-  for (int64_t j0 = int64_t(blockIdx.y) * cpb; i0 < m && j0 < ncols; j0 += jstep) {
-    // the columns that some row of the warp keeps
-    int64_t jb = j0, j1 = j0 + cpb < ncols ? j0 + cpb : ncols;
-    if (uplo == 1 && jb < i0) jb = i0;            // i <= j
-    if (uplo == 2 && j1 > i0 + 32) j1 = i0 + 32;  // i >= j
-    if (jb >= j1) continue;
-    if (EST && uplo == 0) {
-      // sum_j 2^(2(b - mu_i - nu_j)) over the pass's nonzero columns = 2^(2(b - mu_i - nu_min))
-      // sum_j 2^(-2(nu_j - nu_min)): the column sum is the same for every row of the warp, so
-      // lane t takes column jb + t (at most kRecCols of them) and the warp adds them up
-      const int cnt = int(j1 - jb);
-      const int mu_i = i < m ? sc.mu_a[i] : kCrtZeroRow;
-      const int nu = lane < cnt ? sc.mu_b[jb + lane] : kCrtZeroRow;
-      const bool nz = nu != kCrtZeroRow;
-      const int nu_min = __reduce_min_sync(0xffffffffu, nz ? nu : INT_MAX);
-      double t = nz ? exp2_int(-2 * (nu - nu_min)) : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (mu_i != kCrtZeroRow && nu_min != INT_MAX) e_acc = fma(exp2_int(2 * (sc.b - mu_i - nu_min)), t, e_acc);
-    }
+  // the block's columns that some row of the warp keeps
+  int64_t jb = int64_t(blockIdx.y) * R.cols_per_block, j1 = jb + R.cols_per_block;
+  if (j1 > ncols) j1 = ncols;
+  if (uplo == 1 && jb < i0) jb = i0;            // i <= j
+  if (uplo == 2 && j1 > i0 + 32) j1 = i0 + 32;  // i >= j
+  if (i0 < m && jb < j1) {
+    const int mu_i = EST && i < m ? sc.mu_a[i] : kCrtZeroRow;
     // one commit group per group of columns (empty past the last), so that waiting for all but the
     // newest leaves the current one landed; every lane reads a slot's last words before the
     // __syncwarp that precedes any copy into it
@@ -1350,6 +1335,19 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
       cp_async_commit();
       cp_async_wait<kRecStages - 1>();
       __syncwarp();
+      if (EST && uplo == 0 && t % 8 == 0) {
+        // sum_j 2^(2(b - mu_i - nu_j)) over the next 32 columns' nonzero ones = 2^(2(b - mu_i -
+        // nu_min)) sum_j 2^(-2(nu_j - nu_min)): the column sum is the same for every row of the warp,
+        // so a lane takes a column and the warp adds them up
+        const int64_t jl = 4 * (g0 + t) + lane;
+        const int nu = jl < j1 ? sc.mu_b[jl] : kCrtZeroRow;
+        const bool nz = nu != kCrtZeroRow;
+        const int nu_min = __reduce_min_sync(0xffffffffu, nz ? nu : INT_MAX);
+        double sum = nz ? exp2_int(-2 * (nu - nu_min)) : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (mu_i != kCrtZeroRow && nu_min != INT_MAX) e_acc = fma(exp2_int(2 * (sc.b - mu_i - nu_min)), sum, e_acc);
+      }
       const uint32_t* const slot = wring[t & 1];
       const int64_t j = 4 * (g0 + t) + e_col;
       const bool col_ok = j >= jb && j < j1;
@@ -1426,7 +1424,6 @@ __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __gri
       else
         entries(std::false_type{});
     }
-    __syncwarp();  // the slots are read before the next pass copies into them
   }
   if (EST) {
     __syncthreads();
@@ -1655,14 +1652,19 @@ cudaError_t launch_crt_reconstruct(const CrtReconstructArgs& args, cudaStream_t 
                    args.plane >= (args.n + 3) / 4 * 4 * args.ld_res;
   const int64_t rows_per_block = 256;
   const unsigned gx = unsigned((args.m + rows_per_block - 1) / rows_per_block);
-  // whole groups of four columns: up to kRecCols per block while that leaves about three rounds of
-  // four blocks per SM, so that a block's set-up and first copies are spread over many columns
+  // Whole groups of four columns.  All of C: one run of groups per block, as many blocks as are
+  // resident at four per SM, so that set-up and first copies are paid once and every block ends
+  // together (against runs of 4 .. 32 columns in three rounds of blocks: 2048^3 267.0 -> 262.9 us,
+  // 4096 x 1024 x 3000 337.8 -> 335.2 us, dtrsm 4096 x 2048 1384 -> 1361 us, 8192^3 the same).  A
+  // triangle: runs of kRecCols, since a block may have nothing to do.
   int64_t cpb = kRecCols;
-  while (cpb > 4 && int64_t(gx) * args.n < cpb * 3 * 4 * 148) cpb /= 2;
-  R.cols_per_block = int(cpb);
-  const int64_t groups = (args.n + cpb - 1) / cpb;
-  const unsigned gy = unsigned(groups < 65535 ? groups : 65535);
-  const dim3 grid(gx, gy);
+  if (args.uplo == 0) {
+    const int64_t runs = 4 * 148 / gx > 0 ? 4 * 148 / gx : 1, groups = (args.n + 3) / 4;
+    cpb = 4 * ((groups + runs - 1) / runs);
+  }
+  while ((args.n + cpb - 1) / cpb > 65535) cpb *= 2;  // gridDim.y
+  R.cols_per_block = cpb;
+  const dim3 grid(gx, unsigned((args.n + cpb - 1) / cpb));
   const bool est = args.err_sq != nullptr;
   switch (args.moduli) {
     case 8: launch_rec128<8>(est, mma, grid, stream, R); break;
