@@ -59,3 +59,29 @@ def test_block_edges(dtype, order, side, uplo, trans, diag):
 def test_vectors_per_block(dtype, count, side):
     m, n = (40, count) if side == "L" else (count, 40)
     _solve(dtype, side, "L", "N", "N", m, n)
+
+
+@pytest.mark.parametrize("dtype", ["d", "s"])
+@pytest.mark.parametrize("count", [37, 16 * 148 + 1, 32 * 148 + 1])
+def test_block_error(dtype, count):
+    """A vector entry is rounded at its own size once per 16-row sub-block above it (8 on average in 256
+    rows), by half of its own sub-block's 15 updates, its reciprocal and its product: about 17.5
+    independent roundings, each of variance at most u^2 / 3 of the entry.  (Rounded by every one of
+    the 128 rows above it on average, the error would be 2.4 times the bound.)"""
+    td = torch.float64 if dtype == "d" else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(count)
+    order = 256
+    a = (torch.rand((order, order), dtype=td, device="cuda", generator=g) * 2 - 1) / 16
+    a.diagonal().uniform_(1, 2, generator=g)
+    b = torch.rand((count, order), dtype=td, device="cuda", generator=g) * 2 - 1
+    x = b.clone()
+    torch.cuda.synchronize()
+    eb.level3("dtrsm" if dtype == "d" else "strsm", "L", "L", "N", "N", order, count, 1.0, a, order, x, order)
+    low = np.tril(a.cpu().numpy().T).astype(np.longdouble)
+    ref = b.cpu().numpy().T[:, :32].astype(np.longdouble)
+    for c in range(order):
+        ref[c] /= low[c, c]
+        ref[c + 1:] -= low[c + 1:, c:c + 1] * ref[c]
+    err = np.sqrt((((x.cpu().numpy().T[:, :32] - ref) ** 2).sum()) / (ref ** 2).sum())
+    u = 2.0 ** -53 if dtype == "d" else 2.0 ** -24
+    assert err <= u * np.sqrt(17.5 / 3)
