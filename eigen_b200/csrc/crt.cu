@@ -1263,11 +1263,11 @@ __device__ __forceinline__ void mma_u8_16x8x16(int (&d)[4], uint32_t a0, uint32_
 // S in four 32-bit-aligned columns, X_0 + 2^16 X_1, X_2 + 2^16 X_3, Y_0 + 2^16 Y_1, Y_2 + 2^16 Y_3;
 // the tail (crt_finish_small) and the store follow.  Bit for bit the per-row kernel: S is the same
 // integer and it is rounded the same way.
-// Bound by issue slots and, with few groups per warp, by the wait for the first one (2048^3: 191
-// warp instructions per 32 entries, 55 % of the slots).  Groups of which every entry is kept take a
-// path without per-entry conditions, its four steps unrolled: with the one rounding path above, 243
-// instructions before, 52.4 -> 46.9 us; the call 275.9 -> 269.7 us, 8192^3 7.73 -> 7.62 ms.  A block
-// takes one run of columns, so that set-up and first copies are paid once.
+// Bound by issue slots and the wait for the residues (2048^3: 160 warp instructions per 32 entries, 55 %
+// of the slots).  Groups of which every entry is kept take a path without per-entry conditions, its
+// four steps unrolled, and a block takes one run of columns, so that set-up and first copies are paid
+// once: with the one rounding path above, 243 instructions before, 52.4 -> 40.0 us; the call 275.9 ->
+// 265 us, 8192^3 7.73 -> 7.6 ms.
 constexpr int kRecStages = 2;  // groups of residues in each warp's ring
 template <int N, bool EST>
 __global__ void __launch_bounds__(256, 4) crt_reconstruct_mma_kernel(const __grid_constant__ CrtRecParams R) {
