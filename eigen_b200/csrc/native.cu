@@ -591,9 +591,13 @@ bool sgemm_small_applies(int64_t m, int64_t n, int64_t k) {
   // Rounds of tiles over the SMs times K, up to where split-BF16 takes over (device time, us, this
   // kernel / split-BF16 or the FFMA kernel before): 64^3 2.9 / 11.6, 128^3 3.9 / 26.2, 256^3 5.7 /
   // 24.8, 384^3 7.4 / 23.3, 512^3 16.0 / 23.7, 32 x 4096 x 1024 16.1 / 27.7; past the line
-  // 300 x 517 x 1100 33 / 26.9, 640^3 28.9 / 25.8.
-  const int64_t tiles = ((m + kFTile - 1) / kFTile) * ((n + kFTile - 1) / kFTile);
-  return (n + kFTile - 1) / kFTile <= 65535 && (tiles + 147) / 148 * k <= 1200;
+  // 300 x 517 x 1100 33 / 26.9, 640^3 28.9 / 25.8.  And not too many rounds, since a round costs a
+  // whole K tile and the sum of the shares (0.75 us each) however short K is, while the other
+  // kernels' time steps up past K = 64 (a call, us): 1216^2 x 32 (10 rounds) 18.5 / 18.9, 1344^2 x 32
+  // (12) 22.6 / 18.9, 3000^2 x 4 (60) 96 / 35, 6000^2 x 4 (239) 374 / 83; 1216^2 x 100 25.7 / 29.8,
+  // 1344^2 x 100 30.8 / 29.9, 1536^2 x 75 (16) 39 / 32.
+  const int64_t tiles = ((m + kFTile - 1) / kFTile) * ((n + kFTile - 1) / kFTile), rounds = (tiles + 147) / 148;
+  return (n + kFTile - 1) / kFTile <= 65535 && rounds * k <= 1200 && rounds <= (k <= kFKT ? 10 : 11);
 }
 
 cudaError_t launch_sgemm_small(bool transA, bool transB, int64_t m, int64_t n, int64_t k, float alpha, const float* A,

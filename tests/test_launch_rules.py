@@ -1,0 +1,27 @@
+"""The rules that choose a kernel's launch from the sizes (CPU): called in the built library by their
+C++ names, they launch nothing."""
+import ctypes
+
+import pytest
+
+import eigen_b200 as eb
+
+I64 = ctypes.c_int64
+
+
+def _rule(symbol, restype, *argtypes):
+    f = eb.load()[symbol]
+    f.restype, f.argtypes = restype, argtypes
+    return f
+
+
+@pytest.mark.parametrize("rounds,k,small", [(1, 1200, True), (1, 1201, False), (2, 600, True), (2, 601, False),
+                                            (10, 1, True), (11, 1, False), (10, 64, True), (11, 64, False),
+                                            (11, 65, True), (12, 65, False), (12, 100, False), (60, 4, False),
+                                            (1200, 1, False)])
+def test_small_sgemm_pays_whole_k_tiles(rounds, k, small):
+    # a round of 148 tiles costs a whole 64-deep K tile however short K is, so shallow products take
+    # the kernel for few rounds only
+    applies = _rule("_ZN3eb219sgemm_small_appliesElll", ctypes.c_bool, I64, I64, I64)
+    assert applies(148 * 32, 32 * rounds, k) == small
+    assert applies(32 * rounds, 148 * 32, k) == small
