@@ -33,6 +33,9 @@ struct StridedView {
 cudaError_t launch_dgemm_native(bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha,
                                 const double* A, int64_t lda, const double* B, int64_t ldb, double beta, double* C,
                                 int64_t ldc, const int* only_if_flag, cudaStream_t stream);
+// The side (32, 64 or 128) of the tiles that a native FP64 product takes; `wide`: both operands allow
+// 16-byte copies.
+int dmma_tile(int64_t m, int64_t n, int64_t k, bool wide);
 cudaError_t launch_sgemm_native(bool transA, bool transB, int64_t m, int64_t n, int64_t k, float alpha,
                                 const float* A, int64_t lda, const float* B, int64_t ldb, float beta, float* C,
                                 int64_t ldc, const int* only_if_flag, cudaStream_t stream);

@@ -502,6 +502,9 @@ __global__ void scale_matrix_kernel(int64_t m, int64_t n, T beta, T* C, int64_t 
 
 namespace {
 
+// 16-byte copies where the operand allows them
+bool dmma_wide(const double* X, int64_t ld) { return reinterpret_cast<uintptr_t>(X) % 16 == 0 && ld % 2 == 0; }
+
 template <class D>
 cudaError_t launch_dmma(bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
                         int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc,
@@ -516,9 +519,7 @@ cudaError_t launch_dmma(bool transA, bool transB, int64_t m, int64_t n, int64_t 
                                                          nullptr);
     return cudaGetLastError();
   };
-  // 16-byte copies where the operand allows them
-  const bool va = reinterpret_cast<uintptr_t>(A) % 16 == 0 && lda % 2 == 0;
-  const bool vb = reinterpret_cast<uintptr_t>(B) % 16 == 0 && ldb % 2 == 0;
+  const bool va = dmma_wide(A, lda), vb = dmma_wide(B, ldb);
   auto by_vec = [&](auto k11, auto k12, auto k21, auto k22) -> cudaError_t {
     if (va) return vb ? pick(k22) : pick(k21);
     return vb ? pick(k12) : pick(k11);
@@ -533,30 +534,41 @@ cudaError_t launch_dmma(bool transA, bool transB, int64_t m, int64_t n, int64_t 
 #undef EB2_DMMA_VARIANTS
 }
 
-// The tile side for an m x n output: the one whose busiest SM has the least work, tiles per SM
-// (rounded up) times the tile's area, weighted by how far each size falls short of the DMMA rate
-// when the chip is full (4096 x 4096 x 1024: 1033, 1056 and 1209 us for sides 128, 64 and 32).
-// Measured with 128 / 64 / 32 (us): 128^3 24.7 / 10.4 / 6.3; 512^3 78 / 24.7 / 16.5; 768^3 115 /
-// 35.0 / 41.7; 1000 x 1531 x 777 117 / 95 / 103; 1536 x 1536 x 256 43.1 / 44.1 / 53.3.
-int dmma_tile(int64_t m, int64_t n) {
+}  // namespace
+
+int dmma_tile(int64_t m, int64_t n, int64_t k, bool wide) {
+  // The side whose busiest SM has the least work, tiles per SM (rounded up) times the tile's area,
+  // weighted by how far each size falls short of the DMMA rate when the chip is full (4096 x 4096 x
+  // 1024: 1033, 1056 and 1209 us for sides 128, 64 and 32).  Measured with 128 / 64 / 32 (us): 128^3
+  // 24.7 / 10.4 / 6.3; 512^3 78 / 24.7 / 16.5; 768^3 115 / 35.0 / 41.7; 1000 x 1531 x 777 117 / 95 /
+  // 103; 1536 x 1536 x 256 43.1 / 44.1 / 53.3.
   constexpr int64_t kSms = 148;
+  auto tiles = [&](int64_t side) { return ((m + side - 1) / side) * ((n + side - 1) / side); };
   auto cost = [&](int64_t side, double weight) {
-    const int64_t tiles = ((m + side - 1) / side) * ((n + side - 1) / side);
-    return double((tiles + kSms - 1) / kSms) * double(side * side) * weight;
+    return double((tiles(side) + kSms - 1) / kSms) * double(side * side) * weight;
   };
   const double c128 = cost(128, 1.0), c64 = cost(64, 1.02), c32 = cost(32, 1.2);
   if (c32 < c64 && c32 < c128) return 32;
-  return c64 < c128 ? 64 : 128;
+  if (c64 >= c128) return 128;
+  // A shallow product is its tiles' fill, first copies and stores: a wave of 128 tiles takes 5 us and
+  // 2.3 us per K tile, a wave of 64 tiles (two on an SM) 2.9 and 1.15 us (us, 128 / 64: 2048 x 2048 x
+  // 32 19.0 / 20.2, 2500 x 2500 x 16 21.0 / 22.1, 3000 x 3000 x 20 36.8 / 39.0, but 1700 x 1700 x 32
+  // 18.7 / 15.3, 1000 x 1000 x 16 7.7 / 4.9).  Many waves are bound by the copies and stores, where
+  // 8-byte copies favour the smaller tile (7000 x 7000 x 4: 140 / 148 aligned, 173 / 165 not).
+  if (k <= 64) {
+    const double kt = double((k + kDBK - 1) / kDBK);
+    const int64_t w128 = (tiles(128) + kSms - 1) / kSms, w64 = (tiles(64) + 2 * kSms - 1) / (2 * kSms);
+    if ((wide || w128 <= 6) && double(w128) * (5.0 + 2.3 * kt) < double(w64) * (2.9 + 1.15 * kt)) return 128;
+  }
+  return 64;
 }
-
-}  // namespace
 
 cudaError_t launch_dgemm_native(bool transA, bool transB, int64_t m, int64_t n, int64_t k, double alpha,
                                 const double* A, int64_t lda, const double* B, int64_t ldb, double beta, double* C,
                                 int64_t ldc, const int* only_if_flag, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return cudaSuccess;
   // a launch that will usually leave at once (only_if_flag) takes the fewest blocks
-  const int tile = only_if_flag ? 128 : dmma_tile(m, n);
+  const int tile = only_if_flag ? 128 : dmma_tile(m, n, k, dmma_wide(A, lda) && dmma_wide(B, ldb));
   auto go = [&](auto d) {
     return launch_dmma<decltype(d)>(transA, transB, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, only_if_flag,
                                     stream);

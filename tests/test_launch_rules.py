@@ -25,3 +25,14 @@ def test_small_sgemm_pays_whole_k_tiles(rounds, k, small):
     applies = _rule("_ZN3eb219sgemm_small_appliesElll", ctypes.c_bool, I64, I64, I64)
     assert applies(148 * 32, 32 * rounds, k) == small
     assert applies(32 * rounds, 148 * 32, k) == small
+
+
+@pytest.mark.parametrize("m,n,k,aligned,unaligned", [
+    (2048, 2048, 32, 128, 128), (2500, 2500, 16, 128, 128), (3000, 3000, 20, 128, 128), (1300, 1300, 16, 128, 128),
+    (7000, 7000, 4, 128, 64), (1700, 1700, 32, 64, 64), (1000, 1000, 16, 64, 64), (3500, 1000, 24, 64, 64),
+    (2048, 2048, 128, 64, 64), (128, 128, 128, 32, 32), (4096, 4096, 1024, 128, 128)])
+def test_native_tile_of_shallow_products(m, n, k, aligned, unaligned):
+    # few K tiles: the wave's fixed cost decides, as timed
+    tile = _rule("_ZN3eb29dmma_tileElllb", ctypes.c_int, I64, I64, I64, ctypes.c_bool)
+    assert tile(m, n, k, True) == aligned
+    assert tile(m, n, k, False) == unaligned
