@@ -16,7 +16,7 @@
 //     flight while the current stage computes, which hides the latency of these short,
 //     scattered products' loads;
 //   * bound by the L1 data pipe (66 % busy for FP64: element-wise copies in, fragments out) and issue
-//     slots (57 %; DMMA pipe 46 %), so a stage carries no work for padding: lines outside the product are
+//     slots (60 %; DMMA pipe 50 %), so a stage carries no work for padding: lines outside the product are
 //     not copied (their outputs are not stored), only the K tail is zero-filled, and the fragments
 //     computed are those the item has (FP32: column fragments in pairs, four variants of the stage
 //     instead of eight, which the instruction cache holds: 262 -> 249 us).  10,000 products of sides
@@ -55,6 +55,15 @@ constexpr int kWarpsPerBlock = 2;
 constexpr int kStages64 = 2;  // 9.2 KB per block
 constexpr int kStages32 = 3;  // 6.9 KB per warp
 constexpr int kBlocks64 = 12, kBlocks32 = 8;  // per SM
+// A launch of few items is the latency of one item's chain of stages, and memory for longer rings and
+// registers for more copies in flight are free: FP64 takes a longer ring (us, 2 stages / 4: 100
+// products of 32 x 32 x 2048 184 / 119, 30 of 64 x 64 x 4096 377 / 246; 1184 items, eight per SM, 69 /
+// 69), and both unroll the copies of small products, FP32 with a copy path of its own where all are
+// small (500 products of 8 x 8 x 4000 361 / 297, 100 of 16 x 16 x 4000 343 / 275; 343 and 287 in the
+// kernel that knows tiles too).  Unrolled, FP32 is slower from 1184 items on (62.8 / 67.7).
+constexpr int kDeepStages64 = 4;
+constexpr int64_t kDeepK = 128;  // the longest item's K, at least (at 32 the ring only takes longer to fill)
+constexpr int kDeepBlocks64 = 6, kDeepBlocks32 = 2;  // per SM, at most
 constexpr int kPanelElems = kKc * kLineStride;
 // K rows 4 .. 7 of an FP64 panel start two elements later: the 8-byte copies of a half-warp, 8 K
 // offsets of two lines, then hit distinct banks, and so do its fragment reads (307.5 -> 299.3 us).
@@ -201,9 +210,12 @@ struct PanelCopy {
 
   // `contig`: the lines are contiguous (element t is K offset t); `left`: K from the stage's start to
   // the end; `wide`: class 32 and the step fits 32 bits (`left` and `contig` are then the warp's).
+  // SMALL: no item of class 32.
+  template <bool DEEP, bool SMALL>
   __device__ __forceinline__ void issue(uint32_t panel, const void* dummy, bool contig, int left, int r, bool wide) {
+    constexpr int kUnroll = DEEP ? kKc : 16 / kSize;
     const uint32_t d = panel + dst0;
-    if (wide) {
+    if (!SMALL && wide) {
       using Seq = std::make_integer_sequence<int, kKc>;
       if (contig)
         issue_wide<true>(d, left, Seq{});
@@ -214,7 +226,14 @@ struct PanelCopy {
       uint32_t dt = d;
       const uint32_t dstep = uint32_t((contig ? kLineStride : r / kKc) * kSize);
       const int kk0 = contig ? 0 : int(threadIdx.x) % kKc;  // ls % kKc: R is a multiple of kKc
-#pragma unroll 2
+      if (SMALL && __all_sync(0xffffffffu, left >= kKc)) {
+#pragma unroll
+        for (int t = 0; t < kKc; ++t, p += step, dt += dstep)
+          cp_async_elem_if<kSize, 0>(dt + (contig && t >= 4 ? kRowGap<T> * kSize : 0), p, t, valid);
+        ptr += contig ? kKc * step : int64_t(kKc * kSize);
+        return;
+      }
+#pragma unroll kUnroll
       for (int t = 0; t < kKc; ++t, p += step, dt += dstep) {
         const bool in = kk0 + (contig ? t : 0) < left;
         const uint32_t gap = contig && t >= 4 ? kRowGap<T> * kSize : 0;
@@ -257,8 +276,9 @@ struct ItemCopy {
     open(src, it, lane, false, pa);
     how &= wide_b;
   }
+  template <bool DEEP, bool SMALL>
   __device__ __forceinline__ void issue(PanelCopy<T>& p, const T* panel, bool rhs, const void* dummy) const {
-    p.issue(smem_u32(panel), dummy, (how & (rhs ? 128u : 64u)) != 0u, left, int(how & 63u), (how & 256u) != 0u);
+    p.template issue<DEEP, SMALL>(smem_u32(panel), dummy, (how & (rhs ? 128u : 64u)) != 0u, left, int(how & 63u), (how & 256u) != 0u);
   }
 };
 
@@ -296,18 +316,28 @@ __device__ __forceinline__ void frag_b(const float* sB, int l0, int g, int tig, 
   const float* x = sB + (2 * tig) * kLineStride + l0 + g;
   split_pair(x[0], x[kLineStride], p[0], p[1], p[2]);
 }
-// the six piece products of one 8-deep chunk, smallest first, into a fresh fragment that is
-// then added to the result (round to nearest)
-__device__ __forceinline__ void chunk_product(float (&acc)[4], const uint32_t (&pa)[3][2], const uint32_t (&pb)[3]) {
-  float d[4];
-  mma_bf16_1688_fresh(d, pa[0], pb[2]);  // h l
-  mma_bf16_1688(d, pa[2], pb[0]);        // l h
-  mma_bf16_1688(d, pa[1], pb[1]);        // m m
-  mma_bf16_1688(d, pa[0], pb[1]);        // h m
-  mma_bf16_1688(d, pa[1], pb[0]);        // m h
-  mma_bf16_1688(d, pa[0], pb[0]);        // h h
+// C fragments' six piece products of one 8-deep chunk, smallest first, each into a fresh fragment that
+// is then added to its result (round to nearest): fragment c is acc[slot(c)] += A piece ia(c) times B
+// piece ib(c).  The chains of six go a step of each in turn, or a lone warp would wait for each MMA
+// (100 products of 32 x 32 x 2048, A transposed: 215 -> 197 us with the copies above).
+template <int C, int NA, int NB, class Slot, class Ia, class Ib>
+__device__ __forceinline__ void chunk_products(float (&acc)[8][4], const uint32_t (&pa)[NA][3][2],
+                                               const uint32_t (&pb)[NB][3], Slot slot, Ia ia, Ib ib) {
+  constexpr int kPieceA[6] = {0, 2, 1, 0, 1, 0}, kPieceB[6] = {2, 0, 1, 1, 0, 0};  // hl lh mm hm mh hh
+  float d[C][4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) acc[e] = __fadd_rn(acc[e], d[e]);
+  for (int q = 0; q < 6; ++q)
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      if (q == 0)
+        mma_bf16_1688_fresh(d[c], pa[ia(c)][kPieceA[q]], pb[ib(c)][kPieceB[q]]);
+      else
+        mma_bf16_1688(d[c], pa[ia(c)][kPieceA[q]], pb[ib(c)][kPieceB[q]]);
+    }
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[slot(c)][e] = __fadd_rn(acc[slot(c)][e], d[c][e]);
 }
 // MI row blocks (of 16) by NJ column blocks (of 8) of a class-32 stage.
 template <int MI, int NJ>
@@ -317,10 +347,10 @@ __device__ __forceinline__ void stage32(float (&acc)[8][4], const float* st, int
   for (int i = 0; i < MI; ++i) frag_a(st, i * 16, false, g, tig, pa[i]);
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
-    uint32_t pb[3];
-    frag_b(st + kPanelElems, j * 8, g, tig, pb);
-#pragma unroll
-    for (int i = 0; i < MI; ++i) chunk_product(acc[i * 4 + j], pa[i], pb);
+    uint32_t pb[1][3];
+    frag_b(st + kPanelElems, j * 8, g, tig, pb[0]);
+    chunk_products<MI>(
+        acc, pa, pb, [j](int i) { return i * 4 + j; }, [](int i) { return i; }, [](int) { return 0; });
   }
 }
 
@@ -329,32 +359,32 @@ __device__ __forceinline__ void stage_small(float (&acc)[8][4], const float* st,
   const float* sA = st;
   const float* sB = st + kPanelElems;
   if (mid) {
+    uint32_t pa[2][3][2], pb[4][3];
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
-      uint32_t pa[3][2];
-      frag_a(sA, p * 16, false, g, tig, pa);
+      frag_a(sA, p * 16, false, g, tig, pa[p]);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        uint32_t pb[3];
-        frag_b(sB, p * 16 + j * 8, g, tig, pb);
-        chunk_product(acc[p * 2 + j], pa, pb);
-      }
+      for (int j = 0; j < 2; ++j) frag_b(sB, p * 16 + j * 8, g, tig, pb[p * 2 + j]);
     }
+    chunk_products<4>(
+        acc, pa, pb, [](int c) { return c; }, [](int c) { return c / 2; }, [](int c) { return c; });
   } else {
+    uint32_t pa[4][3][2], pb[4][3];
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-      uint32_t pa[3][2], pb[3];
-      frag_a(sA, p * 8, true, g, tig, pa);
-      frag_b(sB, p * 8, g, tig, pb);
-      chunk_product(acc[p], pa, pb);
+      frag_a(sA, p * 8, true, g, tig, pa[p]);
+      frag_b(sB, p * 8, g, tig, pb[p]);
     }
+    chunk_products<4>(
+        acc, pa, pb, [](int c) { return c; }, [](int c) { return c; }, [](int c) { return c; });
   }
 }
 
 // One stage of an item: the fragments it has (grouped_frags), nothing for padding.
+template <bool SMALL>
 __device__ __forceinline__ void compute_stage(float (&acc)[8][4], const float* st, const GroupedItem& it, int g,
                                               int tig) {
-  if (it.cls != 32) return stage_small(acc, st, it.cls == 16, g, tig);
+  if (SMALL || it.cls != 32) return stage_small(acc, st, it.cls == 16, g, tig);
   switch (it.frags >> 1) {
     case 0: return stage32<1, 2>(acc, st, g, tig);
     case 1: return stage32<1, 4>(acc, st, g, tig);
@@ -418,10 +448,10 @@ __device__ __forceinline__ void store_tile(const ProductStore<T>& ps, int64_t r0
   }
 }
 
-template <class Src>
+template <bool SMALL, class Src>
 __device__ __forceinline__ void epilogue_f32(const Src& src, const GroupedItem& it, float (&acc)[8][4], int g, int tig) {
   ProductStore<float> ps;
-  if (it.cls == 32) {
+  if (!SMALL && it.cls == 32) {
     ps.load(src.problem(it.problem[0]));
     store_tile<2, 4>(ps, int64_t(it.tile_m) * 32 + g, int64_t(it.tile_n) * 32 + 2 * tig, (it.frags & 3) + 1, acc);
   } else if (it.cls == 16) {
@@ -448,11 +478,10 @@ __device__ __forceinline__ void epilogue_f32(const Src& src, const GroupedItem& 
 }
 
 // ---------------------------------------------------------------- FP32: a warp's pipeline
-// Items w0, w0 + W, w0 + 2W, ... in stage order; copies run kStages32 - 1 stages ahead of the
+// Items w0, w0 + W, w0 + 2W, ... in stage order; copies run S - 1 stages ahead of the
 // compute, across item boundaries.
-template <class Src>
+template <int S, bool DEEP, bool SMALL, class Src>
 __device__ __forceinline__ void run_items_f32(const Src& src, int64_t w0, int64_t W, float* ring) {
-  constexpr int S = kStages32;
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
 
@@ -474,8 +503,8 @@ __device__ __forceinline__ void run_items_f32(const Src& src, int64_t w0, int64_
   auto produce = [&](int slot) {
     if (p_idx < src.count) {
       const float* stage = ring + slot * kStageElems;
-      cp.issue(pa, stage, false, dummy);
-      cp.issue(pb, stage + kPanelElems, true, dummy);
+      cp.template issue<DEEP, SMALL>(pa, stage, false, dummy);
+      cp.template issue<DEEP, SMALL>(pb, stage + kPanelElems, true, dummy);
       cp.left -= kKc;
       if (--p_left == 0) {
         p_idx += W;
@@ -507,10 +536,10 @@ __device__ __forceinline__ void run_items_f32(const Src& src, int64_t w0, int64_
     cp_async_wait<S - 2>();
     __syncwarp();  // every lane's copies of this stage have landed; the slot refilled below is free
     produce(slot == 0 ? S - 1 : slot - 1);
-    compute_stage(acc, ring + slot * kStageElems, cur, g, tig);
+    compute_stage<SMALL>(acc, ring + slot * kStageElems, cur, g, tig);
     slot = slot == S - 1 ? 0 : slot + 1;
     if (--c_stages == 0) {
-      epilogue_f32(src, cur, acc, g, tig);
+      epilogue_f32<SMALL>(src, cur, acc, g, tig);
 #pragma unroll
       for (int f = 0; f < 8; ++f)
 #pragma unroll
@@ -530,9 +559,8 @@ __device__ __forceinline__ void run_items_f32(const Src& src, int64_t w0, int64_
 // columns of op(B); each computes half of the fragments: a 16-row block of a 32 x 32 tile (or half
 // of its columns when it has one row block), one of two products, two of four.  Half the FP64 sums
 // per lane leaves registers for 24 warps per SM instead of 16, with half the copies each.
-template <class Src>
+template <int S, bool DEEP, class Src>
 __device__ __forceinline__ void run_items_f64(const Src& src, int64_t w0, int64_t W, double* ring) {
-  constexpr int S = kStages64;
   const int warp = int(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
 
@@ -551,7 +579,7 @@ __device__ __forceinline__ void run_items_f64(const Src& src, int64_t w0, int64_
   const void* const dummy = src.dummy();
   auto produce = [&](int slot) {
     if (p_idx < src.count) {
-      cp.issue(pc, ring + slot * kStageElems + warp * kPanelElems, warp != 0, dummy);
+      cp.template issue<DEEP, false>(pc, ring + slot * kStageElems + warp * kPanelElems, warp != 0, dummy);
       cp.left -= kKc;
       if (--p_left == 0) {
         p_idx += W;
@@ -651,67 +679,83 @@ __device__ __forceinline__ void run_items_f64(const Src& src, int64_t w0, int64_
   cp_async_wait<0>();
 }
 
-constexpr size_t kRing64 = size_t(kStages64) * kStageElems * sizeof(double);
-constexpr size_t kRing32 = size_t(kStages32) * kStageElems * sizeof(float);
+// Dynamic shared memory of a block: a ring per item at a time.
+template <typename T>
+constexpr size_t ring_bytes(int stages) {
+  return size_t(stages) * kStageElems * sizeof(T) * (sizeof(T) == 8 ? 1 : kWarpsPerBlock);
+}
 
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, kBlocks64)
+template <bool DEEP>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, DEEP ? kDeepBlocks64 : kBlocks64)
     grouped_f64_kernel(const GroupedProblem* __restrict__ problems, const GroupedItem* __restrict__ items,
                        int64_t num_items) {
   extern __shared__ __align__(16) unsigned char grouped_smem[];
-  run_items_f64(PlanItems{problems, items, num_items}, int64_t(blockIdx.x), int64_t(gridDim.x),
-                reinterpret_cast<double*>(grouped_smem));
+  run_items_f64<DEEP ? kDeepStages64 : kStages64, DEEP>(PlanItems{problems, items, num_items}, int64_t(blockIdx.x),
+                                                        int64_t(gridDim.x), reinterpret_cast<double*>(grouped_smem));
 }
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, kBlocks32)
+template <bool DEEP, bool SMALL>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, DEEP ? kDeepBlocks32 : kBlocks32)
     grouped_f32_kernel(const GroupedProblem* __restrict__ problems, const GroupedItem* __restrict__ items,
                        int64_t num_items) {
   extern __shared__ __align__(16) unsigned char grouped_smem[];
   const int warp = threadIdx.x >> 5;
-  run_items_f32(PlanItems{problems, items, num_items}, int64_t(blockIdx.x) * kWarpsPerBlock + warp,
-                int64_t(gridDim.x) * kWarpsPerBlock,
-                reinterpret_cast<float*>(grouped_smem) + size_t(warp) * kStages32 * kStageElems);
+  run_items_f32<kStages32, DEEP, SMALL>(
+      PlanItems{problems, items, num_items}, int64_t(blockIdx.x) * kWarpsPerBlock + warp,
+      int64_t(gridDim.x) * kWarpsPerBlock, reinterpret_cast<float*>(grouped_smem) + size_t(warp) * kStages32 * kStageElems);
 }
 
-// One FP32 product, one warp per 32 x 32 tile: the per-product launches of the same arithmetic.
-__global__ void __launch_bounds__(32) grouped_one_kernel(const GroupedProblem pr, int tiles_m, int64_t tiles) {
+// One FP32 product, one warp per 32 x 32 tile: the per-product launches of the same arithmetic.  A
+// warp alone on its scheduler, so it takes the registers it can use (without a block count the
+// compiler keeps to 104 of them: 10 products of 128 x 100 x 2000 2.53 / 1.80 ms).
+__global__ void __launch_bounds__(32, 1) grouped_one_kernel(const GroupedProblem pr, int tiles_m, int64_t tiles) {
   extern __shared__ __align__(16) unsigned char grouped_smem[];
-  run_items_f32(OneProduct{pr, tiles_m, tiles}, int64_t(blockIdx.x), int64_t(gridDim.x),
-                reinterpret_cast<float*>(grouped_smem));
+  run_items_f32<kStages32, false, false>(OneProduct{pr, tiles_m, tiles}, int64_t(blockIdx.x), int64_t(gridDim.x),
+                                  reinterpret_cast<float*>(grouped_smem));
 }
 
 cudaError_t set_smem(const void* kern, size_t bytes) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
 }
 
+struct GroupedKernel {
+  void (*kern)(const GroupedProblem*, const GroupedItem*, int64_t);
+  size_t smem;
+};
+GroupedKernel grouped_kernel(bool f64, GroupedVariant v) {
+  if (f64)
+    return v == GroupedVariant::kMany ? GroupedKernel{grouped_f64_kernel<false>, ring_bytes<double>(kStages64)}
+                                      : GroupedKernel{grouped_f64_kernel<true>, ring_bytes<double>(kDeepStages64)};
+  return GroupedKernel{v == GroupedVariant::kMany       ? grouped_f32_kernel<false, false>
+                       : v == GroupedVariant::kFewSmall ? grouped_f32_kernel<true, true>
+                                                        : grouped_f32_kernel<true, false>,
+                       ring_bytes<float>(kStages32)};
+}
+
 }  // namespace
 
-size_t grouped_block_smem(bool f64) { return f64 ? kRing64 : kWarpsPerBlock * kRing32; }
-
-cudaError_t grouped_grid(bool f64, int64_t num_items, int num_sms, unsigned* blocks) {
-  *blocks = 0;
-  const size_t smem = grouped_block_smem(f64);
-  const void* kern =
-      f64 ? reinterpret_cast<const void*>(grouped_f64_kernel) : reinterpret_cast<const void*>(grouped_f32_kernel);
-  cudaError_t e = set_smem(kern, smem);
-  if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarpsPerBlock, smem);
-  if (e != cudaSuccess) return e;
+cudaError_t grouped_grid(bool f64, int64_t num_items, int64_t longest, bool small, int num_sms, GroupedGrid* grid) {
   const int64_t per_block = f64 ? 1 : kWarpsPerBlock;  // items at a time
   int64_t b = (num_items + per_block - 1) / per_block;
+  const bool few = b <= int64_t(num_sms) * (f64 ? kDeepBlocks64 : kDeepBlocks32) && longest >= kDeepK;
+  *grid = GroupedGrid{0, !few ? GroupedVariant::kMany : (small ? GroupedVariant::kFewSmall : GroupedVariant::kFew)};
+  const GroupedKernel k = grouped_kernel(f64, grid->variant);
+  cudaError_t e = set_smem(reinterpret_cast<const void*>(k.kern), k.smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(k.kern), 32 * kWarpsPerBlock,
+                                                    k.smem);
+  if (e != cudaSuccess) return e;
   const int64_t cap = int64_t(num_sms) * (per_sm > 0 ? per_sm : 1);
   if (b > cap) b = cap;
-  *blocks = unsigned(b > 0 ? b : 0);
+  grid->blocks = unsigned(b > 0 ? b : 0);
   return cudaSuccess;
 }
 
 cudaError_t launch_grouped_gemm(bool f64, const GroupedProblem* problems, const GroupedItem* items,
-                                int64_t num_items, unsigned blocks, cudaStream_t stream) {
-  if (num_items <= 0 || blocks == 0) return cudaSuccess;
-  const size_t smem = grouped_block_smem(f64);
-  if (f64)
-    grouped_f64_kernel<<<blocks, 32 * kWarpsPerBlock, smem, stream>>>(problems, items, num_items);
-  else
-    grouped_f32_kernel<<<blocks, 32 * kWarpsPerBlock, smem, stream>>>(problems, items, num_items);
+                                int64_t num_items, GroupedGrid grid, cudaStream_t stream) {
+  if (num_items <= 0 || grid.blocks == 0) return cudaSuccess;
+  const GroupedKernel k = grouped_kernel(f64, grid.variant);
+  k.kern<<<grid.blocks, 32 * kWarpsPerBlock, k.smem, stream>>>(problems, items, num_items);
   return cudaGetLastError();
 }
 
@@ -719,11 +763,12 @@ cudaError_t launch_grouped_one(const GroupedProblem& pr, cudaStream_t stream) {
   if (pr.m <= 0 || pr.n <= 0) return cudaSuccess;
   const int64_t tm = (pr.m + 31) / 32, tn = (pr.n + 31) / 32;
   if (tm > 65535 || tn > 65535) return cudaErrorInvalidValue;
-  const cudaError_t e = set_smem(reinterpret_cast<const void*>(grouped_one_kernel), kRing32);
+  constexpr size_t kSmem = ring_bytes<float>(kStages32) / kWarpsPerBlock;
+  const cudaError_t e = set_smem(reinterpret_cast<const void*>(grouped_one_kernel), kSmem);
   if (e != cudaSuccess) return e;
   const int64_t tiles = tm * tn;
   const unsigned grid = unsigned(tiles < 65535 ? tiles : 65535);
-  grouped_one_kernel<<<grid, 32, kRing32, stream>>>(pr, int(tm), tiles);
+  grouped_one_kernel<<<grid, 32, kSmem, stream>>>(pr, int(tm), tiles);
   return cudaGetLastError();
 }
 

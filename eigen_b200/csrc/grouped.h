@@ -40,19 +40,25 @@ __host__ __device__ inline uint8_t grouped_frags(int64_t m, int64_t n, int tile_
   return uint8_t((rows > 16 ? 4 : 0) + (cols > 24 ? 3 : int(cols - 1) / 8));
 }
 
-// Grid of the persistent grouped kernel for `num_items` items (as many two-warp blocks as fit
-// on the SMs, at most one worker per item); sets the kernel's shared-memory attribute.  Call it
-// outside any stream capture.
-cudaError_t grouped_grid(bool f64, int64_t num_items, int num_sms, unsigned* blocks);
-// Launches the persistent grouped kernel for `num_items` items on `stream` with `blocks`
-// blocks from grouped_grid (capturable).
+// The kernels of a launch: for many items (or shallow ones), for so few that latency within an item
+// counts, and for few items without a class-32 one.
+enum class GroupedVariant { kMany, kFew, kFewSmall };
+// Grid of the persistent grouped kernel.
+struct GroupedGrid {
+  unsigned blocks;
+  GroupedVariant variant;
+};
+// The grid for `num_items` items (as many two-warp blocks as fit on the SMs, at most one worker per
+// item; `longest`: the largest k of an item; `small`: none of class 32); sets the kernel's
+// shared-memory attribute.  Call it outside any stream capture.
+cudaError_t grouped_grid(bool f64, int64_t num_items, int64_t longest, bool small, int num_sms, GroupedGrid* grid);
+// Launches the persistent grouped kernel for `num_items` items on `stream` with the grid from
+// grouped_grid (capturable).
 cudaError_t launch_grouped_gemm(bool f64, const GroupedProblem* problems, const GroupedItem* items,
-                                int64_t num_items, unsigned blocks, cudaStream_t stream);
+                                int64_t num_items, GroupedGrid grid, cudaStream_t stream);
 // The same arithmetic for one FP32 product (one warp per 32 x 32 tile): the per-product launches
 // that a grouped launch replaces (FP64: the native kernel's, the same bits).
 cudaError_t launch_grouped_one(const GroupedProblem& pr, cudaStream_t stream);
-// Dynamic shared memory of one block of the grouped kernel.
-size_t grouped_block_smem(bool f64);
 
 // Largest max(m, n) of the products that share a warp four (class 8) or two (class 16) at a
 // time; 0 disables the class.  Process-wide; read when a plan is built.

@@ -215,12 +215,15 @@ int eb2_grouped_plan_create(char dtype, int64_t count, const eb2_gemm_problem* p
     ok = eb2::cuda_ok(cudaMemcpy(p->d_items, items.data(), items.size() * sizeof(eb2::GroupedItem),
                                  cudaMemcpyHostToDevice),
                       "upload schedule");
-  unsigned blocks = 0;
-  ok = ok && eb2::cuda_ok(eb2::grouped_grid(p->f64, p->num_items, cx->num_sms, &blocks), "grouped grid");
+  eb2::GroupedGrid grid{};
+  const bool small =
+      std::none_of(items.begin(), items.end(), [](const eb2::GroupedItem& it) { return it.cls == 32; });
+  const int64_t longest = items.empty() ? 0 : items[0].k;  // longest K first
+  ok = ok && eb2::cuda_ok(eb2::grouped_grid(p->f64, p->num_items, longest, small, cx->num_sms, &grid), "grouped grid");
   if (ok) {
     ok = eb2::cuda_ok(cudaStreamBeginCapture(p->capture_stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     if (ok) {
-      cudaError_t le = eb2::launch_grouped_gemm(p->f64, p->d_problems, p->d_items, p->num_items, blocks,
+      cudaError_t le = eb2::launch_grouped_gemm(p->f64, p->d_problems, p->d_items, p->num_items, grid,
                                                p->capture_stream);
       cudaError_t ee = cudaStreamEndCapture(p->capture_stream, &p->graph);
       ok = eb2::cuda_ok(le, "grouped launch (capture)") && eb2::cuda_ok(ee, "end capture");

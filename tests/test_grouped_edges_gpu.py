@@ -21,13 +21,13 @@ def defaults():
     eb.set_dgemm_method(eb.METHOD_AUTO)
 
 
-def _problems(dtype, seed):
+def _problems(dtype, seed, deeper=0):
     rng = np.random.default_rng(seed)
     td = torch.float64 if dtype == "d" else torch.float32
     probs, keep = [], []
     for i, m in enumerate(SIDES):
         for j, n in enumerate(SIDES):
-            k = DEPTHS[(3 * i + j) % len(DEPTHS)]
+            k = DEPTHS[(3 * i + j) % len(DEPTHS)] + deeper
             ta, tb, pad = "NT"[i % 2], "NT"[j % 2], (i + j) % 3
             ar, ac = (m, k) if ta == "N" else (k, m)
             br, bc = (k, n) if tb == "N" else (n, k)
@@ -97,3 +97,60 @@ def test_large_leading_dimension(dtype):
         torch.cuda.synchronize()
         out.append(c)
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("dtype", ["d", "s"])
+@pytest.mark.parametrize("classes", [(8, 16), (0, 0)])
+def test_few_and_many_items_agree(dtype, classes):
+    # the kernel of a launch of few deep items and that of many: the same bits
+    eb.set_grouped_classes(*classes)
+    probs, keep = _problems(dtype, 13, 128)
+    many = [dict(p, c=p["c"].clone()) for _ in range(30) for p in probs]
+    # and that of few items without a 32 x 32 tile
+    small = [i for i, p in enumerate(probs) if max(p["m"], p["n"]) <= 16]
+    few_small = [dict(probs[i], c=probs[i]["c"].clone()) for i in small]
+    assert eb.gemm_grouped(dtype, probs) == eb.EB2_OK
+    assert eb.gemm_grouped(dtype, many) == eb.EB2_OK
+    assert eb.gemm_grouped(dtype, few_small) == eb.EB2_OK
+    torch.cuda.synchronize()
+    for i, p in enumerate(many):
+        assert torch.equal(p["c"], probs[i % len(probs)]["c"]), i
+    for i, p in zip(small, few_small):
+        assert torch.equal(p["c"], probs[i]["c"]), i
+
+
+def _deep(dtype, count, k=8192):
+    td = torch.float64 if dtype == "d" else torch.float32
+    a = torch.rand((count, k, 32), dtype=td, device="cuda")
+    b = torch.rand((count, 32, k), dtype=td, device="cuda")
+    c = torch.zeros((count, 32, 32), dtype=td, device="cuda")
+    return [dict(m=32, n=32, k=k, a=a[i], lda=32, b=b[i], ldb=k, c=c[i], ldc=32) for i in range(count)]
+
+
+def _best_ms(run):
+    times = []
+    for _ in range(8):
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        run()
+        t1.record()
+        torch.cuda.synchronize()
+        times.append(t0.elapsed_time(t1))
+    return min(times)
+
+
+def test_few_deep_fp64_items_hide_their_loads():
+    # one item per SM: the copies of the stages ahead must cover the latency of memory, so a hundred
+    # items whose operands do not fit L2 take about as long as one whose operands do
+    one, many = eb.GroupedPlan("d", _deep("d", 1)), eb.GroupedPlan("d", _deep("d", 100))
+    t1, t100 = _best_ms(one.execute), _best_ms(many.execute)
+    assert t100 < 1.25 * t1, (t1, t100)
+
+
+def test_one_fp32_product_per_launch_keeps_the_plan_s_pace():
+    # a warp per tile in both
+    probs = _deep("s", 1)
+    arr = eb.problems_array(probs)
+    plan = eb.GroupedPlan("s", probs)
+    t_plan, t_each = _best_ms(plan.execute), _best_ms(lambda: eb.gemm_each("s", arr))
+    assert t_each < 1.15 * t_plan, (t_plan, t_each)
