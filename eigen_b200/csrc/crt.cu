@@ -22,6 +22,7 @@
 // reproducible bit for bit and can be checked against an exact CPU model.
 #include <cuda.h>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -878,8 +879,6 @@ __device__ __forceinline__ void crt_reduce_energies(const CrtRecParams& R, doubl
   }
 }
 
-constexpr int kRecCols = 32;  // columns of a block that finishes a part of a triangle
-
 // Byte of row i, column j in a residue plane ([cols/4][ld_res][4]: the GEMM's epilogue writes four
 // neighbouring columns of a row as one word).
 __device__ __forceinline__ int64_t residue_index(int64_t i, int64_t j, int64_t ld_res) {
@@ -1616,6 +1615,35 @@ cudaError_t launch_crt_merge_splits(uint8_t* cres, int64_t plane, int moduli, in
   return cudaGetLastError();
 }
 
+// The blocks resident at four per SM work through the grid in rounds, and a block costs its run and
+// about one more group for its set-up and first copies; the fewest rounds that lose nothing to a last
+// one that is nearly empty.  2048^3: one round of 592 blocks (against runs of 4 .. 32 columns in three
+// rounds 267.0 -> 262.9 us a call).  Tall products, whose row blocks alone fill a good part of a round,
+// take several (a call, us, one run per resident block / these: 40000 x 2000 x 128 1325 / 1165, 76000 x
+// 1000 x 128 1419 / 1162, 152000 x 500 x 128 1393 / 1249).
+//
+// A triangle keeps half of the entries, in blocks of any share of work: runs short enough for two
+// rounds of blocks that have some, but four groups while those rounds are few and eight after (dsyrk,
+// K = 2000, us, always eight groups / these: n = 600 109 / 94, 2000 198 / 179, 3000 293 / 287).
+int64_t crt_rec_run(int64_t row_blocks, int64_t groups, bool triangle) {
+  constexpr int64_t kResident = 4 * 148;
+  if (triangle) {
+    const int64_t rounds = row_blocks * groups / (2 * kResident);
+    return rounds >= 16 ? 8 : std::min<int64_t>(std::max<int64_t>(rounds, 1), 4);
+  }
+  int64_t best = 0, best_cost = 0;
+  for (int64_t rounds = 1; rounds <= 16; ++rounds) {
+    const int64_t runs = std::max<int64_t>(rounds * kResident / row_blocks, 1);
+    const int64_t run = (groups + runs - 1) / runs, used = (groups + run - 1) / run;
+    const int64_t cost = (row_blocks * used + kResident - 1) / kResident * (run + 1);
+    if (best == 0 || cost < best_cost) {
+      best = run;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 cudaError_t launch_crt_reconstruct(const CrtReconstructArgs& args, cudaStream_t stream) {
   if (args.moduli < 1 || args.moduli > kCrtMaxModuli) return cudaErrorInvalidValue;
   if (args.m == 0 || args.n == 0) return cudaSuccess;
@@ -1652,16 +1680,7 @@ cudaError_t launch_crt_reconstruct(const CrtReconstructArgs& args, cudaStream_t 
                    args.plane >= (args.n + 3) / 4 * 4 * args.ld_res;
   const int64_t rows_per_block = 256;
   const unsigned gx = unsigned((args.m + rows_per_block - 1) / rows_per_block);
-  // Whole groups of four columns.  All of C: one run of groups per block, as many blocks as are
-  // resident at four per SM, so that set-up and first copies are paid once and every block ends
-  // together (against runs of 4 .. 32 columns in three rounds of blocks: 2048^3 267.0 -> 262.9 us,
-  // 4096 x 1024 x 3000 337.8 -> 335.2 us, dtrsm 4096 x 2048 1384 -> 1361 us, 8192^3 the same).  A
-  // triangle: runs of kRecCols, since a block may have nothing to do.
-  int64_t cpb = kRecCols;
-  if (args.uplo == 0) {
-    const int64_t runs = 4 * 148 / gx > 0 ? 4 * 148 / gx : 1, groups = (args.n + 3) / 4;
-    cpb = 4 * ((groups + runs - 1) / runs);
-  }
+  int64_t cpb = 4 * crt_rec_run(gx, (args.n + 3) / 4, args.uplo != 0);
   while ((args.n + cpb - 1) / cpb > 65535) cpb *= 2;  // gridDim.y
   R.cols_per_block = cpb;
   const dim3 grid(gx, unsigned((args.n + cpb - 1) / cpb));

@@ -36,3 +36,19 @@ def test_native_tile_of_shallow_products(m, n, k, aligned, unaligned):
     tile = _rule("_ZN3eb29dmma_tileElllb", ctypes.c_int, I64, I64, I64, ctypes.c_bool)
     assert tile(m, n, k, True) == aligned
     assert tile(m, n, k, False) == unaligned
+
+
+def test_reconstruction_rounds_of_blocks():
+    # 592 resident blocks; a round costs its run and one group: never much above an even split
+    run_of = _rule("_ZN3eb211crt_rec_runEllb", I64, I64, I64, ctypes.c_bool)
+    for row_blocks in [*range(1, 40), 100, 148, 157, 199, 297, 313, 400, 591, 592, 593, 594, 625, 1000, 3000]:
+        for groups in (1, 2, 7, 32, 125, 225, 250, 500, 512, 2048):
+            run = run_of(row_blocks, groups, False)
+            assert 1 <= run <= groups
+            used = -(-groups // run)
+            cost = -(-row_blocks * used // 592) * (run + 1)
+            even = row_blocks * groups / 592
+            assert cost <= 1.3 * even + 6, (row_blocks, groups, run, cost, even)
+            # the blocks with work fill the chip, unless a run is down to one group
+            tri = run_of(row_blocks, groups, True)
+            assert tri == 1 or row_blocks * (-(-groups // tri)) / 2 >= 592, (row_blocks, groups, tri)
