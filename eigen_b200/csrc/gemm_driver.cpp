@@ -317,21 +317,23 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
   ok = product(true);
   // IEEE semantics for NaN/Inf inputs: the FP64 kernel runs only when the scan saw one (for a
   // triangle into the workspace, then merged into the triangle).  A call that reads the flags on
-  // the host launches it when they say so; a stream-ordered one launches it behind the flag.
+  // the host launches it when they say so, without the flag: it will run, on the tile that fits.  A
+  // stream-ordered one launches it behind the flag.
+  const bool host_reads = opt.sync || check;
   auto non_finite = [&]() -> bool {
+    const int* const flag = host_reads ? nullptr : &df->nonfinite;
     if (!tri) {
       info.launches += 1;
-      return check_cuda(launch_dgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, &df->nonfinite, st),
+      return check_cuda(launch_dgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, flag, st),
                         "non-finite fallback");
     }
     double* full = reinterpret_cast<double*>(ws + o_full);
     info.launches += 2;
-    return check_cuda(launch_dgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, 0.0, full, m, &df->nonfinite, st),
+    return check_cuda(launch_dgemm_native(ta, tb, m, n, k, alpha, A, lda, B, ldb, 0.0, full, m, flag, st),
                       "non-finite fallback") &&
-           check_cuda(launch_merge_triangle<double>(full, m, n, opt.uplo == 1, beta, C, ldc, st, &df->nonfinite),
+           check_cuda(launch_merge_triangle<double>(full, m, n, opt.uplo == 1, beta, C, ldc, st, flag),
                       "non-finite merge");
   };
-  const bool host_reads = opt.sync || check;
   if (!host_reads) ok = ok && non_finite();
   if (!ok) return EB2_ERR_CUDA;
   info.slices = nmod;
@@ -365,7 +367,8 @@ int dgemm_crt(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t k, do
     }
     if (hf.nonfinite) {
       info.nonfinite = 1;
-      if (!non_finite() || (opt.sync && !check_cuda(cudaStreamSynchronize(st), "DGEMM"))) return EB2_ERR_CUDA;
+      // (a call with the check returns with C complete, as it does for finite inputs)
+      if (!non_finite() || !check_cuda(cudaStreamSynchronize(st), "DGEMM")) return EB2_ERR_CUDA;
       break;
     }
     // energies that overflowed (products near the FP64 range) leave the estimate unknown

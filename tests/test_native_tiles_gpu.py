@@ -2,6 +2,8 @@
 on both sides of the tile choice, every transpose, odd and even leading dimensions.  The sum of an
 output has one order whatever tile it lies in, so a product equals the same block of a larger
 product bit for bit; against FP64 sums of the absolute values it stays within k u."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -66,3 +68,37 @@ def test_tiles_update_c(m, n):
     # 1.5 p is rounded once and 0.5 c + that once more
     want = 0.5 * c[:, :m] + 1.5 * plain
     assert torch.equal(got[:, :m], want) and torch.equal(got[:, m], c[:, m])
+
+
+def test_fallback_of_a_checked_call_takes_the_tile_that_fits():
+    # a call that reads the flags on the host launches the fallback knowing that it will run: 16 tiles of
+    # 32 x 32; behind the flag it is one of 128 x 128, on one SM
+    m = n = 128
+    k = 8192
+    a = torch.rand((k, m), dtype=torch.float64, device="cuda")
+    b = torch.rand((n, k), dtype=torch.float64, device="cuda")
+    a[7, 3] = float("nan")
+    c = {flag: torch.zeros((n, m), dtype=torch.float64, device="cuda") for flag in (True, False)}
+
+    def call(check):
+        assert eb.dgemm_device("N", "N", m, n, k, 1.0, a, m, b, k, 0.0, c[check], m, check_accuracy=check) == eb.EB2_OK
+        torch.cuda.synchronize()
+
+    def best(check):
+        times = []
+        for _ in range(8):
+            t0 = time.perf_counter()
+            call(check)
+            times.append(time.perf_counter() - t0)
+        return min(times)
+
+    eb.set_dgemm_method(eb.METHOD_CRT)
+    try:
+        call(True)
+        assert eb.last_call_info()["nonfinite"] == 1
+        checked, flagged = best(True), best(False)
+    finally:
+        eb.set_dgemm_method(eb.METHOD_AUTO)
+    assert torch.equal(torch.nan_to_num(c[True], nan=-1.0), torch.nan_to_num(c[False], nan=-1.0))
+    assert torch.isnan(c[True][:, 3]).all() and torch.isnan(c[True]).sum() == n
+    assert checked < 0.7 * flagged, (checked, flagged)
