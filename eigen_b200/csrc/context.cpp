@@ -90,28 +90,32 @@ bool DeviceBuffer::ensure(size_t bytes) {
   return true;
 }
 
-int reserve_buffer(DeviceBuffer& buf, size_t bytes, cudaStream_t st, const char* what) {
+namespace {
+bool capturing(cudaStream_t st) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
-    (void)cudaGetLastError();
-    status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) != cudaSuccess) (void)cudaGetLastError();
+  return status != cudaStreamCaptureStatusNone;
+}
+}  // namespace
+
+bool try_reserve_buffer(DeviceBuffer& buf, size_t bytes, cudaStream_t st) {
+  if (!capturing(st)) return buf.ensure(bytes);
+  if (bytes > buf.cap) return false;
+  buf.held_by_graph = true;
+  return true;
+}
+
+int reserve_buffer(DeviceBuffer& buf, size_t bytes, cudaStream_t st, const char* what) {
+  if (try_reserve_buffer(buf, bytes, st)) return EB2_OK;
+  if (capturing(st)) {
+    set_error(EB2_ERR_ARG,
+              "a captured call needs %zu bytes of %s, more than the %zu sized so far; make a direct call of this "
+              "size first",
+              bytes, what, buf.cap);
+    return EB2_ERR_ARG;
   }
-  if (status != cudaStreamCaptureStatusNone) {
-    if (bytes > buf.cap) {
-      set_error(EB2_ERR_ARG,
-                "a captured call needs %zu bytes of %s, more than the %zu sized so far; make a direct call of this "
-                "size first",
-                bytes, what, buf.cap);
-      return EB2_ERR_ARG;
-    }
-    buf.held_by_graph = true;
-    return EB2_OK;
-  }
-  if (!buf.ensure(bytes)) {
-    set_error(EB2_ERR_ALLOC, "could not allocate %zu bytes of %s", bytes, what);
-    return EB2_ERR_ALLOC;
-  }
-  return EB2_OK;
+  set_error(EB2_ERR_ALLOC, "could not allocate %zu bytes of %s", bytes, what);
+  return EB2_ERR_ALLOC;
 }
 
 StreamFence::StreamFence(Context& cx, cudaStream_t st) : cx_(cx), st_(st), active_(false) {

@@ -34,6 +34,8 @@ struct DeviceBuffer {
 // enough becomes held by the graph.  Sets the thread's error on failure; `what` names the
 // buffer in the message.
 int reserve_buffer(DeviceBuffer& buf, size_t bytes, cudaStream_t st, const char* what);
+// The same for a caller that can do with less: false instead of an error.
+bool try_reserve_buffer(DeviceBuffer& buf, size_t bytes, cudaStream_t st);
 
 // Flags the kernels write; mirrored into pinned host memory after a call.
 struct DeviceFlags {

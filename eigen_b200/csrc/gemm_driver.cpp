@@ -679,10 +679,15 @@ int sgemm_on_device(Context& cx, bool ta, bool tb, int64_t m, int64_t n, int64_t
   const size_t o_b = off;
   off = align256(off + size_t(3) * n_pad * k_pad * 2);
   const int64_t tile_area = tile_m_of(tile_n, false) * tile_n_of(tile_n, false), tiles = m_pad * n_pad / tile_area;
-  const Bf16Split split = bf16_split_rule(tiles, k_pad, tile_n == kTilePair ? cx.num_sms / 2 : cx.num_sms);
+  Bf16Split split = bf16_split_rule(tiles, k_pad, tile_n == kTilePair ? cx.num_sms / 2 : cx.num_sms);
   const size_t o_part = off;
-  off = align256(off + size_t(split.ranges) * (tiles - split.whole_tiles) * tile_area * 4);
-  if (const int rc = reserve_buffer(cx.ws, off, st, "emulation workspace"); rc != EB2_OK) return rc;
+  const size_t part = size_t(split.ranges) * (tiles - split.whole_tiles) * tile_area * 4;
+  if (part == 0 || !try_reserve_buffer(cx.ws, off + part, st)) {
+    // no K ranges, or no room for their sums (a captured call cannot grow the workspace, and memory
+    // may be short): every tile over all of K
+    split = Bf16Split{tiles, 1};
+    if (const int rc = reserve_buffer(cx.ws, off, st, "emulation workspace"); rc != EB2_OK) return rc;
+  }
   uint8_t* ws = static_cast<uint8_t*>(cx.ws.ptr);
   Bf16Operand oa{ws + o_a, m, m_pad, k, k_pad};
   Bf16Operand ob{ws + o_b, n, n_pad, k, k_pad};
