@@ -473,16 +473,50 @@ __global__ void __launch_bounds__(kFThreads, 2)
     *reinterpret_cast<float4*>(p + 16) = make_float4(sum[4][j], sum[5][j], sum[6][j], sum[7][j]);
   }
   __syncthreads();
+  constexpr int kOut = kFTile * kFTile / kFThreads;  // outputs of a thread: row r, columns c0, c0 + 8, ..
+  const int r = t % kFTile, c0 = t / kFTile;
+  float v[kOut];
+  bool lost = false;  // an output of the product is not finite
 #pragma unroll
-  for (int idx = t; idx < kFTile * kFTile; idx += kFThreads) {
-    const int r = idx % kFTile, cc = idx / kFTile;
-    float v = fsmem[cc * kFLd + r];
+  for (int q = 0; q < kOut; ++q) {
+    const int cc = c0 + 8 * q;
+    v[q] = fsmem[cc * kFLd + r];
 #pragma unroll
-    for (int w = 1; w < kFWarps; ++w) v += fsmem[(w * kFTile + cc) * kFLd + r];
+    for (int w = 1; w < kFWarps; ++w) v[q] += fsmem[(w * kFTile + cc) * kFLd + r];
+    lost |= m0 + r < m && n0 + cc < n && !isfinite(v[q]);
+  }
+  if (__any_sync(0xffffffffu, lost)) {
+    // Partial sums that overflow with both signs add up to NaN.  One chain of FMAs keeps the infinity it
+    // reaches first, as the FFMA kernel's does; where NaN and Inf come from the operands it gives the
+    // same.  Rare, so a warp reads its operands again from global memory (edges clamped).
+    const int64_t row = m0 + r < m ? m0 + r : m - 1;
+    const float* ap = TA ? A + row * lda : A + row;
+    const float* bp[kOut];
+    float s[kOut];
+#pragma unroll
+    for (int q = 0; q < kOut; ++q) {
+      const int64_t col = n0 + c0 + 8 * q < n ? n0 + c0 + 8 * q : n - 1;
+      bp[q] = TB ? B + col : B + col * ldb;
+      s[q] = 0.f;
+    }
+    const int64_t sa = TA ? 1 : lda, sb = TB ? ldb : 1;
+#pragma unroll 8
+    for (int64_t l = 0; l < k; ++l) {
+      const float a = ap[l * sa];
+#pragma unroll
+      for (int q = 0; q < kOut; ++q) s[q] = fmaf(a, bp[q][l * sb], s[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kOut; ++q)
+      if (!isfinite(v[q])) v[q] = s[q];
+  }
+#pragma unroll
+  for (int q = 0; q < kOut; ++q) {
+    const int cc = c0 + 8 * q;
     if (m0 + r < m && n0 + cc < n) {
       float* dst = C + (m0 + r) + (n0 + cc) * ldc;
-      v = __fmul_rn(alpha, v);
-      *dst = (beta == 0.f) ? v : __fmaf_rn(beta, *dst, v);
+      const float x = __fmul_rn(alpha, v[q]);
+      *dst = (beta == 0.f) ? x : __fmaf_rn(beta, *dst, x);
     }
   }
 }

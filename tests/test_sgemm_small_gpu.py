@@ -77,3 +77,30 @@ def test_alpha_zero_and_empty():
     assert eb.sgemm_device("N", "N", 4, 4, 0, 1.0, a, 4, a, 4, 0.5, c, 4) == eb.EB2_OK
     torch.cuda.synchronize()
     assert torch.equal(c, torch.full_like(c, 0.25))
+
+
+@pytest.mark.parametrize("m,n,k", [(9, 103, 39), (70, 40, 200), (33, 31, 1000)])
+@pytest.mark.parametrize("ta,tb", [("N", "N"), ("T", "T")])
+def test_sums_that_overflow(m, n, k, ta, tb):
+    # products beyond the FP32 range with both signs: one chain of FMAs stays at the infinity it reaches
+    # first, as the FFMA kernel's does, and never turns to NaN
+    a, b, A, B = _operands(ta, tb, m, n, k, 2)
+    ar, ac = (m, k) if ta == "N" else (k, m)
+    a[:ac, :ar] *= 1e30
+    b[: b.shape[0] - 1, : b.shape[1] - 2] *= 1e20
+    a[:ac, :ar][torch.rand((ac, ar), device="cuda") < 0.5] *= 1e-30  # and some that stay in range
+    out = []
+    for method in (eb.METHOD_AUTO, eb.METHOD_NATIVE):
+        c = torch.zeros((n, m), device="cuda")
+        eb.set_sgemm_method(method)
+        try:
+            assert eb.sgemm_device(ta, tb, m, n, k, 1.0, a, a.shape[1], b, b.shape[1], 0.0, c, m) == eb.EB2_OK
+        finally:
+            eb.set_sgemm_method(eb.METHOD_AUTO)
+        out.append(c)
+    torch.cuda.synchronize()
+    small, ffma = out
+    assert torch.isinf(ffma).any() and not torch.isnan(ffma).any()
+    bad = ~torch.isfinite(small)
+    assert torch.equal(bad, torch.isinf(ffma))
+    assert torch.equal(small[bad], ffma[bad])
