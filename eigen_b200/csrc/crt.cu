@@ -707,43 +707,6 @@ __constant__ CrtTable kCrtTable = make_crt_table();
 // the same table as a compile-time value, for constants folded into instructions
 constexpr CrtTable kCrtTableC = make_crt_table();
 
-// Moduli 2g and 2g+1 share the factor Q_g = P / (p_2g p_2g+1) of their weights:
-// W_2g = Q_g X_2g and W_2g+1 = Q_g X_2g+1 with X_2g = p_2g+1 ((P/p_2g)^-1 mod p_2g) and
-// X_2g+1 = p_2g ((P/p_2g+1)^-1 mod p_2g+1), both below p_2g p_2g+1 < 2^16.  A last unpaired
-// modulus has Q = P/p and X = (P/p)^-1 mod p.  Then S = sum_l r_l W_l = sum_g Q_g R_g with
-// R_g = r_2g X_2g + r_2g+1 X_2g+1 < 2^25: the same S, with 32-bit multiply-adds for R_g and
-// half as many 64-bit ones for the 128-bit part.  Up to 16 moduli (P < 2^128).
-struct CrtPairTable {
-  uint32_t X[kCrtMaxModuli + 1][kCrtMaxModuli];
-  uint32_t Q[kCrtMaxModuli + 1][kCrtMaxModuli / 2][4];
-};
-__host__ __device__ constexpr CrtPairTable make_crt_pair_table() {
-  CrtPairTable t{};
-  for (int n = 1; n <= 16; ++n) {
-    uint32_t P[kCrtLimbs] = {1, 0, 0, 0, 0, 0};
-    for (int l = 0; l < n; ++l) ct_mul_small(P, uint32_t(crt_modulus(l)));
-    for (int g = 0; 2 * g < n; ++g) {
-      const bool pair = 2 * g + 1 < n;
-      const uint32_t pa = uint32_t(crt_modulus(2 * g)), pb = pair ? uint32_t(crt_modulus(2 * g + 1)) : 1u;
-      uint32_t Q[kCrtLimbs] = {P[0], P[1], P[2], P[3], P[4], P[5]};
-      (void)ct_div_small(Q, pa);
-      uint32_t Ma[kCrtLimbs] = {Q[0], Q[1], Q[2], Q[3], Q[4], Q[5]};  // P / p_a
-      const uint32_t ma = ct_div_small(Ma, pa);                        // (P / p_a) mod p_a
-      t.X[n][2 * g] = pb * ct_inverse_mod(ma, pa);
-      if (pair) {
-        uint32_t Mb[kCrtLimbs] = {P[0], P[1], P[2], P[3], P[4], P[5]};
-        (void)ct_div_small(Mb, pb);
-        const uint32_t mb = ct_div_small(Mb, pb);  // (P / p_b) mod p_b
-        t.X[n][2 * g + 1] = pa * ct_inverse_mod(mb, pb);
-        (void)ct_div_small(Q, pb);
-      }
-      for (int q = 0; q < 4; ++q) t.Q[n][g][q] = Q[q];
-    }
-  }
-  return t;
-}
-__constant__ CrtPairTable kCrtPairs = make_crt_pair_table();
-
 struct CrtRecParams {
   uint32_t W[kCrtMaxModuli][kCrtLimbs];
   uint32_t P[kCrtLimbs];
@@ -763,7 +726,7 @@ struct CrtRecParams {
   int write_c;
   double* save;
   int64_t ld_save;
-  int64_t cols_per_block;  // columns of a block (a multiple of 4; the per-row kernels: per pass)
+  int64_t cols_per_block;  // columns of a block (a multiple of 4; the per-row kernel: per pass)
   int uplo;            // 0: all of C; 1: i <= j only; 2: i >= j only
 };
 
@@ -969,99 +932,6 @@ __global__ void __launch_bounds__(256) crt_reconstruct_kernel(const __grid_const
   }
   __shared__ double red[2][8];
   if (R.err_sq) crt_reduce_energies(R, e_acc, v_acc, red);
-}
-
-// C' from the residues rc[0..N) of one entry (N <= 16): RN(|C'|) = d 2^shift, returns the
-// sign.  S = sum_g Q_g R_g, then R = S - q P with q = rint(S / P) and a range fix, exact in
-// 128-bit two's complement.
-template <int N>
-__device__ __forceinline__ bool crt_combine128(const uint32_t (&rc)[N], double P_inv, double& d, int& shift) {
-  using u128 = unsigned __int128;
-  using s128 = __int128;
-  const u128 P = (u128(kCrtTable.P[N][3]) << 96) | (u128(kCrtTable.P[N][2]) << 64) | (u128(kCrtTable.P[N][1]) << 32) |
-                 u128(kCrtTable.P[N][0]);
-  const s128 half = s128(P >> 1);
-  // S = sum_g Q_g R_g in four 32-bit limb columns (each < 8 * 2^25 * 2^32 = 2^60); S itself
-  // (< 2^28 P) may pass 2^128, and the 128-bit arithmetic below works modulo 2^128, which
-  // leaves the small remainder S - q P exact
-  unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-  for (int g = 0; 2 * g < N; ++g) {
-    uint32_t Rg = rc[2 * g] * kCrtPairs.X[N][2 * g];
-    if (2 * g + 1 < N) Rg += rc[2 * g + 1] * kCrtPairs.X[N][2 * g + 1];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] += static_cast<unsigned long long>(Rg) * kCrtPairs.Q[N][g][q];
-  }
-  // q = rint(S / P) from the partial sums in FP64; it may be off by one near a
-  // half-integer, which the range fix below absorbs
-  const double sd =
-      fma(double(acc[3]), 0x1p96, fma(double(acc[2]), 0x1p64, fma(double(acc[1]), 0x1p32, double(acc[0]))));
-  const u128 q = u128(static_cast<unsigned long long>(rint(sd * P_inv)));
-  const u128 S = u128(acc[0]) + (u128(acc[1]) << 32) + (u128(acc[2]) << 64) + (u128(acc[3]) << 96);
-  s128 r = s128(S - q * P);
-  if (r > half)
-    r -= s128(P);
-  else if (r < -half)
-    r += s128(P);
-  const bool negative = r < 0;
-  const u128 mag = negative ? u128(-r) : u128(r);
-  const unsigned long long hi = static_cast<unsigned long long>(mag >> 64);
-  const unsigned long long lo = static_cast<unsigned long long>(mag);
-  shift = 0;
-  if (hi == 0) {
-    d = __ull2double_rn(lo);
-  } else {  // top 64 bits and a sticky bit: one correct rounding
-    const int lz = __clzll(static_cast<long long>(hi));
-    const unsigned long long u = lz ? (hi << lz) | (lo >> (64 - lz)) : hi;
-    const unsigned long long sticky = (lo << lz) != 0ull ? 1ull : 0ull;
-    d = __ull2double_rn(u | sticky);
-    shift = 64 - lz;
-  }
-  return negative;
-}
-
-// The same for N <= 16 moduli, N a template parameter: P < 2^126, so W_l fits four limbs,
-// S = sum r_l W_l is known modulo 2^128, and R = S - q P (|R| < 1.5 P < 2^127) is exact in
-// 128-bit two's complement.  W_l, P and P/2 come from the compile-time table.  Bit for bit
-// the result of the kernel above (both round C' once).
-// Four blocks per SM (at most 64 registers): at 66 registers only three fit, 11% slower.
-template <int N, bool EST>
-__global__ void __launch_bounds__(256, 4) crt_reconstruct128_kernel(const __grid_constant__ CrtRecParams R) {
-  static_assert(N >= 1 && N <= 16, "128-bit path");
-  if (R.skip_if_flag && *R.skip_if_flag) return;
-  CrtStoreCtx sc = store_ctx(R);
-  sc.estimate = EST;  // compiled separately with and without the estimate
-  const uint8_t* const res = R.res;
-  const int64_t ld_res = R.ld_res, plane = R.plane, m = R.m, ncols = R.ncols;
-  const double P_inv = R.P_inv;
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  double e_acc = 0.0, v_acc = 0.0;
-  const int64_t cpb = R.cols_per_block;
-  const int64_t jstep = int64_t(gridDim.y) * cpb;
-  for (int64_t j0 = int64_t(blockIdx.y) * cpb; i < m && j0 < ncols; j0 += jstep) {
-    int64_t jb, j1;
-    triangle_cols(R.uplo, i, j0, j0 + cpb < ncols ? j0 + cpb : ncols, jb, j1);
-    if (jb >= j1) continue;
-    // software pipeline: the residues of column j+1 are loaded while column j is reduced
-    uint32_t rn[N];
-#pragma unroll
-    for (int l = 0; l < N; ++l) rn[l] = res[residue_index(i, jb, ld_res) + l * plane];
-    for (int64_t j = jb; j < j1; ++j) {
-      uint32_t rc[N];
-#pragma unroll
-      for (int l = 0; l < N; ++l) rc[l] = rn[l];
-      if (j + 1 < j1) {
-#pragma unroll
-        for (int l = 0; l < N; ++l) rn[l] = res[residue_index(i, j + 1, ld_res) + l * plane];
-      }
-      double d;
-      int shift;
-      const bool negative = crt_combine128<N>(rc, P_inv, d, shift);
-      crt_store(sc, i, j, negative ? -d : d, shift, e_acc, v_acc);
-    }
-  }
-  __shared__ double red[2][8];
-  if (EST) crt_reduce_energies(R, e_acc, v_acc, red);
 }
 
 // RN(|R| 2^escale) with its sign, for R = (r3 r2 r1 r0) in [-P/2, P/2) (128-bit two's
@@ -1456,20 +1326,11 @@ __global__ void __launch_bounds__(256) crt_merge_splits_kernel(uint8_t* __restri
 }
 
 template <int N>
-void launch_rec128(bool est, bool mma, dim3 grid, cudaStream_t stream, const CrtRecParams& R) {
-  if constexpr (N >= kCrtMinModuli) {
-    if (mma) {
-      if (est)
-        crt_reconstruct_mma_kernel<N, true><<<grid, 256, 0, stream>>>(R);
-      else
-        crt_reconstruct_mma_kernel<N, false><<<grid, 256, 0, stream>>>(R);
-      return;
-    }
-  }
+void launch_rec_mma(bool est, dim3 grid, cudaStream_t stream, const CrtRecParams& R) {
   if (est)
-    crt_reconstruct128_kernel<N, true><<<grid, 256, 0, stream>>>(R);
+    crt_reconstruct_mma_kernel<N, true><<<grid, 256, 0, stream>>>(R);
   else
-    crt_reconstruct128_kernel<N, false><<<grid, 256, 0, stream>>>(R);
+    crt_reconstruct_mma_kernel<N, false><<<grid, 256, 0, stream>>>(R);
 }
 
 template <int BN, int STAGES, bool PAIR, int MT = 1, int NW = 4>
@@ -1675,9 +1536,10 @@ cudaError_t launch_crt_reconstruct(const CrtReconstructArgs& args, cudaStream_t 
   // the tensor-core sum: whole warps of 32 rows copy the residue planes 16 bytes at a time and
   // four columns together, so the planes must be 16-byte aligned, hold every row of those warps
   // and whole groups of columns
-  const bool mma = args.moduli >= kCrtMinModuli && args.moduli <= 16 && reinterpret_cast<uintptr_t>(args.cres) % 16 == 0 &&
-                   args.ld_res % 32 == 0 && args.plane % 16 == 0 && args.ld_res >= (args.m + 31) / 32 * 32 &&
-                   args.plane >= (args.n + 3) / 4 * 4 * args.ld_res;
+  if (args.moduli >= kCrtMinModuli && args.moduli <= 16 &&
+      (reinterpret_cast<uintptr_t>(args.cres) % 16 != 0 || args.ld_res % 32 != 0 || args.plane % 16 != 0 ||
+       args.ld_res < (args.m + 31) / 32 * 32 || args.plane < (args.n + 3) / 4 * 4 * args.ld_res))
+    return cudaErrorInvalidValue;
   const int64_t rows_per_block = 256;
   const unsigned gx = unsigned((args.m + rows_per_block - 1) / rows_per_block);
   int64_t cpb = 4 * crt_rec_run(gx, (args.n + 3) / 4, args.uplo != 0);
@@ -1686,16 +1548,16 @@ cudaError_t launch_crt_reconstruct(const CrtReconstructArgs& args, cudaStream_t 
   const dim3 grid(gx, unsigned((args.n + cpb - 1) / cpb));
   const bool est = args.err_sq != nullptr;
   switch (args.moduli) {
-    case 8: launch_rec128<8>(est, mma, grid, stream, R); break;
-    case 9: launch_rec128<9>(est, mma, grid, stream, R); break;
-    case 10: launch_rec128<10>(est, mma, grid, stream, R); break;
-    case 11: launch_rec128<11>(est, mma, grid, stream, R); break;
-    case 12: launch_rec128<12>(est, mma, grid, stream, R); break;
-    case 13: launch_rec128<13>(est, mma, grid, stream, R); break;
-    case 14: launch_rec128<14>(est, mma, grid, stream, R); break;
-    case 15: launch_rec128<15>(est, mma, grid, stream, R); break;
-    case 16: launch_rec128<16>(est, mma, grid, stream, R); break;
-    default: crt_reconstruct_kernel<<<grid, 256, 0, stream>>>(R); break;  // other counts: 192-bit path
+    case 8: launch_rec_mma<8>(est, grid, stream, R); break;
+    case 9: launch_rec_mma<9>(est, grid, stream, R); break;
+    case 10: launch_rec_mma<10>(est, grid, stream, R); break;
+    case 11: launch_rec_mma<11>(est, grid, stream, R); break;
+    case 12: launch_rec_mma<12>(est, grid, stream, R); break;
+    case 13: launch_rec_mma<13>(est, grid, stream, R); break;
+    case 14: launch_rec_mma<14>(est, grid, stream, R); break;
+    case 15: launch_rec_mma<15>(est, grid, stream, R); break;
+    case 16: launch_rec_mma<16>(est, grid, stream, R); break;
+    default: crt_reconstruct_kernel<<<grid, 256, 0, stream>>>(R); break;  // more: 192-bit path
   }
   return cudaGetLastError();
 }

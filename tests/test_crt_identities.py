@@ -1,9 +1,8 @@
 """The integer identities the CRT kernels rest on, checked exactly on the CPU (Python integers
 and rationals; no GPU).
 
-* reconstruction: moduli in pairs share the factor Q_g = P / (p_2g p_2g+1) of their CRT weights,
-  W_l = Q_g X_l with X_l < 2^16, so sum_l r_l W_l = sum_g Q_g (r_2g X_2g + r_2g+1 X_2g+1)
-  exactly, each pair sum < 2^25 and each 32-bit limb column < 2^60;
+* reconstruction: with T_b = sum_l r_l (byte b of W_l), pairs T_2c + 2^8 T_2c+1 < 2^29 and columns
+  of two pairs < 2^46 give S = sum_l r_l W_l exactly, and S + q (2^128 - P) modulo 2^128 is S - q P;
 * split: for |t| <= 2^62 = hi 2^32 + lo, one FMA s = hi (2^32 mod p) + lo (exact, < 2^39) and
   one FMA with 1.5 2^52 give q = rint(s / p), and lo + hi c32 - q p (mod 2^32) is the symmetric
   residue of t for every odd modulus; for p = 256 it is t's low byte;
@@ -30,40 +29,27 @@ def crt_weights(n):
     return P, W
 
 
-def pair_table(n):
-    P, _ = crt_weights(n)
-    X, Q = [0] * n, []
-    for g in range(0, n, 2):
-        pa = MODULI[g]
-        pb = MODULI[g + 1] if g + 1 < n else 1
-        Q.append(P // (pa * pb))
-        X[g] = pb * pow(P // pa, -1, pa)
-        if g + 1 < n:
-            X[g + 1] = pa * pow(P // pb, -1, pb)
-    return P, X, Q
-
-
-@pytest.mark.parametrize("n", range(1, 17))
-def test_pair_weights_reproduce_the_crt_weights(n):
+@pytest.mark.parametrize("n", range(8, 17))
+def test_byte_sums_reproduce_the_crt_sum(n):
     P, W = crt_weights(n)
-    _, X, Q = pair_table(n)
     assert P < 2**128
-    for l in range(n):
-        assert Q[l // 2] * X[l] == W[l]
-        assert X[l] < 2**16
+    byte = [[(w >> (8 * b)) & 0xFF for b in range(16)] for w in W]
     rng = random.Random(n)
-    for _ in range(200):
-        r = [rng.randrange(p) for p in MODULI[:n]]
-        s_direct = sum(ri * wi for ri, wi in zip(r, W))
-        sums = [r[g] * X[g] + (r[g + 1] * X[g + 1] if g + 1 < n else 0) for g in range(0, n, 2)]
-        assert all(s < 2**25 for s in sums)
-        assert sum(Q[g] * R for g, R in enumerate(sums)) == s_direct
-        # the four 32-bit limb columns of sum_g Q_g R_g stay below 2^60
-        for q in range(4):
-            col = sum(((Q[g] >> (32 * q)) & 0xFFFFFFFF) * R for g, R in enumerate(sums))
-            assert col < 2**60
+    largest = [p - 1 for p in MODULI[:n]]
+    for r in [largest, *([rng.randrange(p) for p in MODULI[:n]] for _ in range(200))]:
+        T = [sum(ri * wb[b] for ri, wb in zip(r, byte)) for b in range(16)]
+        pairs = [T[2 * c] + 2**8 * T[2 * c + 1] for c in range(8)]  # X_0 .. X_3, Y_0 .. Y_3
+        assert all(x < 2**29 for x in pairs)
+        cols = [pairs[2 * q] + 2**16 * pairs[2 * q + 1] for q in range(4)]
+        assert all(x < 2**46 for x in cols)
+        S = sum(x << (32 * q) for q, x in enumerate(cols))
+        assert S == sum(ri * wi for ri, wi in zip(r, W))
+        # q within one of S / P, then S + q (2^128 - P) modulo 2^128 is S - q P
+        for q in (S // P, S // P + 1):
+            R = (S + q * (2**128 - P)) % 2**128
+            assert (R - 2**128 if R >> 127 else R) == S - q * P
         # and the value reconstructs: S mod P is the number the residues encode
-        x = s_direct % P
+        x = S % P
         assert all(x % p == ri for p, ri in zip(MODULI[:n], r))
 
 
