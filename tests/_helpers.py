@@ -6,7 +6,10 @@ from __future__ import annotations
 
 import ctypes
 import json
+import math
+import random
 import subprocess
+from fractions import Fraction
 from functools import lru_cache
 from pathlib import Path
 
@@ -172,3 +175,54 @@ def check_against_reference(case, C, eps_scale=1.0):
     assert np.all(np.abs(c - r)[fin] <= bound[fin])
     # padding rows of C (ldc > m) are never touched
     np.testing.assert_array_equal(C[m:, :], case["Cin"][m:, :])
+
+
+DBL_MIN = 2.0 ** -1022
+
+
+def exact_rn(R: int, escale: int) -> float:
+    """Nearest double (ties to even) of R 2^escale, for results in the normal range."""
+    x = Fraction(R) * Fraction(2) ** escale
+    if x == 0:
+        return 0.0
+    sign = -1.0 if x < 0 else 1.0
+    x = abs(x)
+    e = math.floor(math.log2(x.numerator) - math.log2(x.denominator))
+    while Fraction(2) ** e > x:
+        e -= 1
+    while Fraction(2) ** (e + 1) <= x:
+        e += 1
+    ulp = Fraction(2) ** (e - 52)
+    q, r = divmod(x, ulp)
+    if r * 2 > ulp or (r * 2 == ulp and q % 2 == 1):
+        q += 1
+    return sign * math.ldexp(float(q), e - 52)
+
+
+def remainders(bits: int, rng: random.Random, count: int):
+    """Random |R| < 2^bits, exact ties and lone sticky bits at random positions, values around
+    the least size that takes the reconstruction's one-rounding path (2^56 above the kB bits that
+    are folded into a sticky bit) and small ones, both signs."""
+    least = 56 + max(0, bits + 1 - 103)
+    for _ in range(count):
+        kind = rng.randrange(6)
+        L = rng.randrange(1, bits + 1)
+        if kind == 0:
+            m = rng.getrandbits(L)
+        elif kind == 1:  # a tie: bits below the 53-bit window are exactly 100..0
+            top = rng.getrandbits(53) | (1 << 52)
+            sh = rng.randrange(1, max(2, L - 53))
+            m = (top << sh) | (1 << (sh - 1))
+        elif kind == 2:  # just above a tie: a lone sticky bit far below
+            top = rng.getrandbits(53) | (1 << 52)
+            sh = rng.randrange(2, max(3, L - 53))
+            m = (top << sh) | (1 << (sh - 1)) | (1 << rng.randrange(0, sh - 1))
+        elif kind == 3:  # at the threshold
+            m = (1 << least) + rng.randrange(-(1 << 40), 1 << 40)
+        elif kind == 4:  # a few bits above and below it
+            m = rng.getrandbits(least + rng.randrange(-4, 5))
+        else:  # exactly representable values and their neighbours
+            m = (rng.getrandbits(53) | (1 << 52)) << rng.randrange(0, max(1, L - 53))
+            m += rng.choice([-1, 0, 1])
+        m = min(max(m, 0), (1 << bits) - 1)
+        yield -m if rng.random() < 0.5 else m

@@ -13,8 +13,7 @@ import random
 
 import pytest
 
-from _helpers import crt_model
-from test_crt_rounding_windows import DBL_MIN, exact_rn, remainders
+from _helpers import DBL_MIN, crt_model, exact_rn, remainders
 
 
 def one_path(R: int, escale: int, bits: int):
