@@ -1459,8 +1459,8 @@ cudaError_t launch_crt_gemm(const CrtOperand& a, const CrtOperand& b, const CrtG
   if (a.k_pad != b.k_pad || a.k_pad % kSliceKBytes != 0) return cudaErrorInvalidValue;
   if (args.tile_n == kTilePair) return launch_gemm_config<256, 6, true>(a, b, args, stream);
   if (args.tile_n == 256) return launch_gemm_config<256, 4, false>(a, b, args, stream);
-  // 256 x 256 per CTA: 64 KB stages (three), sixteen epilogue warps (four per TMEM lane
-  // quadrant: the single accumulator buffer is drained while the MMAs wait, so the drain is
+  // 256 x 256 per CTA: 64 KB stages (three), sixteen epilogue warps (four per TMEM lane quadrant: the
+  // next item's MMAs wait for each row tile of the single accumulator to be read out, so the read is
   // spread over as many warps as the registers allow)
   if (args.tile_n == kTileWide) return launch_gemm_config<256, 3, false, 2, 16>(a, b, args, stream);
   return cudaErrorInvalidValue;

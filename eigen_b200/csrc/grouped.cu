@@ -57,10 +57,10 @@ constexpr int kStages32 = 3;  // 6.9 KB per warp
 constexpr int kBlocks64 = 12, kBlocks32 = 8;  // per SM
 // A launch of few items is the latency of one item's chain of stages, and memory for longer rings and
 // registers for more copies in flight are free: FP64 takes a longer ring (us, 2 stages / 4: 100
-// products of 32 x 32 x 2048 184 / 119, 30 of 64 x 64 x 4096 377 / 246; 1184 items, eight per SM, 69 /
-// 69), and both unroll the copies of small products, FP32 with a copy path of its own where all are
-// small (500 products of 8 x 8 x 4000 361 / 297, 100 of 16 x 16 x 4000 343 / 275; 343 and 287 in the
-// kernel that knows tiles too).  Unrolled, FP32 is slower from 1184 items on (62.8 / 67.7).
+// products of 32 x 32 x 2048 184 / 119, 30 of 64 x 64 x 4096 372 / 246; 1184 items, eight per SM, 69 /
+// 69), and both unroll the copies of small products, FP32 in a kernel without the code of tiles where
+// all are small (500 products of 8 x 8 x 4000 361 / 257, 100 of 16 x 16 x 4000 343 / 247; 343 and 287
+// in the kernel that knows tiles too).  Unrolled, FP32 is slower from 1184 items on (62.8 / 67.7).
 constexpr int kDeepStages64 = 4;
 constexpr int64_t kDeepK = 128;  // the longest item's K, at least (at 32 the ring only takes longer to fill)
 constexpr int kDeepBlocks64 = 6, kDeepBlocks32 = 2;  // per SM, at most
@@ -318,8 +318,9 @@ __device__ __forceinline__ void frag_b(const float* sB, int l0, int g, int tig, 
 }
 // C fragments' six piece products of one 8-deep chunk, smallest first, each into a fresh fragment that
 // is then added to its result (round to nearest): fragment c is acc[slot(c)] += A piece ia(c) times B
-// piece ib(c).  The chains of six go a step of each in turn, or a lone warp would wait for each MMA
-// (100 products of 32 x 32 x 2048, A transposed: 215 -> 197 us with the copies above).
+// piece ib(c).  The chains of six go a step of each in turn, so that a warp with few others beside it
+// does not wait for each MMA (100 products of 32 x 32 x 2048, A transposed: 215 -> 191 us with the
+// unrolled copies).
 template <int C, int NA, int NB, class Slot, class Ia, class Ib>
 __device__ __forceinline__ void chunk_products(float (&acc)[8][4], const uint32_t (&pa)[NA][3][2],
                                                const uint32_t (&pb)[NB][3], Slot slot, Ia ia, Ib ib) {

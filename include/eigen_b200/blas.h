@@ -280,7 +280,8 @@ typedef struct eb2_call_info {
 } eb2_call_info;
 int eb2_last_call_info(eb2_call_info* out);
 /* The configuration class of this thread's last product (see eb2_set_config; -1 if none) and,
- * for a CRT DGEMM, its K splits per output tile and modulus (1: no split).  A separate call,
+ * for a CRT DGEMM, its K splits per output tile and modulus, for a split-BF16 SGEMM the K ranges
+ * of the tiles in its last round of CTAs (1: no split).  A separate call,
  * so that eb2_call_info keeps its layout for programs built against it. */
 int eb2_last_call_config(int* config, int* splits);
 
@@ -296,7 +297,9 @@ long long eb2_routine_calls(const char* name);
 int eb2_set_timing(int on);
 
 /* Stream-ordered product on device pointers; no host synchronisation unless the
- * a-posteriori check of the emulated DGEMM needs one (check_accuracy != 0).
+ * a-posteriori check of the emulated DGEMM needs one (check_accuracy != 0).  A CRT DGEMM that the
+ * picker configures waits on the host for its scan's statistics before its GEMM is enqueued (not
+ * in a capture, with a forced configuration class, or with both the modulus count and the tile set).
  * `stream` is a cudaStream_t (NULL = the legacy default stream).  Returns EB2_*.
  * Both can be captured into a CUDA graph once a direct call of the same size has sized the
  * workspace; a captured call that would need a larger workspace returns EB2_ERR_ARG without
