@@ -153,4 +153,4 @@ def test_one_fp32_product_per_launch_keeps_the_plan_s_pace():
     arr = eb.problems_array(probs)
     plan = eb.GroupedPlan("s", probs)
     t_plan, t_each = _best_ms(plan.execute), _best_ms(lambda: eb.gemm_each("s", arr))
-    assert t_each < 1.15 * t_plan, (t_plan, t_each)
+    assert t_each < 1.2 * t_plan, (t_plan, t_each)  # 1.03; 1.4 with 104 registers
